@@ -309,7 +309,8 @@ int  pmpic_ensemble_autotune(pmpic_ensemble* e);
 int  pmpic_ensemble_step(pmpic_ensemble* e, int nsteps, float* device_ms);
 /* The tuning in use: host threads, and per member the par2grid segment. */
 int  pmpic_ensemble_tuning(pmpic_ensemble* e, int* threads, int32_t* xseg_per_member);
-/* Columns per x segment of the par2grid row pass of one context (default 64). */
+/* Columns per x segment of the par2grid row pass of one context (default:
+ * by the grid and the form, enough segments to fill the GPU). */
 int  pmpic_set_p2g_segment(pmpic_ctx* ctx, int xseg);
 
 /* ---- instrumentation ------------------------------------------------------ */

@@ -197,7 +197,6 @@ int pmpic_create(const pmpic_config* cfg, pmpic_ctx** out) {
   std::memset((void*)&ctx->g, 0, sizeof(ctx->g));
   ctx->cfg = *cfg;
   ctx->mixed = cfg->precision == PMPIC_MIXED;
-  ctx->p2g_xseg = 64;
   ctx->device = cfg->device;
   ctx->parcels = nullptr;
   cudaError_t e = cudaSetDevice(cfg->device);
@@ -232,6 +231,7 @@ int pmpic_create(const pmpic_config* cfg, pmpic_ctx** out) {
   g.vmin = g.dx * g.dy * g.dz / 6. / 6. / 6.;       // parcel_mixing.F90:54
   g.rNz = 1.0 / (double)g.Nz;
   g.rNy = 1.0 / (double)g.Ny;
+  ctx->p2g_xseg = p2g_default_xseg(g, ctx->mixed);
   ctx->cap = cfg->max_parcels;
   ctx->n = 0;
   ctx->sorted_valid = false;

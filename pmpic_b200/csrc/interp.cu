@@ -22,6 +22,7 @@
 //               summing its contributions in one fixed order.
 #include <cuda_runtime.h>
 
+#include <algorithm>
 #include <mutex>
 #include <type_traits>
 
@@ -329,7 +330,6 @@ constexpr int NLV = ZC + 1;               // grid levels a chunk contributes to
 constexpr int BATCH = 128;                // sorted positions staged per batch
 constexpr int SPAD = BATCH + BATCH / 16;  // staged field stride: position p sits at p + p/16
 constexpr int RW = 4;                     // warps per CTA of the row pass
-constexpr int XSEG = 64;                  // default columns per x segment of a warp (tunable per context)
 // grid points in x per CTA of the combine pass (its staged rows fit the
 // 48 KB of static shared memory)
 template <class R>
@@ -883,12 +883,31 @@ int bin_and_sort(pmpic_ctx* ctx) {
   return 0;
 }
 
+// Columns per x segment of a warp of the row pass.  A warp walks its columns
+// one after the other (and one more to seed the carry), so a small grid's pass
+// lasts as long as one warp's walk, while on a large grid short segments only
+// repeat seed columns.  Measured (both passes of four fields, 8 parcels per
+// cell, against 64 columns): FP32 at 32^3 110 -> 22 us (1 column), 64^3 245 ->
+// 60 (5), 96^3 263 -> 130 (16: one wave; 32 columns 163), 128^3 330 -> 294 (8:
+// 4.6 waves; 16 columns, 2.3 waves, 305; 32 columns, 1.2 waves, 354), 192^3 881
+// -> 882 (32); FP64 at 32^3 95 -> 26 (1), 64^3 223 -> 88 (8), 128^3 520 -> 495 (16).
+int p2g_default_xseg(const Geom& g, bool fp32) {
+  const int64_t rows = (int64_t)((g.Nz + ZC - 1) / ZC) * g.Ny;
+  const int64_t resident = (int64_t)148 * RW * (fp32 ? 6 : 4);  // warps of one wave (k_p2g_rows' launch bounds)
+  const int64_t nxs = std::max<int64_t>(1, resident / rows);
+  const int one = (int)std::max<int64_t>(1, (g.Nx + nxs - 1) / nxs);  // the longest segment that is still one wave
+  if (one <= 24) return one;
+  for (int s = 32; s > 8; s >>= 1)  // several waves: the last one is then a small part
+    if (10 * rows * ((g.Nx + s - 1) / s) >= 34 * resident) return s;
+  return 8;
+}
+
 // the two passes of par2grid on `st`; rowpart holds 2 * nzc * Ny * Nx records
 // of P2GLayout::RPS / 2 values of type R (the y-low half, then the y-high half)
 template <int NQ, int MODE, bool BT, class R = double>
 static cudaError_t run_p2g(const Geom& g, const int32_t* start, const int32_t* sorted, const R* dx, const R* dy,
                            const R* dz, int ds, const R* vol, const P2GArgs<NQ, R>& a, R* rowpart, cudaStream_t st,
-                           int xseg = XSEG) {
+                           int xseg) {
   const int nzc = (g.Nz + ZC - 1) / ZC;
   const int nxs = (g.Nx + xseg - 1) / xseg;
   const int64_t nw = (int64_t)nxs * g.Ny * nzc;
@@ -1268,7 +1287,7 @@ extern "C" int pmpic_par2grid_static(int32_t nx, int32_t ny, int32_t nz, double 
   a.out[0] = out;
   a.nslot = n;
   if (run_p2g<1, 0, false>(g, cstart, sorted, del, del + SP_MAX_PARCELS, del + 2 * SP_MAX_PARCELS, 1, vol, a, rows,
-                           st) != cudaSuccess)
+                           st, p2g_default_xseg(g, false)) != cudaSuccess)
     return PMPIC_ERR_CUDA;
   int err = 0;
   if (cudaMemcpyAsync(&err, &info->error, sizeof(int), cudaMemcpyDeviceToHost, st) != cudaSuccess)
