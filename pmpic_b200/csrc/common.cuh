@@ -33,8 +33,9 @@ struct FftPlan {
   int nst;
   int radix[FFT_MAX_STAGES];
   int tw_off[FFT_MAX_STAGES];  // offset (in double2) of each stage's twiddle table
-  int n1, n2;                  // four-step split n = n1 * n2 (0: generic Stockham path)
-  int tw4_off;                 // offset of the four-step twiddles W_n^(n2 k1), [n2 * n1 + k1]
+  int n1, n2;                  // register split n = n1 * n2 (0: generic Stockham path)
+  bool st;                     // n1 and n2 are the products of the Stockham path's first and other stages
+  int tw4_off;                 // offset of the split's twiddles (fft.cu: fs_twiddles)
 };
 
 // Geometry of one rank covering the whole domain (setup_grid.F90:45-104,
@@ -389,30 +390,30 @@ int p2g_default_xseg(const Geom& g, bool fp32);
 int prop_upload(pmpic_ctx* ctx, int pid, int64_t off, int64_t n, const double* src);
 int prop_download(pmpic_ctx* ctx, int pid, int64_t off, int64_t n, double* dst);
 // fft.cu
-// Elementwise operators fused into an inverse transform: one on its spectral
-// input, applied as the first (x) pass reads it, and one on its physical
-// output, applied as the last (y) pass writes it.  Each repeats the arithmetic
-// of the separate operator kernel it replaces (same operands, same order), so
-// fused and unfused sequences give the same bits.
+// Elementwise operators fused into the inverse transforms' x pass, applied to
+// the spectra as they are read.  Each repeats the arithmetic of the separate
+// operator kernel it replaces (same operands, same order).  x, y, fs and zbar
+// are per array of a batch.
 enum SpecOpKind {
   SPEC_PLAIN = 0,
-  SPEC_DX,    // diffx (fft_ops.F90:266-295) of the input, tab = kx
-  SPEC_DY,    // diffy (fft_ops.F90:366-394) of the input, tab = ky
-  SPEC_FILT,  // the de-aliasing filter (fft_ops.F90:176-197), tab = filt
-  SPEC_VEL    // a velocity spectrum of vort2vel.F90:254-315 (see k_vel), no input array
+  SPEC_DX,    // diffx (fft_ops.F90:266-295) of x
+  SPEC_DY,    // diffy (fft_ops.F90:366-394) of x
+  SPEC_FILT,  // the de-aliasing filter (fft_ops.F90:176-197) of x
+  SPEC_VEL,   // the velocity spectra of vort2vel.F90:254-315: u, v from x = e and y = c, w from x = a and
+              // y = b; the filtered copy is stored to fs; zbar is the mean flow of u and v
+  SPEC_PAIR   // both derivatives of x, from one read
 };
 template <class R>
 struct SpecIn {
   int op = SPEC_PLAIN;
-  const R* tab = nullptr;
-  // SPEC_VEL: component vmode (0 u, 1 v, 2 w) from e, c (u, v) or a, b (w);
-  // its filtered copy is stored to fs; zbar is the mean flow of u or v
-  int vmode = 0;
-  const R *e = nullptr, *c = nullptr, *a = nullptr, *b = nullptr;
+  const R* x[4] = {};
+  const R* y[4] = {};
+  R* fs[4] = {};
+  const double* zbar[2] = {};
   const R *kx = nullptr, *ky = nullptr, *filt = nullptr;
-  R* fs = nullptr;
-  const double* zbar = nullptr;
 };
+// the pointwise operators on the output of a Stockham inverse y pass
+// (vorticity_tendency's products; the four-step lengths have k4_vt_y)
 enum PhysOpKind {
   PHYS_STORE = 0,
   PHYS_ADD_MUL,      // o = o + in0 * v
@@ -429,14 +430,20 @@ struct PhysOut {
   const R* in[6] = {};
 };
 int fft_init(pmpic_ctx* ctx);
+// Forward and inverse transforms of nb arrays (1..4) at once.  mids: nb
+// scratch arrays of nspec values that are no input or output of the call.
+int fft_forward(pmpic_ctx* ctx, int nb, const double* const* phys, double* const* spec, double* const* mids);
+int fft_forward(pmpic_ctx* ctx, int nb, const float* const* phys, float* const* spec, float* const* mids);
+int fft_inverse(pmpic_ctx* ctx, int nb, const SpecIn<double>& S, double* const* phys, double* const* mids);
+int fft_inverse(pmpic_ctx* ctx, int nb, const SpecIn<float>& S, float* const* phys, float* const* mids);
+// the inverse transforms and products of vorticity_tendency (fft_impl.cuh)
+int fft_tendency(pmpic_ctx* ctx, const SpecIn<double>& S, const double* const* pqr, double* const* dpqr,
+                 double* const* mids, double* const* work);
+int fft_tendency(pmpic_ctx* ctx, const SpecIn<float>& S, const float* const* pqr, float* const* dpqr,
+                 float* const* mids, float* const* work);
+// one array, with the context's own scratch
 int fft_forward(pmpic_ctx* ctx, const double* phys, double* spec);
 int fft_backward(pmpic_ctx* ctx, const double* spec, double* phys);
-int fft_forward(pmpic_ctx* ctx, const float* phys, float* spec);
-int fft_backward(pmpic_ctx* ctx, const float* spec, float* phys);
-int fft_backward(pmpic_ctx* ctx, const double* spec, double* phys, const SpecIn<double>& si,
-                 const PhysOut<double>& po);
-int fft_backward(pmpic_ctx* ctx, const float* spec, float* phys, const SpecIn<float>& si,
-                 const PhysOut<float>& po);
 // spectral.cu
 int spec_diffx(pmpic_ctx* ctx, const double* in, double* out);
 int spec_diffy(pmpic_ctx* ctx, const double* in, double* out);

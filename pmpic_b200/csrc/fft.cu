@@ -12,8 +12,9 @@
 // (Nz+1) x (Ny+2) x (Nx+2) after the x pass (the reference's four reals per
 // (kx, ky) mode, pencilfft.F90:838-864).
 //
-// Each CTA stages a batch of rows in shared memory and runs a radix-4/2/3/5
-// Stockham FFT over them.  Two real rows are packed into one complex row
+// Rows of two register radices (fft_impl.cuh: the four-step kernels) or, for
+// the other lengths, a radix-4/2/3/5 Stockham FFT over rows staged in shared
+// memory.  Two real rows are packed into one complex row
 // (re = row A, im = row B) and separated after the transform, which halves the
 // arithmetic of the reference's zero-imaginary complex transforms.
 #include <cuda_runtime.h>
@@ -23,13 +24,11 @@
 #include <vector>
 
 #include "common.cuh"
+#include "fft_rows.h"
 
 namespace pmpic {
 
 namespace {
-
-constexpr int FFT_THREADS = 256;
-constexpr int FS_THREADS = 128;
 
 bool factor(int n, std::vector<int>& out) {
   out.clear();
@@ -41,29 +40,57 @@ bool factor(int n, std::vector<int>& out) {
   return m == 1;
 }
 
-// the four-step split used for a row length (0: none)
-void fs_split(int n, int& n1, int& n2) {
-  n1 = n2 = 0;
-  switch (n) {
-    case 16: n1 = 4; n2 = 4; break;
-    case 32: n1 = 8; n2 = 4; break;
-    case 64: n1 = 8; n2 = 8; break;
-    case 128: n1 = 16; n2 = 8; break;
-    case 256: n1 = 16; n2 = 16; break;
-    default: break;
+// The register split n = n1 n2 of a row length (0: none), n1 and n2 in 2 .. 16.
+// Powers of two from 16 to 256 take the four-step split (st false: any
+// factorisation, one twiddle table).  The other lengths take a prefix of the
+// Stockham path's stages as n1 and the rest as n2 (st true), so that their
+// rows keep that path's arithmetic.  Of several the most even one.
+void fs_split(FftPlan& p, bool st) {
+  p.n1 = p.n2 = 0;
+  p.st = st;
+  if (!st) {
+    for (int a = 4; a <= 16; a *= 2)
+      for (int b = 4; b <= a; b *= 2)
+        if (a * b == p.n && (!p.n1 || a < p.n1)) {
+          p.n1 = a;
+          p.n2 = b;
+        }
+    return;
+  }
+  int a = 1;
+  for (int s = 0; s + 1 < p.nst; ++s) {
+    a *= p.radix[s];
+    const int b = p.n / a;
+    if (a <= 16 && b <= 16 && (!p.n1 || std::max(a, b) < std::max(p.n1, p.n2))) {
+      p.n1 = a;
+      p.n2 = b;
+    }
   }
 }
 
-// four-step twiddles W_n^(n2 k1), [n2 * n1 + k1], long double accuracy
-void fs_twiddles(FftPlan& p, std::vector<double2>& tw) {
-  fs_split(p.n, p.n1, p.n2);
+// The split's twiddles, long double accuracy, the index n2 fastest.
+// st false: W_n^(n2 k1).  st true, n1 = m1 m2 (m2 = 1: one stage): the first
+// stage's W_n^((n2 + n2's range m) k), [m m1 + k], then the second stage's
+// W_(n / m1)^(n2 k), [k].
+void fs_twiddles(FftPlan& p, bool st, std::vector<double2>& tw) {
+  fs_split(p, st);
   p.tw4_off = (int)tw.size();
   if (!p.n1) return;
-  for (int n2 = 0; n2 < p.n2; ++n2)
-    for (int k1 = 0; k1 < p.n1; ++k1) {
-      long double ang = -2.0L * 3.14159265358979323846264338327950288L * (long double)(n2 * k1) / (long double)p.n;
-      tw.push_back(make_double2((double)cosl(ang), (double)sinl(ang)));
-    }
+  auto put = [&](long long num, int den) {
+    const long double ang = -2.0L * 3.14159265358979323846264338327950288L * (long double)num / (long double)den;
+    tw.push_back(make_double2((double)cosl(ang), (double)sinl(ang)));
+  };
+  if (!p.st) {
+    for (int k1 = 0; k1 < p.n1; ++k1)
+      for (int n2 = 0; n2 < p.n2; ++n2) put((long long)n2 * k1, p.n);
+    return;
+  }
+  const int m1 = p.radix[0], m2 = p.n1 / m1;
+  for (int m = 0; m < m2; ++m)
+    for (int k = 0; k < m1; ++k)
+      for (int n2 = 0; n2 < p.n2; ++n2) put((long long)(n2 + p.n2 * m) * k, p.n);
+  for (int k = 0; k < m2; ++k)
+    for (int n2 = 0; n2 < p.n2; ++n2) put((long long)n2 * k, p.n / m1);
 }
 
 FftPlan make_plan(int n, std::vector<double2>& tw) {
@@ -90,34 +117,16 @@ FftPlan make_plan(int n, std::vector<double2>& tw) {
   return p;
 }
 
-int pick_txf(int nx) {
-  if (nx % 16 == 0) return 16;
-  if (nx % 8 == 0) return 8;
-  if (nx % 4 == 0) return 4;
-  return 2;
-}
-int pick_rp(int n) {  // complex rows per CTA for the x passes
-  int rp = 4096 / n;
-  if (rp < 1) rp = 1;
-  if (rp > 8) rp = 8;
-  return rp;
-}
-
 }  // namespace
 
-// the transform kernels, once per precision
+// the transform kernels of the FP64 path (fft32.cu: the FP32 form's)
 namespace f64 {
 using real = double;
 using real2 = double2;
 __host__ __device__ __forceinline__ double2 mk2(double a, double b) { return make_double2(a, b); }
 #include "fft_impl.cuh"
 }  // namespace f64
-namespace f32 {
-using real = float;
-using real2 = float2;
-__host__ __device__ __forceinline__ float2 mk2(float a, float b) { return make_float2(a, b); }
-#include "fft_impl.cuh"
-}  // namespace f32
+cudaError_t fft_attributes32();
 
 int fft_init(pmpic_ctx* ctx) {
   std::vector<int> tmp;
@@ -125,15 +134,14 @@ int fft_init(pmpic_ctx* ctx) {
     return set_error(ctx, PMPIC_ERR_CONFIG, "nx and ny must have only the prime factors 2, 3 and 5");
   std::vector<double2> tw;
   FftPlan px = make_plan(ctx->g.Nx, tw);
-  fs_twiddles(px, tw);
+  auto pow2 = [](int n) { return n >= 16 && n <= 256 && (n & (n - 1)) == 0; };
+  fs_twiddles(px, !pow2(px.n), tw);
   ctx->ftw_off_y = (int)tw.size();
   ctx->ftw_off_x = 0;
   FftPlan py = make_plan(ctx->g.Ny, tw);
-  fs_twiddles(py, tw);
+  fs_twiddles(py, !(pow2(py.n) && ctx->g.Nx % 16 == 0), tw);
   for (int s = 0; s < py.nst; ++s) py.tw_off[s] -= ctx->ftw_off_y;
   py.tw4_off -= ctx->ftw_off_y;
-  // the y passes of the four-step path take 16 columns per CTA
-  if (ctx->g.Nx % 16 != 0) py.n1 = py.n2 = 0;
   PMPIC_CUDA(cudaMalloc(&ctx->ftw, sizeof(double2) * tw.size()));
   PMPIC_CUDA(cudaMemcpy(ctx->ftw, tw.data(), sizeof(double2) * tw.size(), cudaMemcpyHostToDevice));
   // the FP32 table: the same twiddles rounded once to single precision
@@ -145,28 +153,27 @@ int fft_init(pmpic_ctx* ctx) {
   ctx->plan_y = py;
   // per device (the attribute is a property of the function on the current device)
   PMPIC_CUDA(f64::fft_attributes());
-  PMPIC_CUDA(f32::fft_attributes());
+  PMPIC_CUDA(fft_attributes32());
   return 0;
 }
 
+int fft_forward(pmpic_ctx* ctx, int nb, const double* const* phys, double* const* spec, double* const* mids) {
+  return f64::fft_forward_impl(ctx, nb, phys, spec, mids, (const double2*)ctx->ftw);
+}
+int fft_inverse(pmpic_ctx* ctx, int nb, const SpecIn<double>& S, double* const* phys, double* const* mids) {
+  return f64::fft_inverse_impl(ctx, nb, S, phys, mids, (const double2*)ctx->ftw);
+}
+int fft_tendency(pmpic_ctx* ctx, const SpecIn<double>& S, const double* const* pqr, double* const* dpqr,
+                 double* const* mids, double* const* work) {
+  return f64::fft_tendency_impl(ctx, S, pqr, dpqr, mids, work, (const double2*)ctx->ftw);
+}
 int fft_forward(pmpic_ctx* ctx, const double* phys, double* spec) {
-  return f64::fft_forward_impl(ctx, phys, spec, ctx->fftmid, (const double2*)ctx->ftw);
+  return fft_forward(ctx, 1, &phys, &spec, &ctx->fftmid);
 }
 int fft_backward(pmpic_ctx* ctx, const double* spec, double* phys) {
-  return fft_backward(ctx, spec, phys, SpecIn<double>{}, PhysOut<double>{});
-}
-int fft_backward(pmpic_ctx* ctx, const double* spec, double* phys, const SpecIn<double>& si,
-                 const PhysOut<double>& po) {
-  return f64::fft_backward_impl(ctx, spec, phys, ctx->fftmid, (const double2*)ctx->ftw, si, po);
-}
-int fft_forward(pmpic_ctx* ctx, const float* phys, float* spec) {
-  return f32::fft_forward_impl(ctx, phys, spec, (float*)ctx->fftmid, (const float2*)ctx->ftw32);
-}
-int fft_backward(pmpic_ctx* ctx, const float* spec, float* phys) {
-  return fft_backward(ctx, spec, phys, SpecIn<float>{}, PhysOut<float>{});
-}
-int fft_backward(pmpic_ctx* ctx, const float* spec, float* phys, const SpecIn<float>& si, const PhysOut<float>& po) {
-  return f32::fft_backward_impl(ctx, spec, phys, (float*)ctx->fftmid, (const float2*)ctx->ftw32, si, po);
+  SpecIn<double> S;
+  S.x[0] = spec;
+  return fft_inverse(ctx, 1, S, &phys, &ctx->fftmid);
 }
 
 }  // namespace pmpic

@@ -200,52 +200,59 @@ __device__ __forceinline__ real2 c2r_pack(real2 A, real2 B, int k, int n) {
 // mode) and row ra + 1 the odd one of the same level lev; each value is the
 // element pair (2 km, 2 km + 1) of its row.  The operators repeat the
 // arithmetic of diffx, diffy and the filter (spectral_impl.cuh: dx_of, dy_of,
-// k_filter) and the velocity spectra of vort2vel.F90:251-320 (e - diffy(c),
-// diffx(c) - e, diffy(a) - diffx(b); the mean flow in mode (0, 0) of u and v).
+// k_filter) and the velocity spectra of vort2vel.F90:251-320 (e - diffy(c), diffx(c) - e,
+// diffy(a) - diffx(b); the mean flow in mode (0, 0) of u and v).
 // own: this thread reads mode km unmirrored, so it stores the filtered
 // velocity spectrum of SPEC_VEL.
 __device__ __forceinline__ real2 ld2(const real* __restrict__ p, size_t i) { return *(const real2*)&p[i]; }
 __device__ __forceinline__ void st2(real* __restrict__ p, size_t i, real2 v) { *(real2*)&p[i] = v; }
 
+// one array of a batch (selected without indexing the parameter arrays: no local copy)
+template <class T>
+__device__ __forceinline__ T* pick(T* const (&p)[4], int b) {
+  return b == 0 ? p[0] : (b == 1 ? p[1] : (b == 2 ? p[2] : p[3]));
+}
+
 // The operator on the values of one spectral element pair of rows ra (xa)
 // and ra + 1 (xb); ca, cb are their spectral columns, lev their level.  For
-// SPEC_VEL x is e (u, v) or a (w) and y is c (u, v) or b (w).  The wavenumber
-// tables are laid out like the spectra but kx depends on the x index alone and
-// ky on the row alone, so kx is read from row 0 (x2 = 2 km, the pair's x
-// index) and ky from column 0 of rows ca - x2 and cb - x2: the same values,
-// one small L1-resident row or a per-thread constant instead of a second
-// spectrum-sized read per element.
+// SPEC_VEL the batch index q is the component (0 u, 1 v, 2 w), x is e (u, v)
+// or a (w) and y is c (u, v) or b (w).  The wavenumber tables are laid out
+// like the spectra but kx depends on the x index alone and ky on the row
+// alone, so kx is read from row 0 (x2 = 2 km, the pair's x index) and ky from
+// column 0 of rows ca - x2 and cb - x2: the same values, one small
+// L1-resident row or a per-thread constant instead of a second spectrum-sized
+// read per element.
 template <int OP>
-__device__ __forceinline__ void spec_op(const SpecIn<real>& S, real2 xa, real2 xb, real2 ya, real2 yb, int ca, int cb,
-                                        int x2, int lev, real2& A, real2& B) {
+__device__ __forceinline__ void spec_op(const SpecIn<real>& S, int q, real2 xa, real2 xb, real2 ya, real2 yb, int ca,
+                                        int cb, int x2, int lev, real2& A, real2& B) {
   auto kxp = [&](const real* t) { return ld2(t, x2); };
   auto kyp = [&](const real* t, int c) { const real v = t[c - x2]; return mk2(v, v); };
   if constexpr (OP == SPEC_VEL) {
-    if (S.vmode == 0) {  // f = e - diffy(c), f(:,1,1) = ubar
+    if (q == 0) {  // f = e - diffy(c), f(:,1,1) = ubar
       const real2 ta = kyp(S.ky, ca), tb = kyp(S.ky, cb);
       A = mk2(xa.x - (real(-1) * yb.x) * ta.x, xa.y - (real(-1) * yb.y) * ta.y);
       B = mk2(xb.x - ya.x * tb.x, xb.y - ya.y * tb.y);
-      if (ca == 0) A.x = (real)S.zbar[lev];
-    } else if (S.vmode == 1) {  // f = diffx(c) - e, f(:,1,1) = vbar
+      if (ca == 0) A.x = (real)S.zbar[0][lev];
+    } else if (q == 1) {  // f = diffx(c) - e, f(:,1,1) = vbar
       const real2 ta = kxp(S.kx), tb = ta;
       A = mk2((real(-1) * ya.y) * ta.x - xa.x, ya.x * ta.y - xa.y);
       B = mk2((real(-1) * yb.y) * tb.x - xb.x, yb.x * tb.y - xb.y);
-      if (ca == 0) A.x = (real)S.zbar[lev];
+      if (ca == 0) A.x = (real)S.zbar[1][lev];
     } else {  // f = diffy(a) - diffx(b)
       const real2 ya2 = kyp(S.ky, ca), yb2 = kyp(S.ky, cb), xa2 = kxp(S.kx), xb2 = xa2;
       A = mk2((real(-1) * xb.x) * ya2.x - (real(-1) * ya.y) * xa2.x, (real(-1) * xb.y) * ya2.y - ya.x * xa2.y);
       B = mk2(xa.x * yb2.x - (real(-1) * yb.y) * xb2.x, xa.y * yb2.y - yb.x * xb2.y);
     }
-  } else if constexpr (OP == SPEC_DX) {  // tab = kx
-    const real2 ta = kxp(S.tab), tb = ta;
+  } else if constexpr (OP == SPEC_DX) {
+    const real2 ta = kxp(S.kx), tb = ta;
     A = mk2((real(-1) * xa.y) * ta.x, xa.x * ta.y);
     B = mk2((real(-1) * xb.y) * tb.x, xb.x * tb.y);
-  } else if constexpr (OP == SPEC_DY) {  // tab = ky
-    const real2 ta = kyp(S.tab, ca), tb = kyp(S.tab, cb);
+  } else if constexpr (OP == SPEC_DY) {
+    const real2 ta = kyp(S.ky, ca), tb = kyp(S.ky, cb);
     A = mk2((real(-1) * xb.x) * ta.x, (real(-1) * xb.y) * ta.y);
     B = mk2(xa.x * tb.x, xa.y * tb.y);
   } else if constexpr (OP == SPEC_FILT) {
-    const real2 ta = ld2(S.tab, ca), tb = ld2(S.tab, cb);
+    const real2 ta = ld2(S.filt, ca), tb = ld2(S.filt, cb);
     A = mk2(xa.x * ta.x, xa.y * ta.y);
     B = mk2(xb.x * tb.x, xb.y * tb.y);
   } else {
@@ -254,37 +261,27 @@ __device__ __forceinline__ void spec_op(const SpecIn<real>& S, real2 xa, real2 x
   }
 }
 // the filtered copy of a velocity spectrum pair (SPEC_VEL), at elements ea, eb
-__device__ __forceinline__ void vel_store(const SpecIn<real>& S, size_t ea, size_t eb, int ca, int cb, real2 A,
+__device__ __forceinline__ void vel_store(const SpecIn<real>& S, int q, size_t ea, size_t eb, int ca, int cb, real2 A,
                                           real2 B) {
   const real2 fa = ld2(S.filt, ca), fb = ld2(S.filt, cb);
-  st2(S.fs, ea, mk2(A.x * fa.x, A.y * fa.y));
-  st2(S.fs, eb, mk2(B.x * fb.x, B.y * fb.y));
+  real* fs = pick(S.fs, q);
+  st2(fs, ea, mk2(A.x * fa.x, A.y * fa.y));
+  st2(fs, eb, mk2(B.x * fb.x, B.y * fb.y));
 }
 // the operator's inputs of the element pair read from global memory
 template <int OP>
-__device__ __forceinline__ void spec_pair(const Geom& g, const real* __restrict__ spec, const SpecIn<real>& S,
-                                          int64_t ra, int jp, int lev, int km, bool own, real2& A, real2& B) {
+__device__ __forceinline__ void spec_pair(const Geom& g, const SpecIn<real>& S, int q, int64_t ra, int jp, int lev,
+                                          int km, bool own, real2& A, real2& B) {
   const size_t ea = (size_t)ra * g.sx + 2 * km, eb = ea + g.sx;
   const int ca = jp * g.sx + 2 * km, cb = ca + g.sx;  // spectral columns of elements ea, eb
+  const real* x = pick(S.x, q);
   if constexpr (OP == SPEC_VEL) {
-    const real* x = S.vmode == 2 ? S.a : S.e;
-    const real* y = S.vmode == 2 ? S.b : S.c;
-    spec_op<OP>(S, ld2(x, ea), ld2(x, eb), ld2(y, ea), ld2(y, eb), ca, cb, 2 * km, lev, A, B);
-    if (own) vel_store(S, ea, eb, ca, cb, A, B);
+    const real* y = pick(S.y, q);
+    spec_op<OP>(S, q, ld2(x, ea), ld2(x, eb), ld2(y, ea), ld2(y, eb), ca, cb, 2 * km, lev, A, B);
+    if (own) vel_store(S, q, ea, eb, ca, cb, A, B);
   } else {
-    const real2 a = ld2(spec, ea), b = ld2(spec, eb);
-    spec_op<OP>(S, a, b, a, b, ca, cb, 2 * km, lev, A, B);
-  }
-}
-// the same with the operator chosen at run time (generic-length path)
-__device__ __forceinline__ void spec_pair_rt(const Geom& g, const real* __restrict__ spec, const SpecIn<real>& S,
-                                             int64_t ra, int jp, int lev, int km, bool own, real2& A, real2& B) {
-  switch (S.op) {
-    case SPEC_DX: spec_pair<SPEC_DX>(g, spec, S, ra, jp, lev, km, own, A, B); break;
-    case SPEC_DY: spec_pair<SPEC_DY>(g, spec, S, ra, jp, lev, km, own, A, B); break;
-    case SPEC_FILT: spec_pair<SPEC_FILT>(g, spec, S, ra, jp, lev, km, own, A, B); break;
-    case SPEC_VEL: spec_pair<SPEC_VEL>(g, spec, S, ra, jp, lev, km, own, A, B); break;
-    default: spec_pair<SPEC_PLAIN>(g, spec, S, ra, jp, lev, km, own, A, B); break;
+    const real2 a = ld2(x, ea), b = ld2(x, eb);
+    spec_op<OP>(S, q, a, b, a, b, ca, cb, 2 * km, lev, A, B);
   }
 }
 
@@ -309,18 +306,6 @@ __device__ __forceinline__ real phys_op(const PhysOut<real>& E, size_t i, real v
   }
   return o;
 }
-// two consecutive elements i, i + 1 (i even, rows of even length)
-template <int OP>
-__device__ __forceinline__ void phys_out2(const PhysOut<real>& E, real* __restrict__ phys, size_t i, real2 v) {
-  if (OP == PHYS_STORE || E.store) st2(phys, i, v);
-  if constexpr (OP != PHYS_STORE) {
-    real w0 = real(0), w1 = real(0);
-    const real o0 = phys_op<OP>(E, i, v.x, w0);
-    const real o1 = phys_op<OP>(E, i + 1, v.y, w1);
-    st2(E.o, i, mk2(o0, o1));
-    if constexpr (OP == PHYS_DQ_DR) st2(E.o2, i, mk2(w0, w1));
-  }
-}
 // one element, the operator chosen at run time (generic-length path)
 __device__ __forceinline__ void phys_out_rt(const PhysOut<real>& E, real* __restrict__ phys, size_t i, real v) {
   if (E.op == PHYS_STORE || E.store) phys[i] = v;
@@ -338,9 +323,11 @@ __device__ __forceinline__ void phys_out_rt(const PhysOut<real>& E, real* __rest
 }
 
 // ---- inverse x pass: spec -> mid ------------------------------------------------
+// (one array, batch entry q)
+template <int OP>
 __global__ void __launch_bounds__(FFT_THREADS) k_inv_x(Geom g, int RP, int64_t nrows_total, FftPlan pl,
-                                                       const real2* __restrict__ tw, const real* __restrict__ spec,
-                                                       real* __restrict__ mid, SpecIn<real> S) {
+                                                       const real2* __restrict__ tw, real* __restrict__ mid,
+                                                       SpecIn<real> S, int q) {
   extern __shared__ real2 sm[];
   const int Nx = g.Nx;
   real2* b0 = sm;
@@ -352,8 +339,8 @@ __global__ void __launch_bounds__(FFT_THREADS) k_inv_x(Geom g, int RP, int64_t n
     int64_t ra = row0 + 2 * r;
     real2 A = mk2(real(0), real(0)), B = mk2(real(0), real(0));
     if (ra < nrows_total) {
-      const int lev = (int)(ra / g.sy);
-      spec_pair_rt(g, spec, S, ra, (int)(ra - (int64_t)lev * g.sy), lev, km, 2 * k <= Nx, A, B);
+      const int l = (int)(ra / g.sy);
+      spec_pair<OP>(g, S, q, ra, (int)(ra - (int64_t)l * g.sy), l, km, 2 * k <= Nx, A, B);
     }
     b0[r * Nx + k] = c2r_pack(A, B, k, Nx);
   }
@@ -371,9 +358,9 @@ __global__ void __launch_bounds__(FFT_THREADS) k_inv_x(Geom g, int RP, int64_t n
 }
 
 // ---- inverse y pass: mid -> phys ------------------------------------------------
-__global__ void __launch_bounds__(FFT_THREADS) k_inv_y(Geom g, int TXF, FftPlan pl, const real2* __restrict__ tw,
-                                                       const real* __restrict__ mid, real* __restrict__ phys,
-                                                       PhysOut<real> E) {
+__global__ void __launch_bounds__(FFT_THREADS) k_inv_y(Geom g, int TXF, FftPlan pl,
+                                                       const real2* __restrict__ tw, const real* __restrict__ mid,
+                                                       real* __restrict__ phys, PhysOut<real> E) {
   extern __shared__ real2 sm[];
   const int Ny = g.Ny, Nx = g.Nx;
   const int nr = TXF / 2;
@@ -405,11 +392,16 @@ __global__ void __launch_bounds__(FFT_THREADS) k_inv_y(Geom g, int TXF, FftPlan 
   }
 }
 
-// ---- four-step register FFT for n = n1 * n2, n1, n2 in {4, 8, 16} --------------------
+// ---- four-step register FFT for n = n1 * n2, n1 and n2 in 2 .. 16 ---------------------
 // x[n2 + N2 n1] -> X[k1 + N1 k2]:  n1-point DFTs over n1 (one thread per n2),
 // twiddle W_n^(n2 k1), transpose through shared memory, n2-point DFTs over n2
 // (one thread per k1).  The small DFTs run in registers; loads and stores touch
 // global memory once each.
+// The kernels are instantiated for the splits (N1c, N2c) of FS_SPLITS and once
+// for every other length with the split read at run time (N1c = N2c = 0): the
+// radix then selects among the register DFTs by a branch that is uniform over
+// the grid.  What bounds them is L1 / shared memory: the twiddles are laid out
+// [k1][n2], so that the lanes of a warp, which differ in n2, read one line.
 
 // W_16^m = exp(-2 pi i m / 16), m known at compile time after unrolling
 __device__ __forceinline__ real2 w16(int m) {
@@ -435,14 +427,65 @@ __device__ __forceinline__ real2 w16(int m) {
     default: return mk2(C1, C3);
   }
 }
+// W_R^m for the other composite radices, R = 6, 9, 10, 12, 15 (m <= 8 occurs)
+template <int R>
+__device__ __forceinline__ real2 wr(int m) {
+  if constexpr (R == 6) {
+    switch (m) {
+      case 1: return mk2(0.5, -0.866025403784438646764);
+      default: return mk2(-0.5, -0.866025403784438646764);
+    }
+  } else if constexpr (R == 9) {
+    switch (m) {
+      case 1: return mk2(0.766044443118978035202, -0.642787609686539326323);
+      case 2: return mk2(0.173648177666930348852, -0.984807753012208059367);
+      case 3: return mk2(-0.5, -0.866025403784438646764);
+      default: return mk2(-0.939692620785908384054, -0.342020143325668733044);
+    }
+  } else if constexpr (R == 10) {
+    switch (m) {
+      case 1: return mk2(0.809016994374947424102, -0.587785252292473129169);
+      case 2: return mk2(0.309016994374947424102, -0.951056516295153572116);
+      case 3: return mk2(-0.309016994374947424102, -0.951056516295153572116);
+      default: return mk2(-0.809016994374947424102, -0.587785252292473129169);
+    }
+  } else if constexpr (R == 12) {
+    switch (m) {
+      case 1: return mk2(0.866025403784438646764, -0.5);
+      case 2: return mk2(0.5, -0.866025403784438646764);
+      case 3: return mk2(0.0, -1.0);
+      case 4: return mk2(-0.5, -0.866025403784438646764);
+      case 5: return mk2(-0.866025403784438646764, -0.5);
+      default: return mk2(-1.0, 0.0);
+    }
+  } else {
+    switch (m) {
+      case 1: return mk2(0.913545457642600895502, -0.406736643075800207754);
+      case 2: return mk2(0.669130606358858213826, -0.743144825477394235015);
+      case 3: return mk2(0.309016994374947424102, -0.951056516295153572116);
+      case 4: return mk2(-0.104528463267653471400, -0.994521895368273336923);
+      case 5: return mk2(-0.5, -0.866025403784438646764);
+      case 6: return mk2(-0.809016994374947424102, -0.587785252292473129169);
+      case 7: return mk2(-0.978147600733805637929, -0.207911690817759337102);
+      default: return mk2(-0.978147600733805637929, 0.207911690817759337102);
+    }
+  }
+}
 
-// forward DFT of size R in registers, natural order in and out
+// the first of the (one or two) stages of a register radix, in the Stockham
+// path's order 4, 2, 3, 5
+__host__ __device__ constexpr int first_stage(int R) {
+  return R <= 5 ? R : (R % 4 == 0 ? 4 : (R % 2 == 0 ? 2 : 3));
+}
+// forward DFT of size R in registers, natural order in and out: composite
+// sizes as M1 x M2 with the constants above (8 = 4 x 2, 16 = 4 x 4, 6 = 2 x 3,
+// 9 = 3 x 3, 10 = 2 x 5, 12 = 4 x 3, 15 = 3 x 5)
 template <int R>
 __device__ __forceinline__ void dft(real2* a) {
   if constexpr (R <= 5) {
     small_dft<R>(a);
   } else {
-    constexpr int M1 = 4, M2 = R / 4;  // R = 8: 4 x 2, R = 16: 4 x 4
+    constexpr int M1 = first_stage(R), M2 = R / M1;
     real2 y[R];
 #pragma unroll
     for (int n2 = 0; n2 < M2; ++n2) {
@@ -451,7 +494,11 @@ __device__ __forceinline__ void dft(real2* a) {
       for (int n1 = 0; n1 < M1; ++n1) b[n1] = a[M2 * n1 + n2];
       small_dft<M1>(b);
 #pragma unroll
-      for (int k1 = 0; k1 < M1; ++k1) y[k1 * M2 + n2] = (n2 * k1 == 0) ? b[k1] : cmul(b[k1], w16(n2 * k1 * (16 / R)));
+      for (int k1 = 0; k1 < M1; ++k1) {
+        if (n2 * k1 == 0) y[k1 * M2 + n2] = b[k1];
+        else if constexpr (R == 8 || R == 16) y[k1 * M2 + n2] = cmul(b[k1], w16(n2 * k1 * (16 / R)));
+        else y[k1 * M2 + n2] = cmul(b[k1], wr<R>(n2 * k1));
+      }
     }
 #pragma unroll
     for (int k1 = 0; k1 < M1; ++k1) {
@@ -464,164 +511,264 @@ __device__ __forceinline__ void dft(real2* a) {
     }
   }
 }
-
-
-// step 1 of one row: a[n1] = x[n2 + N2 n1] on entry; Y row [k1][n2] (padded)
-template <int N1, int N2>
-__device__ __forceinline__ void fs_step1(real2* a, int n2, real2* Yrow, const real2* __restrict__ tw4) {
-  dft<N1>(a);
+template <int R>
+struct Rad {
+  static constexpr int value = R;
+};
+// f(Rad<r>) for the radix r: known at compile time (RC > 0), or one of the radices of fs_split
+template <int RC, class F>
+__device__ __forceinline__ void with_radix(int r, F&& f) {
+  if constexpr (RC > 0) {
+    f(Rad<RC>{});
+  } else {
+    switch (r) {
+      case 2: f(Rad<2>{}); break;
+      case 3: f(Rad<3>{}); break;
+      case 4: f(Rad<4>{}); break;
+      case 5: f(Rad<5>{}); break;
+      case 6: f(Rad<6>{}); break;
+      case 8: f(Rad<8>{}); break;
+      case 9: f(Rad<9>{}); break;
+      case 10: f(Rad<10>{}); break;
+      case 12: f(Rad<12>{}); break;
+      case 15: f(Rad<15>{}); break;
+      default: f(Rad<16>{}); break;
+    }
+  }
+}
+// step 1 of one row: a[n1] = x[n2 + N2 n1] on entry; Y row [k1][n2] (padded).
+// ST: the first one or two stages of the Stockham path themselves, with its
+// twiddles (the length's other stages are the step-3 DFTs): a row then has the
+// bits that the Stockham kernels give it, whichever of the two runs.
+// Otherwise an R-point DFT and the twiddle W_n^(n2 k1).
+template <int R, bool ST>
+__device__ __forceinline__ void fs_step1(real2* a, int n2, int N2, real2* Yrow, const real2* __restrict__ tw4) {
+  if constexpr (ST) {
+    constexpr int M1 = first_stage(R), M2 = R / M1;
+    real2 y[R];
 #pragma unroll
-  for (int k1 = 0; k1 < N1; ++k1) Yrow[k1 * (N2 + 1) + n2] = (k1 == 0 || n2 == 0) ? a[k1] : cmul(a[k1], tw4[n2 * N1 + k1]);
+    for (int m = 0; m < M2; ++m) {
+      real2 b[M1];
+#pragma unroll
+      for (int u = 0; u < M1; ++u) b[u] = a[M2 * u + m];
+      small_dft<M1>(b);
+#pragma unroll
+      for (int k = 0; k < M1; ++k) y[k * M2 + m] = k == 0 ? b[k] : cmul(b[k], tw4[(m * M1 + k) * N2 + n2]);
+    }
+    const real2* __restrict__ t2 = tw4 + R * N2;
+#pragma unroll
+    for (int k1 = 0; k1 < M1; ++k1) {
+      real2 c[M2];
+#pragma unroll
+      for (int m = 0; m < M2; ++m) c[m] = y[k1 * M2 + m];
+      if constexpr (M2 > 1) small_dft<M2>(c);
+#pragma unroll
+      for (int k2 = 0; k2 < M2; ++k2)
+        Yrow[(k1 + M1 * k2) * (N2 + 1) + n2] = k2 == 0 ? c[k2] : cmul(c[k2], t2[k2 * N2 + n2]);
+    }
+  } else {
+    dft<R>(a);
+#pragma unroll
+    for (int k1 = 0; k1 < R; ++k1)
+      Yrow[k1 * (N2 + 1) + n2] = (k1 == 0 || n2 == 0) ? a[k1] : cmul(a[k1], tw4[k1 * N2 + n2]);
+  }
 }
 // step 3 of one row: a[k2] = X[k1 + N1 k2] on return
-template <int N1, int N2>
+template <int R>
 __device__ __forceinline__ void fs_step3(real2* a, int k1, const real2* Yrow) {
 #pragma unroll
-  for (int n2 = 0; n2 < N2; ++n2) a[n2] = Yrow[k1 * (N2 + 1) + n2];
-  dft<N2>(a);
+  for (int n2 = 0; n2 < R; ++n2) a[n2] = Yrow[k1 * (R + 1) + n2];
+  dft<R>(a);
 }
+__host__ __device__ constexpr int FS_AM(int n1, int n2) { return n1 == 0 ? 16 : (n1 > n2 ? n1 : n2); }
+// complex rows of an x pass's CTA, and the shared values of a CTA's rows: x
+// passes pad rows to N1 (N2 + 1), y passes by one more, so
+// that the column pairs of a warp fall in distinct banks
+constexpr int FS_YV = 128 / sizeof(real2);  // a row's column pairs are one 128-byte line
+constexpr int FS_YT = 16 * FS_YV;           // threads of a y pass's CTA at most
+__host__ __device__ constexpr int fs_rows(int n1, int n2) { return FS_THREADS / (n1 > n2 ? n1 : n2); }
+__host__ __device__ constexpr int fs_xvals(int n1, int n2) { return n1 == 0 ? 8 * 16 * 17 : fs_rows(n1, n2) * n1 * (n2 + 1); }
+__host__ __device__ constexpr int fs_yvals(int n1, int n2) { return n1 == 0 ? FS_YV * (16 * 17 + 1) : FS_YV * (n1 * (n2 + 1) + 1); }
 
-// forward x pass (mid -> spec): RP complex rows (pairs of real rows) per CTA
-template <int N1, int N2>
-__global__ void __launch_bounds__(FS_THREADS) k4_fwd_x(Geom g, int64_t nrows_total, const real2* __restrict__ tw4,
-                                                       const real* __restrict__ mid, real* __restrict__ spec) {
-  constexpr int N = N1 * N2, RP = FS_THREADS / (N1 > N2 ? N1 : N2), YS = N1 * (N2 + 1);
-  __shared__ real2 Y[RP * YS];
+template <class T>
+struct Arr4 {
+  T* p[4];
+};
+
+// forward x pass (mid -> spec): pairs of real rows; blockIdx.y is the array of the batch
+template <int N1c, int N2c, bool ST>
+__global__ void __launch_bounds__(FS_THREADS) k4_fwd_x(Geom g, int n1, int n2_, int64_t nrows,
+                                                       const real2* __restrict__ tw4, Arr4<const real> mids,
+                                                       Arr4<real> specs) {
+  const int N1 = N1c ? N1c : n1, N2 = N2c ? N2c : n2_, N = N1 * N2;
+  const int RP = FS_THREADS / (N1 > N2 ? N1 : N2), YS = N1 * (N2 + 1);
+  __shared__ real2 Y[fs_xvals(N1c, N2c)];
   real2* X = Y;  // [RP][N], reuses Y after step 3 has read it
+  const real* __restrict__ mid = pick(mids.p, blockIdx.y);
+  real* __restrict__ spec = pick(specs.p, blockIdx.y);
   const int t = threadIdx.x;
   const int64_t row0 = (int64_t)blockIdx.x * RP * 2;
+  real2 a[FS_AM(N1c, N2c)];
   if (t < RP * N2) {
-    const int r = t / N2, n2 = t % N2;
+    const int r = t / N2, n2 = t - r * N2;
     const int64_t ra = row0 + 2 * r, rb = ra + 1;
-    real2 a[N1];
+    with_radix<N1c>(N1, [&](auto rad) {
+      constexpr int R = decltype(rad)::value;
 #pragma unroll
-    for (int n1 = 0; n1 < N1; ++n1) {
-      const int i = n2 + N2 * n1;
-      a[n1] = mk2(ra < nrows_total ? mid[(size_t)ra * N + i] : real(0),
-                           rb < nrows_total ? mid[(size_t)rb * N + i] : real(0));
-    }
-    fs_step1<N1, N2>(a, n2, Y + r * YS, tw4);
+      for (int u = 0; u < R; ++u) {
+        const int i = n2 + N2 * u;
+        a[u] = mk2(ra < nrows ? mid[(size_t)ra * N + i] : real(0), rb < nrows ? mid[(size_t)rb * N + i] : real(0));
+      }
+      fs_step1<R, ST>(a, n2, N2, Y + r * YS, tw4);
+    });
   }
   __syncthreads();
-  {  // every thread reaches the barrier; RP * N1 <= FS_THREADS
-    const bool act = t < RP * N1;
-    const int r = t / N1, k1 = t % N1;
-    real2 a[N2];
-    if (act) fs_step3<N1, N2>(a, k1, Y + r * YS);
-    __syncthreads();
+  const bool act = t < RP * N1;  // every thread reaches the barriers
+  const int r = t / N1, k1 = t - r * N1;
+  if (act) with_radix<N2c>(N2, [&](auto rad) { fs_step3<decltype(rad)::value>(a, k1, Y + r * YS); });
+  __syncthreads();
+  if (act)
+    with_radix<N2c>(N2, [&](auto rad) {
 #pragma unroll
-    for (int k2 = 0; k2 < N2; ++k2)
-      if (act) X[r * N + k1 + N1 * k2] = a[k2];
-  }
+      for (int k2 = 0; k2 < decltype(rad)::value; ++k2) X[r * N + k1 + N1 * k2] = a[k2];
+    });
   __syncthreads();
   // separate the two real rows: A = (Z_b + conj Z_{N-b}) / 2, B = (Z_b - conj Z_{N-b}) / (2i)
-  constexpr int HALF = N / 2 + 1;
+  const int HALF = N / 2 + 1;
   for (int e = t; e < RP * 2 * HALF; e += FS_THREADS) {
     const int rr = e / HALF, b = e - rr * HALF;
     const int64_t row = row0 + rr;
-    if (row >= nrows_total) continue;
-    const int r = rr >> 1;
-    const real2 z1 = X[r * N + b];
-    const real2 z2 = X[r * N + (b == 0 ? 0 : N - b)];
-    real re, im;
-    if ((rr & 1) == 0) {
-      re = real(0.5) * (z1.x + z2.x);
-      im = real(0.5) * (z1.y - z2.y);
-    } else {
-      re = real(0.5) * (z1.y + z2.y);
-      im = real(-0.5) * (z1.x - z2.x);
-    }
-    spec[(size_t)row * g.sx + 2 * b] = re;
-    spec[(size_t)row * g.sx + 2 * b + 1] = im;
+    if (row >= nrows) continue;
+    const int rz = rr >> 1;
+    const real2 z1 = X[rz * N + b];
+    const real2 z2 = X[rz * N + (b == 0 ? 0 : N - b)];
+    real2 v;
+    if ((rr & 1) == 0) v = mk2(real(0.5) * (z1.x + z2.x), real(0.5) * (z1.y - z2.y));
+    else v = mk2(real(0.5) * (z1.y + z2.y), real(-0.5) * (z1.x - z2.x));
+    st2(spec, (size_t)row * g.sx + 2 * b, v);
   }
 }
 
-// inverse x pass (spec -> mid).  The modes are read straight from HBM into
+// Inverse x pass (spec -> mid).  The modes are read straight from HBM into
 // registers (the mirrored half from L1), the input operator applied on the
-// way.  Both transform passes are bound by L1 / shared-memory throughput, not
-// HBM, so no extra staging pass through shared memory is made.
-template <int N1, int N2, int OP>
-__global__ void __launch_bounds__(FS_THREADS) k4_inv_x(Geom g, int64_t nrows_total, const real2* __restrict__ tw4,
-                                                       const real* __restrict__ spec, real* __restrict__ mid,
-                                                       SpecIn<real> S) {
-  constexpr int N = N1 * N2, RP = FS_THREADS / (N1 > N2 ? N1 : N2), YS = N1 * (N2 + 1);
-  __shared__ real2 Y[RP * YS];
+// way.  SPEC_PAIR transforms the x and the y derivative of a spectrum from one
+// read of it.
+template <int N1c, int N2c, bool ST, int OP>
+__global__ void __launch_bounds__(FS_THREADS, sizeof(real) == 4 ? 5 : 3) k4_inv_x(Geom g, int n1, int n2_, int64_t nrows,
+                                                       const real2* __restrict__ tw4, SpecIn<real> S,
+                                                       Arr4<real> mids, Arr4<real> ymids) {
+  const int N1 = N1c ? N1c : n1, N2 = N2c ? N2c : n2_, N = N1 * N2;
+  const int RP = FS_THREADS / (N1 > N2 ? N1 : N2), YS = N1 * (N2 + 1);
+  extern __shared__ real2 sm[];
+  real2* Y = sm;
+  real2* Yd = sm + RP * YS;  // SPEC_PAIR: the y derivative
+  const int q = blockIdx.y;
   const int t = threadIdx.x;
   const int64_t row0 = (int64_t)blockIdx.x * RP * 2;
+  real2 a[FS_AM(N1c, N2c)];
   if (t < RP * N2) {
-    const int r = t / N2, n2 = t % N2;
+    const int r = t / N2, n2 = t - r * N2;
     const int64_t ra = row0 + 2 * r;
-    const bool valid = ra < nrows_total;  // then so is ra + 1: the row count is even
-    const int lev = (int)(ra / g.sy), jp = (int)(ra - (int64_t)lev * g.sy);
-    real2 a[N1];
+    const bool valid = ra < nrows;  // then so is ra + 1: the row count is even
+    const int l = (int)(ra / g.sy), jp = (int)(ra - (int64_t)l * g.sy);
+    with_radix<N1c>(N1, [&](auto rad) {
+      constexpr int R = decltype(rad)::value;
+      [[maybe_unused]] real2 b[OP == SPEC_PAIR ? R : 1];
 #pragma unroll
-    for (int n1 = 0; n1 < N1; ++n1) {
-      const int k = n2 + N2 * n1;
-      const int km = (2 * k <= N) ? k : N - k;
-      real2 A = mk2(real(0), real(0)), B = mk2(real(0), real(0));
-      if (valid) spec_pair<OP>(g, spec, S, ra, jp, lev, km, 2 * k <= N, A, B);
-      a[n1] = c2r_pack(A, B, k, N);
-    }
-    fs_step1<N1, N2>(a, n2, Y + r * YS, tw4);
+      for (int u = 0; u < R; ++u) {
+        const int k = n2 + N2 * u;
+        const int km = (2 * k <= N) ? k : N - k;
+        real2 A = mk2(real(0), real(0)), B = mk2(real(0), real(0));
+        if constexpr (OP == SPEC_PAIR) {
+          const int ca = jp * g.sx + 2 * km, cb = ca + g.sx;
+          real2 xa = A, xb = B;
+          if (valid) {
+            const size_t ea = (size_t)ra * g.sx + 2 * km;
+            xa = ld2(pick(S.x, q), ea);
+            xb = ld2(pick(S.x, q), ea + g.sx);
+          }
+          spec_op<SPEC_DY>(S, q, xa, xb, xa, xb, ca, cb, 2 * km, 0, A, B);
+          b[u] = c2r_pack(A, B, k, N);
+          spec_op<SPEC_DX>(S, q, xa, xb, xa, xb, ca, cb, 2 * km, 0, A, B);
+        } else {
+          if (valid) spec_pair<OP>(g, S, q, ra, jp, l, km, 2 * k <= N, A, B);
+        }
+        a[u] = c2r_pack(A, B, k, N);
+      }
+      fs_step1<R, ST>(a, n2, N2, Y + r * YS, tw4);
+      if constexpr (OP == SPEC_PAIR) fs_step1<R, ST>(b, n2, N2, Yd + r * YS, tw4);
+    });
   }
   __syncthreads();
   const real dn = real(1) / (real)N;
   if (t < RP * N1) {
-    const int r = t / N1, k1 = t % N1;
-    real2 a[N2];
-    fs_step3<N1, N2>(a, k1, Y + r * YS);
+    const int r = t / N1, k1 = t - r * N1;
     const int64_t ra = row0 + 2 * r, rb = ra + 1;
+    with_radix<N2c>(N2, [&](auto rad) {
+      constexpr int R = decltype(rad)::value;
+      auto out = [&](const real2* src, real* __restrict__ mid) {
+        fs_step3<R>(a, k1, src + r * YS);
 #pragma unroll
-    for (int k2 = 0; k2 < N2; ++k2) {
-      const int i = k1 + N1 * k2;  // conj(z) * dn: real part -> row A, imaginary part -> row B
-      if (ra < nrows_total) mid[(size_t)ra * N + i] = a[k2].x * dn;
-      if (rb < nrows_total) mid[(size_t)rb * N + i] = -a[k2].y * dn;
-    }
+        for (int k2 = 0; k2 < R; ++k2) {
+          const int i = k1 + N1 * k2;  // conj(z) * dn: real part -> row A, imaginary part -> row B
+          if (ra < nrows) mid[(size_t)ra * N + i] = a[k2].x * dn;
+          if (rb < nrows) mid[(size_t)rb * N + i] = -a[k2].y * dn;
+        }
+      };
+      out(Y, pick(mids.p, q));
+      if constexpr (OP == SPEC_PAIR) out(Yd, pick(ymids.p, q));
+    });
   }
 }
 
-// forward y pass (phys -> mid): one z level, 16 consecutive x columns
-// (8 complex columns) per CTA; thread order puts consecutive x on consecutive threads
-template <int N1, int N2>
-__global__ void __launch_bounds__(FS_THREADS) k4_fwd_y(Geom g, const real2* __restrict__ tw4,
-                                                       const real* __restrict__ phys, real* __restrict__ mid) {
-  // rows of Y and X are padded so the 8 column pairs of a warp access fall in
-  // distinct shared-memory banks
-  constexpr int N = N1 * N2, RP = 8, YS = N1 * (N2 + 1) + 1, XS = N + 1;
-  __shared__ real2 Y[RP * YS];
+// forward y pass (phys -> mid): one z level, FS_YV consecutive pairs of x
+// columns per CTA; thread order puts consecutive x on consecutive threads, so
+// a warp's access is whole 128-byte lines (FP32 with 8 pairs, half lines: 4
+// instead of 2 lines an access, and L1 is what bounds the y passes)
+template <int N1c, int N2c, bool ST>
+__global__ void __launch_bounds__(FS_YT) k4_fwd_y(Geom g, int n1, int n2_,
+                                                       const real2* __restrict__ tw4, Arr4<const real> physs,
+                                                       Arr4<real> mids) {
+  const int N1 = N1c ? N1c : n1, N2 = N2c ? N2c : n2_, N = N1 * N2;
+  constexpr int RP = FS_YV;
+  const int YS = N1 * (N2 + 1) + 1, XS = N + 1;
+  __shared__ real2 Y[fs_yvals(N1c, N2c)];
   real2* X = Y;  // [RP][XS], reuses Y after step 3 has read it
   const int t = threadIdx.x, Nx = g.Nx;
   const int x0 = blockIdx.x * 2 * RP, k = blockIdx.y;
-  const real* P = phys + (size_t)k * N * Nx;
+  const real* __restrict__ P = pick(physs.p, blockIdx.z) + (size_t)k * N * Nx;
+  real2 a[FS_AM(N1c, N2c)];
+  const int r = t % RP;
   if (t < RP * N2) {
-    const int r = t % RP, n2 = t / RP;
-    real2 a[N1];
+    const int n2 = t / RP;
+    const bool in = x0 + 2 * r < Nx;
+    with_radix<N1c>(N1, [&](auto rad) {
+      constexpr int R = decltype(rad)::value;
 #pragma unroll
-    for (int n1 = 0; n1 < N1; ++n1) {
-      const int j = n2 + N2 * n1;
-      a[n1] = *(const real2*)&P[(size_t)j * Nx + x0 + 2 * r];  // columns x0+2r (re), x0+2r+1 (im)
-    }
-    fs_step1<N1, N2>(a, n2, Y + r * YS, tw4);
+      for (int u = 0; u < R; ++u)  // columns x0+2r (re), x0+2r+1 (im)
+        a[u] = in ? ld2(P, (size_t)(n2 + N2 * u) * Nx + x0 + 2 * r) : mk2(real(0), real(0));
+      fs_step1<R, ST>(a, n2, N2, Y + r * YS, tw4);
+    });
   }
   __syncthreads();
-  {  // every thread reaches the barrier; RP * N1 <= FS_THREADS
-    const bool act = t < RP * N1;
-    const int r = t % RP, k1 = t / RP;
-    real2 a[N2];
-    if (act) fs_step3<N1, N2>(a, k1, Y + r * YS);
-    __syncthreads();
-#pragma unroll
-    for (int k2 = 0; k2 < N2; ++k2)
-      if (act) X[r * XS + k1 + N1 * k2] = a[k2];
-  }
+  const bool act = t < RP * N1;  // every thread reaches the barriers
+  const int k1 = t / RP;
+  if (act) with_radix<N2c>(N2, [&](auto rad) { fs_step3<decltype(rad)::value>(a, k1, Y + r * YS); });
   __syncthreads();
-  constexpr int HALF = N / 2 + 1;
-  real* M = mid + (size_t)k * g.sy * Nx;
-  for (int e = t; e < HALF * 2 * RP; e += FS_THREADS) {
-    const int a = e / (2 * RP), x = e - a * (2 * RP);
-    const int r = x >> 1;
-    const real2 z1 = X[r * XS + a];
-    const real2 z2 = X[r * XS + (a == 0 ? 0 : N - a)];
+  if (act)
+    with_radix<N2c>(N2, [&](auto rad) {
+#pragma unroll
+      for (int k2 = 0; k2 < decltype(rad)::value; ++k2) X[r * XS + k1 + N1 * k2] = a[k2];
+    });
+  __syncthreads();
+  const int HALF = N / 2 + 1;
+  real* __restrict__ M = pick(mids.p, blockIdx.z) + (size_t)k * g.sy * Nx;
+  for (int e = t; e < HALF * 2 * RP; e += blockDim.x) {
+    const int m = e / (2 * RP), x = e - m * (2 * RP);
+    if (x0 + x >= Nx) continue;
+    const int rz = x >> 1;
+    const real2 z1 = X[rz * XS + m];
+    const real2 z2 = X[rz * XS + (m == 0 ? 0 : N - m)];
     real re, im;
     if ((x & 1) == 0) {
       re = real(0.5) * (z1.x + z2.x);
@@ -630,177 +777,402 @@ __global__ void __launch_bounds__(FS_THREADS) k4_fwd_y(Geom g, const real2* __re
       re = real(0.5) * (z1.y + z2.y);
       im = real(-0.5) * (z1.x - z2.x);
     }
-    M[(size_t)(2 * a) * Nx + x0 + x] = re;
-    M[(size_t)(2 * a + 1) * Nx + x0 + x] = im;
+    M[(size_t)(2 * m) * Nx + x0 + x] = re;
+    M[(size_t)(2 * m + 1) * Nx + x0 + x] = im;
   }
 }
 
-// inverse y pass (mid -> phys)
-template <int N1, int N2, int OP>
-__global__ void __launch_bounds__(FS_THREADS) k4_inv_y(Geom g, const real2* __restrict__ tw4,
-                                                       const real* __restrict__ mid, real* __restrict__ phys,
-                                                       PhysOut<real> E) {
-  // rows of Y and X are padded so the 8 column pairs of a warp access fall in
-  // distinct shared-memory banks
-  constexpr int N = N1 * N2, RP = 8, YS = N1 * (N2 + 1) + 1;
-  __shared__ real2 Y[RP * YS];
+// step 1 of an inverse y pass: the modes of column pair r read from M (a level
+// of a mid array) into Y
+// (FEW: at most eight modes' loads in flight, for a caller with sums in registers)
+template <int N1c, bool ST, bool FEW = false>
+__device__ __forceinline__ void inv_y_step1(const Geom& g, int N1, int N2, int t, int x0, const real* __restrict__ M,
+                                            const real2* __restrict__ tw4, real2* a, real2* Y, int YS) {
+  const int N = N1 * N2, Nx = g.Nx;
+  const int r = t % FS_YV, n2 = t / FS_YV;
+  if (n2 >= N2) return;
+  const bool in = x0 + 2 * r < Nx;
+  with_radix<N1c>(N1, [&](auto rad) {
+    constexpr int R = decltype(rad)::value;
+#pragma unroll
+    for (int u = 0; u < R; ++u) {
+      if (FEW && u % (sizeof(real) == 4 ? 8 : 4) == 0) asm volatile("" ::: "memory");
+      const int kk = n2 + N2 * u;
+      const int km = (2 * kk <= N) ? kk : N - kk;
+      real2 re = mk2(real(0), real(0)), im = re;
+      if (in) {
+        const uint32_t o = (uint32_t)(2 * km * Nx + x0 + 2 * r);  // within the level
+        re = ld2(M, o);                                           // (A.re, B.re)
+        im = ld2(M, o + Nx);                                      // (A.im, B.im)
+      }
+      a[u] = c2r_pack(mk2(re.x, im.x), mk2(re.y, im.y), kk, N);
+    }
+    fs_step1<R, ST>(a, n2, N2, Y + r * YS, tw4);
+  });
+}
+
+// inverse y pass (mid -> phys); blockIdx.z is the array of the batch
+template <int N1c, int N2c, bool ST>
+__global__ void __launch_bounds__(FS_YT) k4_inv_y(Geom g, int n1, int n2_,
+                                                       const real2* __restrict__ tw4, Arr4<const real> mids,
+                                                       Arr4<real> physs) {
+  const int N1 = N1c ? N1c : n1, N2 = N2c ? N2c : n2_, N = N1 * N2;
+  constexpr int RP = FS_YV;
+  const int YS = N1 * (N2 + 1) + 1;
+  __shared__ real2 Y[fs_yvals(N1c, N2c)];
   const int t = threadIdx.x, Nx = g.Nx;
   const int x0 = blockIdx.x * 2 * RP, k = blockIdx.y;
-  const real* M = mid + (size_t)k * g.sy * Nx;
-  if (t < RP * N2) {
-    const int r = t % RP, n2 = t / RP;
-    real2 a[N1];
-#pragma unroll
-    for (int n1 = 0; n1 < N1; ++n1) {
-      const int kk = n2 + N2 * n1;
-      const int km = (2 * kk <= N) ? kk : N - kk;
-      const real2 re = *(const real2*)&M[(size_t)(2 * km) * Nx + x0 + 2 * r];      // (A.re, B.re)
-      const real2 im = *(const real2*)&M[(size_t)(2 * km + 1) * Nx + x0 + 2 * r];  // (A.im, B.im)
-      a[n1] = c2r_pack(mk2(re.x, im.x), mk2(re.y, im.y), kk, N);
-    }
-    fs_step1<N1, N2>(a, n2, Y + r * YS, tw4);
-  }
+  real2 a[FS_AM(N1c, N2c)];
+  inv_y_step1<N1c, ST>(g, N1, N2, t, x0, pick(mids.p, blockIdx.z) + (size_t)k * g.sy * Nx, tw4, a, Y, YS);
   __syncthreads();
   const real dn = real(1) / (real)N;
-  if (t < RP * N1) {
-    const int r = t % RP, k1 = t / RP;
-    real2 a[N2];
-    fs_step3<N1, N2>(a, k1, Y + r * YS);
+  const int r = t % RP, k1 = t / RP;
+  if (k1 < N1 && x0 + 2 * r < Nx) {
+    real* __restrict__ phys = pick(physs.p, blockIdx.z);
     const size_t p0 = (size_t)k * N * Nx + x0 + 2 * r;
+    with_radix<N2c>(N2, [&](auto rad) {
+      constexpr int R = decltype(rad)::value;
+      fs_step3<R>(a, k1, Y + r * YS);
 #pragma unroll
-    for (int k2 = 0; k2 < N2; ++k2)
-      phys_out2<OP>(E, phys, p0 + (size_t)(k1 + N1 * k2) * Nx, mk2(a[k2].x * dn, -a[k2].y * dn));
+      for (int k2 = 0; k2 < R; ++k2) st2(phys, p0 + (size_t)(k1 + N1 * k2) * Nx, mk2(a[k2].x * dn, -a[k2].y * dn));
+    });
   }
 }
 
-// launchers by split; return false if the split has no instantiation
-#define PMPIC_FS_CASES(CALL) \
-  if (n1 == 4 && n2 == 4) { CALL(4, 4); return true; } \
-  if (n1 == 8 && n2 == 4) { CALL(8, 4); return true; } \
-  if (n1 == 8 && n2 == 8) { CALL(8, 8); return true; } \
-  if (n1 == 16 && n2 == 8) { CALL(16, 8); return true; } \
-  if (n1 == 16 && n2 == 16) { CALL(16, 16); return true; } \
-  return false;
-
-bool fs_fwd_x(int n1, int n2, unsigned nb, cudaStream_t st, const Geom& g, int64_t nrows, const real2* tw4,
-              const real* mid, real* spec) {
-#define CALL(A, B) k4_fwd_x<A, B><<<nb, FS_THREADS, 0, st>>>(g, nrows, tw4, mid, spec)
-  PMPIC_FS_CASES(CALL)
-#undef CALL
-}
-template <int OP>
-bool fs_inv_x_op(int n1, int n2, unsigned nb, cudaStream_t st, const Geom& g, int64_t nrows, const real2* tw4,
-                 const real* spec, real* mid, const SpecIn<real>& S) {
-#define CALL(A, B) k4_inv_x<A, B, OP><<<nb, FS_THREADS, 0, st>>>(g, nrows, tw4, spec, mid, S)
-  PMPIC_FS_CASES(CALL)
-#undef CALL
-}
-bool fs_inv_x(int n1, int n2, unsigned nb, cudaStream_t st, const Geom& g, int64_t nrows, const real2* tw4,
-              const real* spec, real* mid, const SpecIn<real>& S) {
-  switch (S.op) {
-    case SPEC_DX: return fs_inv_x_op<SPEC_DX>(n1, n2, nb, st, g, nrows, tw4, spec, mid, S);
-    case SPEC_DY: return fs_inv_x_op<SPEC_DY>(n1, n2, nb, st, g, nrows, tw4, spec, mid, S);
-    case SPEC_FILT: return fs_inv_x_op<SPEC_FILT>(n1, n2, nb, st, g, nrows, tw4, spec, mid, S);
-    case SPEC_VEL: return fs_inv_x_op<SPEC_VEL>(n1, n2, nb, st, g, nrows, tw4, spec, mid, S);
-    default: return fs_inv_x_op<SPEC_PLAIN>(n1, n2, nb, st, g, nrows, tw4, spec, mid, S);
+// The inverse y passes of vorticity_tendency's eight derivatives with its
+// pointwise products, in one kernel: a CTA transforms the eight fields of its
+// columns one after the other and sums dp, then dq, in registers, so that no
+// derivative is stored and dp and dq are written once
+// (vorticity_tendency.F90:147-265, in its order of operations):
+//   dp = db/dy + p du/dx + q du/dy + r (q + dw/dx)
+//   dq = -db/dx + p dv/dx + q dv/dy + r (-p + dw/dy)
+//   dr = p dw/dx + q dw/dy - r du/dx - r dv/dy
+// dr's products come in another order than its sum: they wait in dr and two
+// work grids, each element with the thread that owns it.  The FP64 path's sums
+// would take half of the registers: they wait in dp and dq themselves.  The
+// exchange buffer alternates between two halves: one barrier a field.
+// Measured, ms per step of the whole tendency (its eight y passes as kernels
+// of their own before): FP32 256^3 5.1 -> 4.4, 128^3 0.96 -> 0.81; FP64 128^3
+// 1.58 -> 1.30 (sums in registers 1.47); 32^3 0.57 -> 0.20.
+struct VtArgs {
+  const real* m[8];  // x-transformed db/dy, du/dx, du/dy, dw/dx, db/dx, dv/dx, dv/dy, dw/dy
+  const real *P, *Q, *R;
+  real *DP, *DQ, *DR, *tmp, *tmp2;
+};
+template <int N1c, int N2c, bool ST>
+__global__ void __launch_bounds__(FS_YT, sizeof(real) == 4 ? 2 : 4) k4_vt_y(Geom g, int n1, int n2_,
+                                                      const real2* __restrict__ tw4, const __grid_constant__ VtArgs V) {
+  const int N1 = N1c ? N1c : n1, N2 = N2c ? N2c : n2_, N = N1 * N2;
+  constexpr int RP = FS_YV;
+  constexpr bool MEM = sizeof(real) == 8;  // the sums wait in memory
+  const int YS = N1 * (N2 + 1) + 1;
+  extern __shared__ real2 sm[];
+  const int t = threadIdx.x, Nx = g.Nx;
+  const int x0 = blockIdx.x * 2 * RP, k = blockIdx.y;
+  const int r = t % RP, k1 = t / RP;
+  const bool act = k1 < N1 && x0 + 2 * r < Nx;
+  const size_t lev = (size_t)k * N * Nx;
+  const uint32_t p0 = (uint32_t)(k1 * Nx + x0 + 2 * r);  // within the level
+  const real dn = real(1) / (real)N;
+  real2 a[FS_AM(N1c, N2c)], acc[MEM ? 1 : FS_AM(N1c, N2c)];
+#pragma unroll 1
+  for (int f = 0; f < 8; ++f) {
+    real2* Y = sm + (f & 1) * (RP * YS);
+    inv_y_step1<N1c, ST, true>(g, N1, N2, t, x0, V.m[f] + (size_t)k * g.sy * Nx, tw4, a, Y, YS);
+    __syncthreads();
+    if (!act) continue;
+    // field f adds X (Z + v) to the sum (Z: null, q or -p)
+    const real* X = f == 1 || f == 5 ? V.P : (f == 2 || f == 6 ? V.Q : V.R);
+    const real* Z = f == 3 ? V.Q : (f == 7 ? V.P : nullptr);
+    const real sz = f == 7 ? real(-1) : real(1);
+    real* sum = (f < 4 ? V.DP : V.DQ) + lev;
+    with_radix<N2c>(N2, [&](auto rad) {
+      constexpr int R = decltype(rad)::value;
+      fs_step3<R>(a, k1, Y + r * YS);
+#pragma unroll
+      for (int k2 = 0; k2 < R; ++k2) {
+        // (a few elements' loads in flight at a time: more would spill the sums)
+        if (k2 % (sizeof(real) == 4 ? 4 : 2) == 0) asm volatile("" ::: "memory");
+        const uint32_t o = p0 + (uint32_t)(N1 * k2 * Nx);
+        const real2 v = mk2(a[k2].x * dn, -a[k2].y * dn);
+        real2 s;
+        if ((f & 3) == 0) {
+          s = f == 0 ? v : mk2(-v.x, -v.y);
+        } else {
+          const real2 x = ld2(X + lev, o);
+          real2 u = v;
+          if (Z) {
+            const real2 z = ld2(Z + lev, o);
+            u = mk2(sz * z.x + v.x, sz * z.y + v.y);
+          }
+          s = MEM ? ld2(sum, o) : acc[MEM ? 0 : k2];
+          s = mk2(s.x + x.x * u.x, s.y + x.y * u.y);
+        }
+        if (!MEM) acc[MEM ? 0 : k2] = s;
+        if (MEM || (f & 3) == 3) st2(sum, o, s);
+        if (f == 1) {
+          const real2 w = ld2(V.R + lev, o);
+          st2(V.DR + lev, o, mk2(w.x * -v.x, w.y * -v.y));
+        } else if (f == 3) {
+          const real2 w = ld2(V.P + lev, o);
+          st2(V.tmp2 + lev, o, mk2(w.x * v.x, w.y * v.y));
+        } else if (f == 6) {
+          const real2 w = ld2(V.R + lev, o);
+          st2(V.tmp + lev, o, mk2(w.x * -v.x, w.y * -v.y));
+        } else if (f == 7) {
+          const real2 w = ld2(V.Q + lev, o), d0 = ld2(V.tmp2 + lev, o), d1 = ld2(V.DR + lev, o), d2 = ld2(V.tmp + lev, o);
+          st2(V.DR + lev, o, mk2(d0.x + w.x * v.x + d1.x + d2.x, d0.y + w.y * v.y + d1.y + d2.y));
+        }
+      }
+    });
   }
 }
-bool fs_fwd_y(int n1, int n2, dim3 gr, cudaStream_t st, const Geom& g, const real2* tw4, const real* phys,
-              real* mid) {
-#define CALL(A, B) k4_fwd_y<A, B><<<gr, FS_THREADS, 0, st>>>(g, tw4, phys, mid)
-  PMPIC_FS_CASES(CALL)
-#undef CALL
-}
-template <int OP>
-bool fs_inv_y_op(int n1, int n2, dim3 gr, cudaStream_t st, const Geom& g, const real2* tw4, const real* mid,
-                 real* phys, const PhysOut<real>& E) {
-#define CALL(A, B) k4_inv_y<A, B, OP><<<gr, FS_THREADS, 0, st>>>(g, tw4, mid, phys, E)
-  PMPIC_FS_CASES(CALL)
-#undef CALL
-}
-bool fs_inv_y(int n1, int n2, dim3 gr, cudaStream_t st, const Geom& g, const real2* tw4, const real* mid,
-              real* phys, const PhysOut<real>& E) {
-  switch (E.op) {
-    case PHYS_ADD_MUL: return fs_inv_y_op<PHYS_ADD_MUL>(n1, n2, gr, st, g, tw4, mid, phys, E);
-    case PHYS_ADD_MUL_SUM: return fs_inv_y_op<PHYS_ADD_MUL_SUM>(n1, n2, gr, st, g, tw4, mid, phys, E);
-    case PHYS_NEG_ADD_MUL: return fs_inv_y_op<PHYS_NEG_ADD_MUL>(n1, n2, gr, st, g, tw4, mid, phys, E);
-    case PHYS_DQ_DR: return fs_inv_y_op<PHYS_DQ_DR>(n1, n2, gr, st, g, tw4, mid, phys, E);
-    default: return fs_inv_y_op<PHYS_STORE>(n1, n2, gr, st, g, tw4, mid, phys, E);
+
+// f(N1c, N2c, ST) for a plan: the lengths 2^k, 3 2^k, 5 2^k and 9 2^k of common
+// grids at compile time, the others at run time (the same kernels, with the
+// registers of the largest radix: both transforms of a step took 0.67 ms at
+// 96^3 FP32 with the split known, 1.04 with it read at run time)
+constexpr int FS_SPLITS[][3] = {{4, 4, 0},  {8, 4, 0},   {8, 8, 0}, {16, 8, 0}, {16, 16, 0}, {4, 6, 1}, {4, 12, 1},
+                                {16, 6, 1}, {16, 12, 1}, {8, 5, 1}, {16, 5, 1}, {16, 10, 1}, {8, 9, 1}, {16, 9, 1}};
+constexpr int FS_NSPLIT = sizeof(FS_SPLITS) / sizeof(FS_SPLITS[0]);
+template <bool B>
+struct Flag {
+  static constexpr bool value = B;
+};
+template <int I = 0, class F>
+void fs_dispatch(int n1, int n2, bool st, F&& f) {
+  if constexpr (I == FS_NSPLIT) {
+    f(Rad<0>{}, Rad<0>{}, Flag<true>{});
+  } else {
+    constexpr int A = FS_SPLITS[I][0], B = FS_SPLITS[I][1];
+    constexpr bool S = FS_SPLITS[I][2] != 0;
+    if (n1 == A && n2 == B && st == S) f(Rad<A>{}, Rad<B>{}, Flag<S>{});
+    else fs_dispatch<I + 1>(n1, n2, st, f);
   }
 }
-#undef PMPIC_FS_CASES
 
-int fft_forward_impl(pmpic_ctx* ctx, const real* phys, real* spec, real* mid, const real2* tw) {
+// y then x pass of nb arrays (1..4); mids: nb scratch arrays
+int fft_forward_impl(pmpic_ctx* ctx, int nb, const real* const* phys, real* const* spec, real* const* mids,
+                     const real2* tw) {
   TimerScope ts(ctx, T_FFTF);
   const Geom& g = ctx->g;
   const FftPlan& px = ctx->plan_x;
   const FftPlan& py = ctx->plan_y;
   const real2* twy = tw + ctx->ftw_off_y;
+  cudaStream_t st = ctx->stream;
+  Arr4<const real> P{}, MC{};
+  Arr4<real> M{}, Sp{};
+  for (int b = 0; b < nb; ++b) {
+    P.p[b] = phys[b];
+    MC.p[b] = M.p[b] = mids[b];
+    Sp.p[b] = spec[b];
+  }
+  const int64_t nrows = (int64_t)g.nzp * g.sy;
   if (py.n1) {
-    fs_fwd_y(py.n1, py.n2, dim3(g.Nx / 16, g.nzp), ctx->stream, g, twy + py.tw4_off, phys, mid);
+    const dim3 gr((g.Nx + 2 * FS_YV - 1) / (2 * FS_YV), g.nzp, nb);
+    fs_dispatch(py.n1, py.n2, py.st, [&](auto a, auto b, auto c) {
+      k4_fwd_y<decltype(a)::value, decltype(b)::value, decltype(c)::value><<<gr, FS_YV * std::max(py.n1, py.n2), 0, st>>>(g, py.n1, py.n2, twy + py.tw4_off,
+                                                                                     P, M);
+    });
+    ++ctx->nlaunch;
   } else {
-    int txf = pick_txf(g.Nx);
-    size_t sm_y = sizeof(real2) * (size_t)(txf / 2) * g.Ny * 2;
-    dim3 gy(g.Nx / txf, g.nzp);
-    k_fwd_y<<<gy, FFT_THREADS, sm_y, ctx->stream>>>(g, txf, py, twy, phys, mid);
+    const int txf = pick_txf(g.Nx);
+    const size_t sm_y = sizeof(real2) * (size_t)(txf / 2) * g.Ny * 2;
+    for (int b = 0; b < nb; ++b) {
+      k_fwd_y<<<dim3(g.Nx / txf, g.nzp), FFT_THREADS, sm_y, st>>>(g, txf, py, twy, phys[b], mids[b]);
+      ++ctx->nlaunch;
+    }
   }
-  ++ctx->nlaunch;
-  int64_t nrows = (int64_t)g.nzp * g.sy;
   if (px.n1) {
-    const int rp = FS_THREADS / std::max(px.n1, px.n2);
-    fs_fwd_x(px.n1, px.n2, (unsigned)((nrows + 2 * rp - 1) / (2 * rp)), ctx->stream, g, nrows, tw + px.tw4_off,
-             mid, spec);
+    const int rp = fs_rows(px.n1, px.n2);
+    const dim3 gr((unsigned)((nrows + 2 * rp - 1) / (2 * rp)), nb);
+    fs_dispatch(px.n1, px.n2, px.st, [&](auto a, auto b, auto c) {
+      k4_fwd_x<decltype(a)::value, decltype(b)::value, decltype(c)::value><<<gr, FS_THREADS, 0, st>>>(g, px.n1, px.n2, nrows,
+                                                                                  tw + px.tw4_off, MC, Sp);
+    });
+    ++ctx->nlaunch;
   } else {
-    int rp = pick_rp(g.Nx);
-    size_t sm_x = sizeof(real2) * (size_t)rp * g.Nx * 2;
-    k_fwd_x<<<(unsigned)((nrows + 2 * rp - 1) / (2 * rp)), FFT_THREADS, sm_x, ctx->stream>>>(g, rp, nrows, px, tw,
-                                                                                          mid, spec);
+    const int rp = pick_rp(g.Nx);
+    const size_t sm_x = sizeof(real2) * (size_t)rp * g.Nx * 2;
+    for (int b = 0; b < nb; ++b) {
+      k_fwd_x<<<(unsigned)((nrows + 2 * rp - 1) / (2 * rp)), FFT_THREADS, sm_x, st>>>(g, rp, nrows, px, tw, mids[b],
+                                                                                       spec[b]);
+      ++ctx->nlaunch;
+    }
   }
-  ++ctx->nlaunch;
   PMPIC_CUDA(cudaGetLastError());
   return 0;
 }
 
-int fft_backward_impl(pmpic_ctx* ctx, const real* spec, real* phys, real* mid, const real2* tw, const SpecIn<real>& S,
-                      const PhysOut<real>& E) {
-  TimerScope ts(ctx, T_FFTI);
+// the inverse x pass of nb arrays (S.op, for SPEC_PAIR
+// their x derivatives into mids and their y derivatives into ymids)
+void inv_x_pass(pmpic_ctx* ctx, int nb, const SpecIn<real>& S, real* const* mids, real* const* ymids,
+                const real2* tw) {
   const Geom& g = ctx->g;
   const FftPlan& px = ctx->plan_x;
-  const FftPlan& py = ctx->plan_y;
-  int64_t nrows = (int64_t)g.nzp * g.sy;
+  cudaStream_t st = ctx->stream;
+  const int64_t nrows = (int64_t)g.nzp * g.sy;
   if (px.n1) {
-    const int rp = FS_THREADS / std::max(px.n1, px.n2);
-    fs_inv_x(px.n1, px.n2, (unsigned)((nrows + 2 * rp - 1) / (2 * rp)), ctx->stream, g, nrows, tw + px.tw4_off,
-             spec, mid, S);
-  } else {
-    int rp = pick_rp(g.Nx);
-    size_t sm_x = sizeof(real2) * (size_t)rp * g.Nx * 2;
-    k_inv_x<<<(unsigned)((nrows + 2 * rp - 1) / (2 * rp)), FFT_THREADS, sm_x, ctx->stream>>>(g, rp, nrows, px, tw,
-                                                                                          spec, mid, S);
+    Arr4<real> M{}, D{};
+    for (int b = 0; b < nb; ++b) {
+      M.p[b] = mids[b];
+      if (ymids) D.p[b] = ymids[b];
+    }
+    const int rp = fs_rows(px.n1, px.n2);
+    const dim3 gr((unsigned)((nrows + 2 * rp - 1) / (2 * rp)), nb);
+    const size_t sm = sizeof(real2) * (size_t)rp * px.n1 * (px.n2 + 1) * (S.op == SPEC_PAIR ? 2 : 1);
+    fs_dispatch(px.n1, px.n2, px.st, [&](auto a, auto b, auto c) {
+      constexpr int A = decltype(a)::value, B = decltype(b)::value;
+      constexpr bool C = decltype(c)::value;
+      auto go = [&](auto kern) {
+        kern<<<gr, FS_THREADS, sm, st>>>(g, px.n1, px.n2, nrows, tw + px.tw4_off, S, M, D);
+      };
+      switch (S.op) {
+        case SPEC_FILT: go(k4_inv_x<A, B, C, SPEC_FILT>); break;
+        case SPEC_VEL: go(k4_inv_x<A, B, C, SPEC_VEL>); break;
+        case SPEC_PAIR: go(k4_inv_x<A, B, C, SPEC_PAIR>); break;
+        default: go(k4_inv_x<A, B, C, SPEC_PLAIN>); break;
+      }
+    });
+    ++ctx->nlaunch;
+    return;
   }
+  const int rp = pick_rp(g.Nx);
+  const size_t sm = sizeof(real2) * (size_t)rp * g.Nx * 2;
+  const unsigned nblk = (unsigned)((nrows + 2 * rp - 1) / (2 * rp));
+  for (int b = 0; b < nb; ++b) {
+    auto go = [&](auto kern, real* mid) {
+      kern<<<nblk, FFT_THREADS, sm, st>>>(g, rp, nrows, px, tw, mid, S, b);
+      ++ctx->nlaunch;
+    };
+    switch (S.op) {
+      case SPEC_FILT: go(k_inv_x<SPEC_FILT>, mids[b]); break;
+      case SPEC_VEL: go(k_inv_x<SPEC_VEL>, mids[b]); break;
+      case SPEC_PAIR:
+        go(k_inv_x<SPEC_DX>, mids[b]);
+        go(k_inv_x<SPEC_DY>, ymids[b]);
+        break;
+      default: go(k_inv_x<SPEC_PLAIN>, mids[b]); break;
+    }
+  }
+}
+// one Stockham inverse y pass
+void inv_y_generic(pmpic_ctx* ctx, const real* mid, real* phys, const real2* twy,
+                   const PhysOut<real>& E) {
+  const Geom& g = ctx->g;
+  const int txf = pick_txf(g.Nx);
+  const size_t half = (size_t)g.Ny / 2 + 1;
+  const size_t sm = sizeof(real2) * std::max((size_t)(txf / 2) * g.Ny * 2, (size_t)(txf / 2) * g.Ny + txf * half);
+  k_inv_y<<<dim3(g.Nx / txf, g.nzp), FFT_THREADS, sm, ctx->stream>>>(g, txf, ctx->plan_y, twy, mid, phys, E);
   ++ctx->nlaunch;
+}
+
+// x then y pass of nb arrays (1..4), the input operator S.op applied on the way
+int fft_inverse_impl(pmpic_ctx* ctx, int nb, const SpecIn<real>& S, real* const* phys, real* const* mids,
+                     const real2* tw) {
+  TimerScope ts(ctx, T_FFTI);
+  const Geom& g = ctx->g;
+  const FftPlan& py = ctx->plan_y;
   const real2* twy = tw + ctx->ftw_off_y;
-  if (py.n1) {
-    fs_inv_y(py.n1, py.n2, dim3(g.Nx / 16, g.nzp), ctx->stream, g, twy + py.tw4_off, mid, phys, E);
-  } else {
-    int txf = pick_txf(g.Nx);
-    size_t half = (size_t)g.Ny / 2 + 1;
-    size_t sm_y = sizeof(real2) * std::max((size_t)(txf / 2) * g.Ny * 2, (size_t)(txf / 2) * g.Ny + txf * half);
-    dim3 gy(g.Nx / txf, g.nzp);
-    k_inv_y<<<gy, FFT_THREADS, sm_y, ctx->stream>>>(g, txf, py, twy, mid, phys, E);
+  Arr4<const real> M{};
+  Arr4<real> P{};
+  for (int b = 0; b < nb; ++b) {
+    M.p[b] = mids[b];
+    P.p[b] = phys[b];
   }
-  ++ctx->nlaunch;
+  inv_x_pass(ctx, nb, S, mids, nullptr, tw);
+  if (py.n1) {
+    const dim3 gr((g.Nx + 2 * FS_YV - 1) / (2 * FS_YV), g.nzp, nb);
+    fs_dispatch(py.n1, py.n2, py.st, [&](auto a, auto b, auto c) {
+      k4_inv_y<decltype(a)::value, decltype(b)::value, decltype(c)::value><<<gr, FS_YV * std::max(py.n1, py.n2), 0, ctx->stream>>>(g, py.n1, py.n2,
+                                                                                              twy + py.tw4_off, M, P);
+    });
+    ++ctx->nlaunch;
+  } else {
+    for (int b = 0; b < nb; ++b) inv_y_generic(ctx, mids[b], phys[b], twy, PhysOut<real>{});
+  }
   PMPIC_CUDA(cudaGetLastError());
   return 0;
 }
 
+// The eight inverse transforms of vorticity_tendency.F90:147-265 and its
+// products: S.x are the spectra of b, u, v, w, G the grids p, q, r and dp, dq,
+// dr, mids eight scratch arrays, work three grids.
+int fft_tendency_impl(pmpic_ctx* ctx, const SpecIn<real>& S, const real* const* pqr, real* const* dpqr,
+                      real* const* mids, real* const* work, const real2* tw) {
+  TimerScope ts(ctx, T_FFTI);
+  const Geom& g = ctx->g;
+  const FftPlan& py = ctx->plan_y;
+  const real2* twy = tw + ctx->ftw_off_y;
+  inv_x_pass(ctx, 4, S, mids, mids + 4, tw);  // the x, then the y derivatives of b, u, v, w
+  const real *bx = mids[0], *ux = mids[1], *vx = mids[2], *wx = mids[3];
+  const real *by = mids[4], *uy = mids[5], *vy = mids[6], *wy = mids[7];
+  if (py.n1) {
+    VtArgs V{{by, ux, uy, wx, bx, vx, vy, wy}, pqr[0], pqr[1], pqr[2], dpqr[0], dpqr[1], dpqr[2], work[0], work[1]};
+    const dim3 gr((g.Nx + 2 * FS_YV - 1) / (2 * FS_YV), g.nzp);
+    const size_t sm = sizeof(real2) * 2 * FS_YV * (size_t)(py.n1 * (py.n2 + 1) + 1);
+    fs_dispatch(py.n1, py.n2, py.st, [&](auto a, auto b, auto c) {
+      k4_vt_y<decltype(a)::value, decltype(b)::value, decltype(c)::value><<<gr, FS_YV * std::max(py.n1, py.n2), sm, ctx->stream>>>(
+          g, py.n1, py.n2, twy + py.tw4_off, V);
+    });
+    ++ctx->nlaunch;
+    PMPIC_CUDA(cudaGetLastError());
+    return 0;
+  }
+  const real *P = pqr[0], *Q = pqr[1], *R = pqr[2];
+  real *DP = dpqr[0], *DQ = dpqr[1], *DR = dpqr[2], *dudx = work[0], *dwdx = work[1], *dvdy = work[2];
+  auto epi = [](int op, int store, real* o, const real* a, const real* c) {
+    PhysOut<real> E;
+    E.op = op;
+    E.store = store;
+    E.o = o;
+    E.in[0] = a;
+    E.in[1] = c;
+    return E;
+  };
+  auto y = [&](const real* mid, real* phys, const PhysOut<real>& E) {
+    inv_y_generic(ctx, mid, phys, twy, E);
+  };
+  y(by, DP, PhysOut<real>{});
+  y(ux, dudx, epi(PHYS_ADD_MUL, 1, DP, P, nullptr));
+  y(uy, nullptr, epi(PHYS_ADD_MUL, 0, DP, Q, nullptr));
+  y(wx, dwdx, epi(PHYS_ADD_MUL_SUM, 1, DP, R, Q));
+  y(bx, DQ, PhysOut<real>{});
+  y(vx, nullptr, epi(PHYS_NEG_ADD_MUL, 0, DQ, P, nullptr));
+  y(vy, dvdy, epi(PHYS_ADD_MUL, 1, DQ, Q, nullptr));
+  PhysOut<real> last = epi(PHYS_DQ_DR, 0, DQ, R, P);
+  last.o2 = DR;
+  last.in[2] = Q;
+  last.in[3] = dwdx;
+  last.in[4] = dudx;
+  last.in[5] = dvdy;
+  y(wy, nullptr, last);
+  PMPIC_CUDA(cudaGetLastError());
+  return 0;
+}
 
-// shared-memory limits of the Stockham kernels (a property of each function on
-// the current device)
+// shared-memory limits of the kernels with dynamic shared memory (a property
+// of each function on the current device)
 cudaError_t fft_attributes() {
-  cudaError_t e = cudaFuncSetAttribute(k_fwd_y, cudaFuncAttributeMaxDynamicSharedMemorySize, 200 * 1024);
-  if (e == cudaSuccess) e = cudaFuncSetAttribute(k_inv_y, cudaFuncAttributeMaxDynamicSharedMemorySize, 200 * 1024);
-  if (e == cudaSuccess) e = cudaFuncSetAttribute(k_fwd_x, cudaFuncAttributeMaxDynamicSharedMemorySize, 200 * 1024);
-  if (e == cudaSuccess) e = cudaFuncSetAttribute(k_inv_x, cudaFuncAttributeMaxDynamicSharedMemorySize, 200 * 1024);
+  cudaError_t e = cudaSuccess;
+  auto set = [&](auto kern) {
+    if (e == cudaSuccess) e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, 200 * 1024);
+  };
+  set(k_fwd_y);
+  set(k_inv_y);
+  set(k_fwd_x);
+  set(k_inv_x<SPEC_PLAIN>);
+  set(k_inv_x<SPEC_DX>);
+  set(k_inv_x<SPEC_DY>);
+  set(k_inv_x<SPEC_FILT>);
+  set(k_inv_x<SPEC_VEL>);
+  for (int i = 0; i <= FS_NSPLIT; ++i)
+    fs_dispatch(i < FS_NSPLIT ? FS_SPLITS[i][0] : 0, i < FS_NSPLIT ? FS_SPLITS[i][1] : 0,
+                i < FS_NSPLIT && FS_SPLITS[i][2], [&](auto a, auto b, auto c) {
+      constexpr int A = decltype(a)::value, B = decltype(b)::value;
+      constexpr bool C = decltype(c)::value;
+      set(k4_inv_x<A, B, C, SPEC_PAIR>);
+      set(k4_vt_y<A, B, C>);
+    });
   return e;
 }

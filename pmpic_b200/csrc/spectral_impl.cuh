@@ -416,9 +416,13 @@ int vort2vel_spectral_impl(pmpic_ctx* ctx) {
   zero_mode_prepare(ctx);
   const unsigned nb = nblk(g.nspec, 256);
   const int cols = g.sx * g.sy;
-  if ((rc = fft_forward(ctx, G[PMPIC_GRID_P], a))) return rc;
-  if ((rc = fft_forward(ctx, G[PMPIC_GRID_Q], b))) return rc;
-  if ((rc = fft_forward(ctx, G[PMPIC_GRID_R], c))) return rc;
+  // scratch of the transforms: these spectral arrays hold nothing the inversion reads
+  real* mids[3] = {RP(ctx->fftmid), RP(ctx->sas), RP(ctx->sbs)};
+  {
+    const real* in[3] = {G[PMPIC_GRID_P], G[PMPIC_GRID_Q], G[PMPIC_GRID_R]};
+    real* out[3] = {a, b, c};
+    if ((rc = fft_forward(ctx, 3, in, out, mids))) return rc;
+  }
   const real hdzi = (real)(f4div(1.f, 2.f) / g.dz);
   k_div<<<nb, 256, 0, ctx->stream>>>(g, a, b, c, f, tab_kx(ctx), tab_ky(ctx), hdzi); ++ctx->nlaunch;
   if ((rc = spec_laplinv_impl(ctx, f, true))) return rc;
@@ -432,13 +436,16 @@ int vort2vel_spectral_impl(pmpic_ctx* ctx) {
   // :207-226: the top and bottom planes of a and b, then the filtered a, b, c
   // transformed back (the filter applied as the transform reads them)
   k_bt_planes<<<nblk(cols, 256), 256, 0, ctx->stream>>>(g, a, b, RP(ctx->bt)); ++ctx->nlaunch;
-  SpecIn<real> F;
-  F.op = SPEC_FILT;
-  F.tab = tab_filt(ctx);
-  const PhysOut<real> plain;
-  if ((rc = fft_backward(ctx, a, G[PMPIC_GRID_P], F, plain))) return rc;
-  if ((rc = fft_backward(ctx, b, G[PMPIC_GRID_Q], F, plain))) return rc;
-  if ((rc = fft_backward(ctx, c, G[PMPIC_GRID_R], F, plain))) return rc;
+  {
+    SpecIn<real> F;
+    F.op = SPEC_FILT;
+    F.filt = tab_filt(ctx);
+    F.x[0] = a;
+    F.x[1] = b;
+    F.x[2] = c;
+    real* out[3] = {G[PMPIC_GRID_P], G[PMPIC_GRID_Q], G[PMPIC_GRID_R]};
+    if ((rc = fft_inverse(ctx, 3, F, out, mids))) return rc;
+  }
   if ((rc = zero_mode_launch(ctx, a, b))) return rc;
   {
     real* abc[3] = {a, b, c};
@@ -449,17 +456,6 @@ int vort2vel_spectral_impl(pmpic_ctx* ctx) {
   const real* abot = RP(ctx->bt) + cols;
   const real* btop = RP(ctx->bt) + 2 * cols;
   const real* bbot = RP(ctx->bt) + 3 * cols;
-  // each velocity spectrum is formed as its inverse transform reads it, which
-  // also stores the filtered copy (u_s, v_s, w_s)
-  SpecIn<real> V;
-  V.op = SPEC_VEL;
-  V.e = e;
-  V.c = c;
-  V.a = a;
-  V.b = b;
-  V.kx = tab_kx(ctx);
-  V.ky = tab_ky(ctx);
-  V.filt = tab_filt(ctx);
   // dB/dz into e and dA/dz into d (:255, :284), in one launch
   {
     const real* zin[2] = {b, a};
@@ -468,71 +464,54 @@ int vort2vel_spectral_impl(pmpic_ctx* ctx) {
     const real* ztop[2] = {btop, atop};
     if ((rc = diffz_batch_impl(ctx, 2, zin, zout, zbot, ztop))) return rc;
   }
-  // u = dB/dz - dC/dy (:251-276)
-  V.vmode = 0;
-  V.fs = RP(ctx->spec[PMPIC_SPEC_U]);
-  V.zbar = ctx->zmode;
-  if ((rc = fft_backward(ctx, nullptr, G[PMPIC_GRID_U], V, plain))) return rc;
-  // v = dC/dx - dA/dz (:280-302)
-  V.e = d;
-  V.vmode = 1;
-  V.fs = RP(ctx->spec[PMPIC_SPEC_V]);
-  V.zbar = ctx->zmode + g.nzp;
-  if ((rc = fft_backward(ctx, nullptr, G[PMPIC_GRID_V], V, plain))) return rc;
-  // w = dA/dy - dB/dx (:306-320)
-  V.vmode = 2;
-  V.fs = RP(ctx->spec[PMPIC_SPEC_W]);
-  V.zbar = nullptr;
-  if ((rc = fft_backward(ctx, nullptr, G[PMPIC_GRID_W], V, plain))) return rc;
+  // u = dB/dz - dC/dy (:251-276), v = dC/dx - dA/dz (:280-302) and
+  // w = dA/dy - dB/dx (:306-320): each velocity spectrum is formed as its
+  // inverse transform reads it, which also stores the filtered copy (u_s, v_s, w_s)
+  {
+    SpecIn<real> V;
+    V.op = SPEC_VEL;
+    V.x[0] = e;
+    V.y[0] = c;
+    V.x[1] = d;
+    V.y[1] = c;
+    V.x[2] = a;
+    V.y[2] = b;
+    V.fs[0] = RP(ctx->spec[PMPIC_SPEC_U]);
+    V.fs[1] = RP(ctx->spec[PMPIC_SPEC_V]);
+    V.fs[2] = RP(ctx->spec[PMPIC_SPEC_W]);
+    V.zbar[0] = ctx->zmode;
+    V.zbar[1] = ctx->zmode + g.nzp;
+    V.kx = tab_kx(ctx);
+    V.ky = tab_ky(ctx);
+    V.filt = tab_filt(ctx);
+    real* out[3] = {G[PMPIC_GRID_U], G[PMPIC_GRID_V], G[PMPIC_GRID_W]};
+    if ((rc = fft_inverse(ctx, 3, V, out, mids))) return rc;
+  }
   PMPIC_CUDA(cudaGetLastError());
   return 0;
 }
 
-// vorticity_tendency.F90:147-265 (grid B holds par2grid(btot) on entry).
-// Each spectral derivative is applied as its inverse transform reads it, and
-// each pointwise update of dp, dq, dr as the transform writes its result, so
-// no derivative spectrum or intermediate grid makes a round trip through HBM.
+// vorticity_tendency.F90:147-265 (grid B holds par2grid(btot) on entry).  The
+// x pass reads each of the spectra of b, u, v, w once and transforms its two
+// derivatives; the y pass forms dp, dq and dr as it transforms them.
 int vorticity_tendency_grids_impl(pmpic_ctx* ctx) {
   int rc;
-  real *bs = RP(ctx->sbs);
   real* const* G = (real* const*)ctx->grid;
-  real *DP = G[PMPIC_GRID_DP], *DQ = G[PMPIC_GRID_DQ], *DR = G[PMPIC_GRID_DR];
-  const real *P = G[PMPIC_GRID_P], *Q = G[PMPIC_GRID_Q], *R = G[PMPIC_GRID_R];
-  real *dudx = RP(ctx->gwork[0]), *dwdx = RP(ctx->gwork[1]), *dvdy = RP(ctx->gwork[2]);
-  const real *us = RP(ctx->spec[PMPIC_SPEC_U]), *vs = RP(ctx->spec[PMPIC_SPEC_V]), *ws = RP(ctx->spec[PMPIC_SPEC_W]);
-  SpecIn<real> DX, DY;
-  DX.op = SPEC_DX;
-  DX.tab = tab_kx(ctx);
-  DY.op = SPEC_DY;
-  DY.tab = tab_ky(ctx);
-  auto epi = [](int op, int store, real* o, const real* a, const real* b) {
-    PhysOut<real> E;
-    E.op = op;
-    E.store = store;
-    E.o = o;
-    E.in[0] = a;
-    E.in[1] = b;
-    return E;
-  };
-  const PhysOut<real> plain;
-  if ((rc = fft_forward(ctx, G[PMPIC_GRID_B], bs))) return rc;
-  // dp = db/dy + p du/dx + q du/dy + r (q + dw/dx)
-  if ((rc = fft_backward(ctx, bs, DP, DY, plain))) return rc;
-  if ((rc = fft_backward(ctx, us, dudx, DX, epi(PHYS_ADD_MUL, 1, DP, P, nullptr)))) return rc;
-  if ((rc = fft_backward(ctx, us, nullptr, DY, epi(PHYS_ADD_MUL, 0, DP, Q, nullptr)))) return rc;
-  if ((rc = fft_backward(ctx, ws, dwdx, DX, epi(PHYS_ADD_MUL_SUM, 1, DP, R, Q)))) return rc;
-  // dq = -db/dx + p dv/dx + q dv/dy + r (-p + dw/dy)
-  if ((rc = fft_backward(ctx, bs, DQ, DX, plain))) return rc;
-  if ((rc = fft_backward(ctx, vs, nullptr, DX, epi(PHYS_NEG_ADD_MUL, 0, DQ, P, nullptr)))) return rc;
-  if ((rc = fft_backward(ctx, vs, dvdy, DY, epi(PHYS_ADD_MUL, 1, DQ, Q, nullptr)))) return rc;
-  // ... and, with dw/dy, dr = p dw/dx + q dw/dy - r du/dx - r dv/dy
-  PhysOut<real> last = epi(PHYS_DQ_DR, 0, DQ, R, P);
-  last.o2 = DR;
-  last.in[2] = Q;
-  last.in[3] = dwdx;
-  last.in[4] = dudx;
-  last.in[5] = dvdy;
-  if ((rc = fft_backward(ctx, ws, nullptr, DY, last))) return rc;
+  real* bs = RP(ctx->sbs);
+  const real* bg = G[PMPIC_GRID_B];
+  real* mid0 = RP(ctx->fftmid);
+  if ((rc = fft_forward(ctx, 1, &bg, &bs, &mid0))) return rc;
+  SpecIn<real> S;
+  S.op = SPEC_PAIR;
+  S.x[0] = bs;
+  for (int q = 0; q < 3; ++q) S.x[q + 1] = RP(ctx->spec[PMPIC_SPEC_U + q]);
+  S.kx = tab_kx(ctx);
+  S.ky = tab_ky(ctx);
+  const real* pqr[3] = {G[PMPIC_GRID_P], G[PMPIC_GRID_Q], G[PMPIC_GRID_R]};
+  real* dpqr[3] = {G[PMPIC_GRID_DP], G[PMPIC_GRID_DQ], G[PMPIC_GRID_DR]};
+  real* mids[8] = {mid0, RP(ctx->sas), RP(ctx->sa), RP(ctx->sb), RP(ctx->sc), RP(ctx->sd), RP(ctx->se), RP(ctx->sf)};
+  real* work[3] = {RP(ctx->gwork[0]), RP(ctx->gwork[1]), RP(ctx->gwork[2])};
+  if ((rc = fft_tendency(ctx, S, pqr, dpqr, mids, work))) return rc;
   PMPIC_CUDA(cudaGetLastError());
   return 0;
 }
