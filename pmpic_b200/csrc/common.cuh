@@ -335,6 +335,9 @@ struct pmpic_ctx {
   double* fftmid;            // (Nz+1) x (Ny+2) x Nx
   double* ftw;               // twiddle tables (x plan first, then y plan), double2
   float* ftw32;              // the same twiddles as float2 (mixed-precision form)
+  double* zrec;              // reciprocal pivots of the FP64 inversion's z solves (spectral.cu)
+  void* zwork;               // the inversion's columns when they exceed shared memory (else null)
+  int64_t zwork_bytes;
   float* wn32;               // FP32 kx, ky, k2, filter tables and diffz factors
   double* hsum;              // FP64 horizontal sums of p and q per level (mixed form's zero mode)
   double* stage64;           // mixed form: FP64 staging of host transfers (stage_n values, two halves)
@@ -392,25 +395,18 @@ int prop_download(pmpic_ctx* ctx, int pid, int64_t off, int64_t n, double* dst);
 // fft.cu
 // Elementwise operators fused into the inverse transforms' x pass, applied to
 // the spectra as they are read.  Each repeats the arithmetic of the separate
-// operator kernel it replaces (same operands, same order).  x, y, fs and zbar
-// are per array of a batch.
+// operator (same operands, same order).  x: the arrays of a batch.
 enum SpecOpKind {
   SPEC_PLAIN = 0,
   SPEC_DX,    // diffx (fft_ops.F90:266-295) of x
   SPEC_DY,    // diffy (fft_ops.F90:366-394) of x
-  SPEC_FILT,  // the de-aliasing filter (fft_ops.F90:176-197) of x
-  SPEC_VEL,   // the velocity spectra of vort2vel.F90:254-315: u, v from x = e and y = c, w from x = a and
-              // y = b; the filtered copy is stored to fs; zbar is the mean flow of u and v
   SPEC_PAIR   // both derivatives of x, from one read
 };
 template <class R>
 struct SpecIn {
   int op = SPEC_PLAIN;
-  const R* x[4] = {};
-  const R* y[4] = {};
-  R* fs[4] = {};
-  const double* zbar[2] = {};
-  const R *kx = nullptr, *ky = nullptr, *filt = nullptr;
+  const R* x[6] = {};
+  const R *kx = nullptr, *ky = nullptr;
 };
 // the pointwise operators on the output of a Stockham inverse y pass
 // (vorticity_tendency's products; the four-step lengths have k4_vt_y)
@@ -430,7 +426,7 @@ struct PhysOut {
   const R* in[6] = {};
 };
 int fft_init(pmpic_ctx* ctx);
-// Forward and inverse transforms of nb arrays (1..4) at once.  mids: nb
+// Forward and inverse transforms of nb arrays (1..6) at once.  mids: nb
 // scratch arrays of nspec values that are no input or output of the call.
 int fft_forward(pmpic_ctx* ctx, int nb, const double* const* phys, double* const* spec, double* const* mids);
 int fft_forward(pmpic_ctx* ctx, int nb, const float* const* phys, float* const* spec, float* const* mids);

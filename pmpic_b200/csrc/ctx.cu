@@ -121,7 +121,7 @@ void free_all(pmpic_ctx* c) {
   void* ptrs[] = {c->parcels, c->rowpart,  c->gpack,    c->lapcp,    c->cell,     c->del,       c->gspare,     c->sorted,    c->cell_count, c->cell_start, c->cell_fill, c->keep,
                   c->aux,     c->aux2,     c->dir,       c->swapbuf,    c->scan_tmp,   c->npercell,  c->newslot,
                   c->newportion, c->sa,    c->sb,        c->sc,         c->sd,         c->se,        c->sf,
-                  c->sas,     c->sbs,      c->sscratch,  c->fftmid,     c->ftw,        c->ftw32,      c->wn32,       c->hsum,       c->stage64,        c->kx,        c->ky,
+                  c->sas,     c->sbs,      c->sscratch,  c->fftmid,     c->ftw,        c->ftw32,      c->wn32,       c->hsum,       c->zrec,       c->zwork,       c->stage64,        c->kx,        c->ky,
                   c->k2,      c->filt,     c->bt,        c->zmode,      c->csum,       c->near,       c->whint,      c->dinfo};
   for (void* p : ptrs)
     if (p) cudaFree(p);

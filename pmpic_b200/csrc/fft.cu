@@ -126,7 +126,7 @@ using real2 = double2;
 __host__ __device__ __forceinline__ double2 mk2(double a, double b) { return make_double2(a, b); }
 #include "fft_impl.cuh"
 }  // namespace f64
-cudaError_t fft_attributes32();
+cudaError_t fft_attributes32(const FftPlan& px, const FftPlan& py);
 
 int fft_init(pmpic_ctx* ctx) {
   std::vector<int> tmp;
@@ -152,8 +152,7 @@ int fft_init(pmpic_ctx* ctx) {
   ctx->plan_x = px;
   ctx->plan_y = py;
   // per device (the attribute is a property of the function on the current device)
-  PMPIC_CUDA(f64::fft_attributes());
-  PMPIC_CUDA(fft_attributes32());
+  PMPIC_CUDA(ctx->mixed ? fft_attributes32(px, py) : f64::fft_attributes(px, py));
   return 0;
 }
 

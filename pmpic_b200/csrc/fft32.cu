@@ -16,7 +16,7 @@ __host__ __device__ __forceinline__ float2 mk2(float a, float b) { return make_f
 #include "fft_impl.cuh"
 }  // namespace f32
 
-cudaError_t fft_attributes32() { return f32::fft_attributes(); }
+cudaError_t fft_attributes32(const FftPlan& px, const FftPlan& py) { return f32::fft_attributes(px, py); }
 int fft_forward(pmpic_ctx* ctx, int nb, const float* const* phys, float* const* spec, float* const* mids) {
   return f32::fft_forward_impl(ctx, nb, phys, spec, mids, (const float2*)ctx->ftw32);
 }

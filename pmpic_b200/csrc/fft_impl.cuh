@@ -199,89 +199,37 @@ __device__ __forceinline__ real2 c2r_pack(real2 A, real2 B, int k, int n) {
 // Ny + 2 is even, so row ra holds the even y' index jp (the real part of a y
 // mode) and row ra + 1 the odd one of the same level lev; each value is the
 // element pair (2 km, 2 km + 1) of its row.  The operators repeat the
-// arithmetic of diffx, diffy and the filter (spectral_impl.cuh: dx_of, dy_of,
-// k_filter) and the velocity spectra of vort2vel.F90:251-320 (e - diffy(c), diffx(c) - e,
-// diffy(a) - diffx(b); the mean flow in mode (0, 0) of u and v).
-// own: this thread reads mode km unmirrored, so it stores the filtered
-// velocity spectrum of SPEC_VEL.
+// arithmetic of diffx and diffy (spectral.cu: dx_of, dy_of).
 __device__ __forceinline__ real2 ld2(const real* __restrict__ p, size_t i) { return *(const real2*)&p[i]; }
 __device__ __forceinline__ void st2(real* __restrict__ p, size_t i, real2 v) { *(real2*)&p[i] = v; }
 
 // one array of a batch (selected without indexing the parameter arrays: no local copy)
 template <class T>
-__device__ __forceinline__ T* pick(T* const (&p)[4], int b) {
-  return b == 0 ? p[0] : (b == 1 ? p[1] : (b == 2 ? p[2] : p[3]));
+__device__ __forceinline__ T* pick(T* const (&p)[6], int b) {
+  return b < 3 ? (b == 0 ? p[0] : (b == 1 ? p[1] : p[2])) : (b == 3 ? p[3] : (b == 4 ? p[4] : p[5]));
 }
 
-// The operator on the values of one spectral element pair of rows ra (xa)
-// and ra + 1 (xb); ca, cb are their spectral columns, lev their level.  For
-// SPEC_VEL the batch index q is the component (0 u, 1 v, 2 w), x is e (u, v)
-// or a (w) and y is c (u, v) or b (w).  The wavenumber tables are laid out
-// like the spectra but kx depends on the x index alone and ky on the row
-// alone, so kx is read from row 0 (x2 = 2 km, the pair's x index) and ky from
-// column 0 of rows ca - x2 and cb - x2: the same values, one small
+// The operator on the values of one spectral element pair of rows ra (xa) and
+// ra + 1 (xb); ca, cb are their spectral columns, x2 = 2 km the pair's x
+// index.  The wavenumber tables are laid out like the spectra but kx depends
+// on the x index alone and ky on the row alone, so kx is read from row 0 and
+// ky from column 0 of rows ca - x2 and cb - x2: the same values, one small
 // L1-resident row or a per-thread constant instead of a second spectrum-sized
 // read per element.
 template <int OP>
-__device__ __forceinline__ void spec_op(const SpecIn<real>& S, int q, real2 xa, real2 xb, real2 ya, real2 yb, int ca,
-                                        int cb, int x2, int lev, real2& A, real2& B) {
-  auto kxp = [&](const real* t) { return ld2(t, x2); };
-  auto kyp = [&](const real* t, int c) { const real v = t[c - x2]; return mk2(v, v); };
-  if constexpr (OP == SPEC_VEL) {
-    if (q == 0) {  // f = e - diffy(c), f(:,1,1) = ubar
-      const real2 ta = kyp(S.ky, ca), tb = kyp(S.ky, cb);
-      A = mk2(xa.x - (real(-1) * yb.x) * ta.x, xa.y - (real(-1) * yb.y) * ta.y);
-      B = mk2(xb.x - ya.x * tb.x, xb.y - ya.y * tb.y);
-      if (ca == 0) A.x = (real)S.zbar[0][lev];
-    } else if (q == 1) {  // f = diffx(c) - e, f(:,1,1) = vbar
-      const real2 ta = kxp(S.kx), tb = ta;
-      A = mk2((real(-1) * ya.y) * ta.x - xa.x, ya.x * ta.y - xa.y);
-      B = mk2((real(-1) * yb.y) * tb.x - xb.x, yb.x * tb.y - xb.y);
-      if (ca == 0) A.x = (real)S.zbar[1][lev];
-    } else {  // f = diffy(a) - diffx(b)
-      const real2 ya2 = kyp(S.ky, ca), yb2 = kyp(S.ky, cb), xa2 = kxp(S.kx), xb2 = xa2;
-      A = mk2((real(-1) * xb.x) * ya2.x - (real(-1) * ya.y) * xa2.x, (real(-1) * xb.y) * ya2.y - ya.x * xa2.y);
-      B = mk2(xa.x * yb2.x - (real(-1) * yb.y) * xb2.x, xa.y * yb2.y - yb.x * xb2.y);
-    }
-  } else if constexpr (OP == SPEC_DX) {
-    const real2 ta = kxp(S.kx), tb = ta;
-    A = mk2((real(-1) * xa.y) * ta.x, xa.x * ta.y);
-    B = mk2((real(-1) * xb.y) * tb.x, xb.x * tb.y);
+__device__ __forceinline__ void spec_op(const SpecIn<real>& S, real2 xa, real2 xb, int ca, int cb, int x2, real2& A,
+                                        real2& B) {
+  if constexpr (OP == SPEC_DX) {
+    const real2 t = ld2(S.kx, x2);
+    A = mk2((real(-1) * xa.y) * t.x, xa.x * t.y);
+    B = mk2((real(-1) * xb.y) * t.x, xb.x * t.y);
   } else if constexpr (OP == SPEC_DY) {
-    const real2 ta = kyp(S.ky, ca), tb = kyp(S.ky, cb);
-    A = mk2((real(-1) * xb.x) * ta.x, (real(-1) * xb.y) * ta.y);
-    B = mk2(xa.x * tb.x, xa.y * tb.y);
-  } else if constexpr (OP == SPEC_FILT) {
-    const real2 ta = ld2(S.filt, ca), tb = ld2(S.filt, cb);
-    A = mk2(xa.x * ta.x, xa.y * ta.y);
-    B = mk2(xb.x * tb.x, xb.y * tb.y);
+    const real ta = S.ky[ca - x2], tb = S.ky[cb - x2];
+    A = mk2((real(-1) * xb.x) * ta, (real(-1) * xb.y) * ta);
+    B = mk2(xa.x * tb, xa.y * tb);
   } else {
     A = xa;
     B = xb;
-  }
-}
-// the filtered copy of a velocity spectrum pair (SPEC_VEL), at elements ea, eb
-__device__ __forceinline__ void vel_store(const SpecIn<real>& S, int q, size_t ea, size_t eb, int ca, int cb, real2 A,
-                                          real2 B) {
-  const real2 fa = ld2(S.filt, ca), fb = ld2(S.filt, cb);
-  real* fs = pick(S.fs, q);
-  st2(fs, ea, mk2(A.x * fa.x, A.y * fa.y));
-  st2(fs, eb, mk2(B.x * fb.x, B.y * fb.y));
-}
-// the operator's inputs of the element pair read from global memory
-template <int OP>
-__device__ __forceinline__ void spec_pair(const Geom& g, const SpecIn<real>& S, int q, int64_t ra, int jp, int lev,
-                                          int km, bool own, real2& A, real2& B) {
-  const size_t ea = (size_t)ra * g.sx + 2 * km, eb = ea + g.sx;
-  const int ca = jp * g.sx + 2 * km, cb = ca + g.sx;  // spectral columns of elements ea, eb
-  const real* x = pick(S.x, q);
-  if constexpr (OP == SPEC_VEL) {
-    const real* y = pick(S.y, q);
-    spec_op<OP>(S, q, ld2(x, ea), ld2(x, eb), ld2(y, ea), ld2(y, eb), ca, cb, 2 * km, lev, A, B);
-    if (own) vel_store(S, q, ea, eb, ca, cb, A, B);
-  } else {
-    const real2 a = ld2(x, ea), b = ld2(x, eb);
-    spec_op<OP>(S, q, a, b, a, b, ca, cb, 2 * km, lev, A, B);
   }
 }
 
@@ -339,8 +287,10 @@ __global__ void __launch_bounds__(FFT_THREADS) k_inv_x(Geom g, int RP, int64_t n
     int64_t ra = row0 + 2 * r;
     real2 A = mk2(real(0), real(0)), B = mk2(real(0), real(0));
     if (ra < nrows_total) {
-      const int l = (int)(ra / g.sy);
-      spec_pair<OP>(g, S, q, ra, (int)(ra - (int64_t)l * g.sy), l, km, 2 * k <= Nx, A, B);
+      const int jp = (int)(ra % g.sy), ca = jp * g.sx + 2 * km;
+      const size_t ea = (size_t)ra * g.sx + 2 * km;
+      const real* x = pick(S.x, q);
+      spec_op<OP>(S, ld2(x, ea), ld2(x, ea + g.sx), ca, ca + g.sx, 2 * km, A, B);
     }
     b0[r * Nx + k] = c2r_pack(A, B, k, Nx);
   }
@@ -591,15 +541,15 @@ __host__ __device__ constexpr int fs_xvals(int n1, int n2) { return n1 == 0 ? 8 
 __host__ __device__ constexpr int fs_yvals(int n1, int n2) { return n1 == 0 ? FS_YV * (16 * 17 + 1) : FS_YV * (n1 * (n2 + 1) + 1); }
 
 template <class T>
-struct Arr4 {
-  T* p[4];
+struct Arr6 {
+  T* p[6];
 };
 
 // forward x pass (mid -> spec): pairs of real rows; blockIdx.y is the array of the batch
 template <int N1c, int N2c, bool ST>
 __global__ void __launch_bounds__(FS_THREADS) k4_fwd_x(Geom g, int n1, int n2_, int64_t nrows,
-                                                       const real2* __restrict__ tw4, Arr4<const real> mids,
-                                                       Arr4<real> specs) {
+                                                       const real2* __restrict__ tw4, Arr6<const real> mids,
+                                                       Arr6<real> specs) {
   const int N1 = N1c ? N1c : n1, N2 = N2c ? N2c : n2_, N = N1 * N2;
   const int RP = FS_THREADS / (N1 > N2 ? N1 : N2), YS = N1 * (N2 + 1);
   __shared__ real2 Y[fs_xvals(N1c, N2c)];
@@ -656,7 +606,7 @@ __global__ void __launch_bounds__(FS_THREADS) k4_fwd_x(Geom g, int n1, int n2_, 
 template <int N1c, int N2c, bool ST, int OP>
 __global__ void __launch_bounds__(FS_THREADS, sizeof(real) == 4 ? 5 : 3) k4_inv_x(Geom g, int n1, int n2_, int64_t nrows,
                                                        const real2* __restrict__ tw4, SpecIn<real> S,
-                                                       Arr4<real> mids, Arr4<real> ymids) {
+                                                       Arr6<real> mids, Arr6<real> ymids) {
   const int N1 = N1c ? N1c : n1, N2 = N2c ? N2c : n2_, N = N1 * N2;
   const int RP = FS_THREADS / (N1 > N2 ? N1 : N2), YS = N1 * (N2 + 1);
   extern __shared__ real2 sm[];
@@ -670,7 +620,8 @@ __global__ void __launch_bounds__(FS_THREADS, sizeof(real) == 4 ? 5 : 3) k4_inv_
     const int r = t / N2, n2 = t - r * N2;
     const int64_t ra = row0 + 2 * r;
     const bool valid = ra < nrows;  // then so is ra + 1: the row count is even
-    const int l = (int)(ra / g.sy), jp = (int)(ra - (int64_t)l * g.sy);
+    const int jp = (int)(ra % g.sy);
+    const real* __restrict__ x = pick(S.x, q);
     with_radix<N1c>(N1, [&](auto rad) {
       constexpr int R = decltype(rad)::value;
       [[maybe_unused]] real2 b[OP == SPEC_PAIR ? R : 1];
@@ -678,20 +629,19 @@ __global__ void __launch_bounds__(FS_THREADS, sizeof(real) == 4 ? 5 : 3) k4_inv_
       for (int u = 0; u < R; ++u) {
         const int k = n2 + N2 * u;
         const int km = (2 * k <= N) ? k : N - k;
-        real2 A = mk2(real(0), real(0)), B = mk2(real(0), real(0));
+        const int ca = jp * g.sx + 2 * km, cb = ca + g.sx;
+        real2 xa = mk2(real(0), real(0)), xb = xa, A, B;
+        if (valid) {
+          const size_t ea = (size_t)ra * g.sx + 2 * km;
+          xa = ld2(x, ea);
+          xb = ld2(x, ea + g.sx);
+        }
         if constexpr (OP == SPEC_PAIR) {
-          const int ca = jp * g.sx + 2 * km, cb = ca + g.sx;
-          real2 xa = A, xb = B;
-          if (valid) {
-            const size_t ea = (size_t)ra * g.sx + 2 * km;
-            xa = ld2(pick(S.x, q), ea);
-            xb = ld2(pick(S.x, q), ea + g.sx);
-          }
-          spec_op<SPEC_DY>(S, q, xa, xb, xa, xb, ca, cb, 2 * km, 0, A, B);
+          spec_op<SPEC_DY>(S, xa, xb, ca, cb, 2 * km, A, B);
           b[u] = c2r_pack(A, B, k, N);
-          spec_op<SPEC_DX>(S, q, xa, xb, xa, xb, ca, cb, 2 * km, 0, A, B);
+          spec_op<SPEC_DX>(S, xa, xb, ca, cb, 2 * km, A, B);
         } else {
-          if (valid) spec_pair<OP>(g, S, q, ra, jp, l, km, 2 * k <= N, A, B);
+          spec_op<OP>(S, xa, xb, ca, cb, 2 * km, A, B);
         }
         a[u] = c2r_pack(A, B, k, N);
       }
@@ -727,8 +677,8 @@ __global__ void __launch_bounds__(FS_THREADS, sizeof(real) == 4 ? 5 : 3) k4_inv_
 // instead of 2 lines an access, and L1 is what bounds the y passes)
 template <int N1c, int N2c, bool ST>
 __global__ void __launch_bounds__(FS_YT) k4_fwd_y(Geom g, int n1, int n2_,
-                                                       const real2* __restrict__ tw4, Arr4<const real> physs,
-                                                       Arr4<real> mids) {
+                                                       const real2* __restrict__ tw4, Arr6<const real> physs,
+                                                       Arr6<real> mids) {
   const int N1 = N1c ? N1c : n1, N2 = N2c ? N2c : n2_, N = N1 * N2;
   constexpr int RP = FS_YV;
   const int YS = N1 * (N2 + 1) + 1, XS = N + 1;
@@ -814,8 +764,8 @@ __device__ __forceinline__ void inv_y_step1(const Geom& g, int N1, int N2, int t
 // inverse y pass (mid -> phys); blockIdx.z is the array of the batch
 template <int N1c, int N2c, bool ST>
 __global__ void __launch_bounds__(FS_YT) k4_inv_y(Geom g, int n1, int n2_,
-                                                       const real2* __restrict__ tw4, Arr4<const real> mids,
-                                                       Arr4<real> physs) {
+                                                       const real2* __restrict__ tw4, Arr6<const real> mids,
+                                                       Arr6<real> physs) {
   const int N1 = N1c ? N1c : n1, N2 = N2c ? N2c : n2_, N = N1 * N2;
   constexpr int RP = FS_YV;
   const int YS = N1 * (N2 + 1) + 1;
@@ -951,7 +901,7 @@ void fs_dispatch(int n1, int n2, bool st, F&& f) {
   }
 }
 
-// y then x pass of nb arrays (1..4); mids: nb scratch arrays
+// y then x pass of nb arrays (1..6); mids: nb scratch arrays
 int fft_forward_impl(pmpic_ctx* ctx, int nb, const real* const* phys, real* const* spec, real* const* mids,
                      const real2* tw) {
   TimerScope ts(ctx, T_FFTF);
@@ -960,8 +910,8 @@ int fft_forward_impl(pmpic_ctx* ctx, int nb, const real* const* phys, real* cons
   const FftPlan& py = ctx->plan_y;
   const real2* twy = tw + ctx->ftw_off_y;
   cudaStream_t st = ctx->stream;
-  Arr4<const real> P{}, MC{};
-  Arr4<real> M{}, Sp{};
+  Arr6<const real> P{}, MC{};
+  Arr6<real> M{}, Sp{};
   for (int b = 0; b < nb; ++b) {
     P.p[b] = phys[b];
     MC.p[b] = M.p[b] = mids[b];
@@ -1013,7 +963,7 @@ void inv_x_pass(pmpic_ctx* ctx, int nb, const SpecIn<real>& S, real* const* mids
   cudaStream_t st = ctx->stream;
   const int64_t nrows = (int64_t)g.nzp * g.sy;
   if (px.n1) {
-    Arr4<real> M{}, D{};
+    Arr6<real> M{}, D{};
     for (int b = 0; b < nb; ++b) {
       M.p[b] = mids[b];
       if (ymids) D.p[b] = ymids[b];
@@ -1028,8 +978,6 @@ void inv_x_pass(pmpic_ctx* ctx, int nb, const SpecIn<real>& S, real* const* mids
         kern<<<gr, FS_THREADS, sm, st>>>(g, px.n1, px.n2, nrows, tw + px.tw4_off, S, M, D);
       };
       switch (S.op) {
-        case SPEC_FILT: go(k4_inv_x<A, B, C, SPEC_FILT>); break;
-        case SPEC_VEL: go(k4_inv_x<A, B, C, SPEC_VEL>); break;
         case SPEC_PAIR: go(k4_inv_x<A, B, C, SPEC_PAIR>); break;
         default: go(k4_inv_x<A, B, C, SPEC_PLAIN>); break;
       }
@@ -1046,8 +994,6 @@ void inv_x_pass(pmpic_ctx* ctx, int nb, const SpecIn<real>& S, real* const* mids
       ++ctx->nlaunch;
     };
     switch (S.op) {
-      case SPEC_FILT: go(k_inv_x<SPEC_FILT>, mids[b]); break;
-      case SPEC_VEL: go(k_inv_x<SPEC_VEL>, mids[b]); break;
       case SPEC_PAIR:
         go(k_inv_x<SPEC_DX>, mids[b]);
         go(k_inv_x<SPEC_DY>, ymids[b]);
@@ -1067,15 +1013,15 @@ void inv_y_generic(pmpic_ctx* ctx, const real* mid, real* phys, const real2* twy
   ++ctx->nlaunch;
 }
 
-// x then y pass of nb arrays (1..4), the input operator S.op applied on the way
+// x then y pass of nb arrays (1..6), the input operator S.op applied on the way
 int fft_inverse_impl(pmpic_ctx* ctx, int nb, const SpecIn<real>& S, real* const* phys, real* const* mids,
                      const real2* tw) {
   TimerScope ts(ctx, T_FFTI);
   const Geom& g = ctx->g;
   const FftPlan& py = ctx->plan_y;
   const real2* twy = tw + ctx->ftw_off_y;
-  Arr4<const real> M{};
-  Arr4<real> P{};
+  Arr6<const real> M{};
+  Arr6<real> P{};
   for (int b = 0; b < nb; ++b) {
     M.p[b] = mids[b];
     P.p[b] = phys[b];
@@ -1151,28 +1097,30 @@ int fft_tendency_impl(pmpic_ctx* ctx, const SpecIn<real>& S, const real* const* 
   return 0;
 }
 
-// shared-memory limits of the kernels with dynamic shared memory (a property
-// of each function on the current device)
-cudaError_t fft_attributes() {
+// shared-memory limits of the kernels with dynamic shared memory that the
+// context's lengths use (a property of each function on the current device)
+cudaError_t fft_attributes(const FftPlan& px, const FftPlan& py) {
   cudaError_t e = cudaSuccess;
   auto set = [&](auto kern) {
     if (e == cudaSuccess) e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, 200 * 1024);
   };
-  set(k_fwd_y);
-  set(k_inv_y);
-  set(k_fwd_x);
-  set(k_inv_x<SPEC_PLAIN>);
-  set(k_inv_x<SPEC_DX>);
-  set(k_inv_x<SPEC_DY>);
-  set(k_inv_x<SPEC_FILT>);
-  set(k_inv_x<SPEC_VEL>);
-  for (int i = 0; i <= FS_NSPLIT; ++i)
-    fs_dispatch(i < FS_NSPLIT ? FS_SPLITS[i][0] : 0, i < FS_NSPLIT ? FS_SPLITS[i][1] : 0,
-                i < FS_NSPLIT && FS_SPLITS[i][2], [&](auto a, auto b, auto c) {
-      constexpr int A = decltype(a)::value, B = decltype(b)::value;
-      constexpr bool C = decltype(c)::value;
-      set(k4_inv_x<A, B, C, SPEC_PAIR>);
-      set(k4_vt_y<A, B, C>);
+  if (px.n1) {
+    fs_dispatch(px.n1, px.n2, px.st, [&](auto a, auto b, auto c) {
+      set(k4_inv_x<decltype(a)::value, decltype(b)::value, decltype(c)::value, SPEC_PAIR>);
     });
+  } else {
+    set(k_fwd_x);
+    set(k_inv_x<SPEC_PLAIN>);
+    set(k_inv_x<SPEC_DX>);
+    set(k_inv_x<SPEC_DY>);
+  }
+  if (py.n1) {
+    fs_dispatch(py.n1, py.n2, py.st, [&](auto a, auto b, auto c) {
+      set(k4_vt_y<decltype(a)::value, decltype(b)::value, decltype(c)::value>);
+    });
+  } else {
+    set(k_fwd_y);
+    set(k_inv_y);
+  }
   return e;
 }

@@ -8,12 +8,14 @@
 // components/vorticity_tendency/src/vorticity_tendency.F90:147-265.
 //
 // Spectral arrays are (Nz+1) x (Ny+2) x (Nx+2), x' fastest; a column is one
-// (j', i') pair over all z.  Elementwise operators are one thread per element;
-// the compact z operators are one thread per column running the reference's
-// Thomas recurrence with identical arithmetic (no FMA contraction), so they
-// reproduce the CPU results bit for bit on identical inputs.
+// (j', i') pair over all z.  The operators as the C ABI offers them run one
+// thread per element or, the compact z operators, one per column, with the
+// reference's recurrence and arithmetic (no FMA contraction), so that they
+// reproduce the CPU results bit for bit on identical inputs; the inversion's
+// spectral part is one kernel (spectral_impl.cuh: k_invert).
 #include <cuda_runtime.h>
 
+#include <cmath>
 #include <vector>
 
 #include "common.cuh"
@@ -100,6 +102,210 @@ __global__ void __launch_bounds__(256) k_hsum2(Geom g, const float* __restrict__
   }
 }
 
+// ---- elementwise spectral operators --------------------------------------------
+// The wavenumber tables are laid out like a spectral level, but kx depends on
+// the x index ip alone and ky on the row jp alone: kx is read from row 0
+// (kx[ip]) and ky from column 0 (ky[jp * sx]), the same values.
+// diffx (fft_ops.F90:266-295): out(i) = -in(i+1) kx, out(i+1) = in(i) kx
+__device__ __forceinline__ double dx_of(const double* in, int64_t e, int ip, const double* kx) {
+  return (ip & 1) == 0 ? (-1.0 * in[e + 1]) * kx[ip] : in[e - 1] * kx[ip];
+}
+// diffy (fft_ops.F90:366-394)
+__device__ __forceinline__ double dy_of(const double* in, int64_t e, int jp, int sx, const double* ky) {
+  return (jp & 1) == 0 ? (-1.0 * in[e + sx]) * ky[jp * sx] : in[e - sx] * ky[jp * sx];
+}
+
+struct EwIdx {
+  int64_t e;
+  int col, ip, jp, k;
+};
+__device__ __forceinline__ bool ew_index(const Geom& g, EwIdx& x) {
+  int64_t e = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
+  if (e >= g.nspec) return false;
+  int cols = g.sx * g.sy;
+  x.e = e;
+  x.k = (int)(e / cols);
+  x.col = (int)(e - (int64_t)x.k * cols);
+  x.jp = x.col / g.sx;
+  x.ip = x.col - x.jp * g.sx;
+  return true;
+}
+
+__global__ void k_diffx(Geom g, const double* __restrict__ in, double* __restrict__ out, const double* __restrict__ kx) {
+  EwIdx x;
+  if (!ew_index(g, x)) return;
+  out[x.e] = dx_of(in, x.e, x.ip, kx);
+}
+__global__ void k_diffy(Geom g, const double* __restrict__ in, double* __restrict__ out, const double* __restrict__ ky) {
+  EwIdx x;
+  if (!ew_index(g, x)) return;
+  out[x.e] = dy_of(in, x.e, x.jp, g.sx, ky);
+}
+__global__ void k_filter(Geom g, const double* __restrict__ in, double* __restrict__ out,
+                         const double* __restrict__ filt) {
+  EwIdx x;
+  if (!ew_index(g, x)) return;
+  out[x.e] = in[x.e] * filt[x.col];
+}
+
+// ---- compact z operators ----------------------------------------------------------
+// (the C ABI's diffz and laplinv; the inversion runs them inside k_invert)
+// The z recurrences run one thread per spectral column.  The Thomas factors
+// (pivots den and ratios cp of fft_ops.F90:620-656) depend only on the level
+// and, for laplinv, on the column's wavenumber: they are tables built once at set-up that repeat the
+// sequential recurrence exactly; the right-hand side is still divided by the
+// pivot, so the results keep the reference's bits.
+
+// diffz (fft_ops.F90:419-483).  The tridiagonal coefficients are the same for
+// every column, so the Thomas factors (cp and the pivots) are computed once on
+// the host with the reference's arithmetic and passed in.
+__global__ void k_diffz(Geom g, const double* __restrict__ f, double* __restrict__ out,
+                        const double* __restrict__ bot, const double* __restrict__ top,
+                        const double* __restrict__ coef /* a[nz], den[nz], cp[nz] */, double a1) {
+  const int col = blockIdx.x * blockDim.x + threadIdx.x;
+  const int cols = g.sx * g.sy;
+  if (col >= cols) return;
+  const int nz = g.nzp;
+  const uint32_t cs = (uint32_t)cols;  // level offsets fit 32 bits (the spectral grid is < 2^31)
+  const double* A = coef;
+  const double* DEN = coef + nz;
+  const double* CP = coef + 2 * nz;
+  const double dz = (double)g.dz;
+  const bool bt = bot != nullptr;
+  // forward sweep: f'(1) = d(1)/den(1); f'(i) = (d(i) - a(i) f'(i-1)) / den(i).
+  // The loads of each batch of ZB levels are issued before its recurrence, so
+  // the loop waits on one memory latency per batch, not per level.
+  constexpr int ZB = 8;
+  double fm = f[col], f0 = f[cs + col];
+  double d1 = bt ? f0 / dz - a1 * bot[col] * dz : 0.0;
+  double prev = d1 / DEN[0];
+  out[col] = prev;
+  for (int kb = 1; kb < nz - 1; kb += ZB) {
+    double fb[ZB];
+#pragma unroll
+    for (int u = 0; u < ZB; ++u)
+      if (kb + u < nz - 1) fb[u] = f[(uint32_t)(kb + u + 1) * cs + col];
+#pragma unroll
+    for (int u = 0; u < ZB; ++u) {
+      const int k = kb + u;
+      if (k >= nz - 1) break;
+      double d = (fb[u] - fm) / 2.0 / dz;
+      prev = (d - A[k] * prev) / DEN[k];
+      out[(uint32_t)k * cs + col] = prev;
+      fm = f0;
+      f0 = fb[u];
+    }
+  }
+  {
+    int k = nz - 1;
+    double dn = bt ? -fm / dz + a1 * top[col] * dz : 0.0;  // fm = f(nz-1)
+    prev = (dn - A[k] * prev) / DEN[k];
+    out[(uint32_t)k * cs + col] = prev;
+  }
+  // back substitution: f(i) = f(i) - cp(i+1) f(i+1)
+  double nxt = prev;
+  for (int kb = nz - 2; kb >= 0; kb -= ZB) {
+    double ob[ZB];
+#pragma unroll
+    for (int u = 0; u < ZB; ++u)
+      if (kb - u >= 0) ob[u] = out[(uint32_t)(kb - u) * cs + col];
+#pragma unroll
+    for (int u = 0; u < ZB; ++u) {
+      const int k = kb - u;
+      if (k < 0) break;
+      nxt = ob[u] - CP[k + 1] * nxt;
+      out[(uint32_t)k * cs + col] = nxt;
+    }
+  }
+}
+
+// laplinv (fft_ops.F90:505-601), in place, one thread per column; columns with
+// k2 == 0 keep their input (:567).  The Thomas factors of a column depend on
+// its wavenumber only, shared by the four columns (2a-1..2a, 2b-1..2b) of one
+// mode (a, b): tab holds, per boundary form (f0, df0), the pivots (FP32: their
+// reciprocals) and then the ratios cp, each [level][mode], built at set-up
+// (laplinv_tables).
+// blockIdx.y selects one of up to three arrays solved in the same launch
+__global__ void k_laplinv(Geom g, double* __restrict__ f, int df0, const double* __restrict__ tab,
+                          const double* __restrict__ k2) {
+  const int col = blockIdx.x * blockDim.x + threadIdx.x;
+  const int cols = g.sx * g.sy;
+  if (col >= cols) return;
+  const double kk = k2[col];
+  if (kk == 0) return;
+  const int nz = g.nzp;
+  const int64_t cs = cols;
+  const int nmode = (g.sx >> 1) * (g.sy >> 1);
+  const int jp = col / g.sx, ip = col - jp * g.sx;
+  const double* __restrict__ DEN = tab + ((size_t)(2 * df0) * nmode + (jp >> 1) * (g.sx >> 1) + (ip >> 1)) * nz;
+  const double* __restrict__ CP = DEN + (size_t)nz * nmode;
+  const double f16 = (double)f4div(1.f, 6.f), f13 = (double)f4div(1.f, 3.f), f112 = (double)f4div(1.f, 12.f), f56 = (double)f4div(5.f, 6.f);
+  const double dz = (double)g.dz;
+  const double idz2 = 1.0 / dz / dz;
+  const double ai = idz2 - f112 * kk;
+  double an;
+  double fm, f0, fp;
+  f0 = f[col];
+  fp = f[cs + col];
+  double d;
+  if (!df0) {
+    d = 0.0;
+    an = 0.0;
+  } else {
+    d = f13 * f0 + f16 * fp;
+    an = idz2 - f16 * kk;
+  }
+  // tridiagonal (fft_ops.F90:620-656) with the tabulated factors
+  double prev = d / DEN[0];
+  f[col] = prev;
+  // loads of each batch of ZB levels first, then its recurrence (one memory
+  // latency per batch); the batch reads f above the levels it overwrites
+  constexpr int ZB = 4;
+  for (int kb = 1; kb < nz; kb += ZB) {
+    double fb[ZB], db[ZB];
+#pragma unroll
+    for (int u = 0; u < ZB; ++u) {
+      if (kb + u < nz - 1) fb[u] = f[(int64_t)(kb + u + 1) * cs + col];
+      if (kb + u < nz) db[u] = DEN[kb + u];
+    }
+#pragma unroll
+    for (int u = 0; u < ZB; ++u) {
+      const int k = kb + u;
+      if (k >= nz) break;
+      fm = f0;
+      f0 = fp;
+      double a;
+      if (k < nz - 1) {
+        fp = fb[u];
+        a = ai;
+        d = f112 * fm + f56 * f0 + f112 * fp;
+      } else {
+        a = an;
+        d = df0 ? f13 * f0 + f16 * fm : 0.0;
+      }
+      prev = (d - a * prev) / db[u];
+      f[(int64_t)k * cs + col] = prev;
+    }
+  }
+  double nxt = prev;
+  for (int kb = nz - 2; kb >= 0; kb -= ZB) {
+    double fb[ZB], cb[ZB];
+#pragma unroll
+    for (int u = 0; u < ZB; ++u)
+      if (kb - u >= 0) {
+        fb[u] = f[(int64_t)(kb - u) * cs + col];
+        cb[u] = CP[kb - u + 1];
+      }
+#pragma unroll
+    for (int u = 0; u < ZB; ++u) {
+      const int k = kb - u;
+      if (k < 0) break;
+      nxt = fb[u] - cb[u] * nxt;
+      f[(int64_t)k * cs + col] = nxt;
+    }
+  }
+}
+
 // dt rule (vort2vel.F90:329-372, vorticity_tendency.F90:277-313), one thread
 __global__ void k_dt_velocity(Geom g, DevInfo* info, double dtmax) {
   double umax = sqrt(info->umax2), vmax = sqrt(info->vmax2), wmax = sqrt(info->wmax2);
@@ -160,7 +366,8 @@ int diffz_coef(pmpic_ctx* ctx, bool bt, std::vector<double>& out) {
 // sequential recurrence, with the coefficients and the operation order of
 // k_laplinv (FP64: the same IEEE operations, so the device's FP64 solve keeps
 // its bits; FP32 form: 1/den and cp rounded to FP32).  Layout per form:
-// den[nz][nmodes], then cp[nz][nmodes].  A zero pivot is the reference's
+// den[nmodes][nz], then cp[nmodes][nz]: a column's recurrence reads its own
+// lines one after the other.  A zero pivot is the reference's
 // abort (:642-645).
 int laplinv_tables(pmpic_ctx* ctx, const double* k2cols) {
   const Geom& g = ctx->g;
@@ -188,15 +395,15 @@ int laplinv_tables(pmpic_ctx* ctx, const double* k2cols) {
           bn = -idz2 - f13 * kk;
         }
         double den = b1, cprev = c1;
-        DEN[m] = den;
+        DEN[(size_t)m * nz] = den;
         for (int k = 1; k < nz; ++k) {
           const double ak = k < nz - 1 ? ai : an, bk = k < nz - 1 ? bi : bn, ck = k < nz - 1 ? ci : 0.0;
           const double cp = cprev / den;
           den = bk - ak * cp;
           if (den == 0 && kk != 0)
             return set_error(ctx, PMPIC_ERR_ZERO_PIVOT, "zero pivot in tridiagonal solver (laplinv)");
-          CP[(size_t)k * nmode + m] = cp;
-          DEN[(size_t)k * nmode + m] = den;
+          CP[(size_t)m * nz + k] = cp;
+          DEN[(size_t)m * nz + k] = den;
           cprev = ck;
         }
       }
@@ -217,21 +424,42 @@ int laplinv_tables(pmpic_ctx* ctx, const double* k2cols) {
   return 0;
 }
 
+// a table of the inversion's recurrences: reciprocal pivots (FP64: with the
+// residual rl of the rounded reciprocal) and ratios cp, level by level
+template <class R>
+struct ZTab {
+  const R *r, *rl, *cp;
+};
+// rh = 1 / den rounded, rl = its residual: n rh + n rl is n / den before rounding
+__global__ void k_recip(int64_t n, const double* __restrict__ den, double* __restrict__ rh, double* __restrict__ rl) {
+  const int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
+  if (i >= n) return;
+  const double d = den[i], h = 1.0 / d;
+  rh[i] = h;
+  rl[i] = __dmul_rn(__fma_rn(-d, h, 1.0), h);
+}
+
 namespace f64 {
 using real = double;
 inline const double* tab_kx(pmpic_ctx* c) { return c->kx; }
 inline const double* tab_ky(pmpic_ctx* c) { return c->ky; }
 inline const double* tab_k2(pmpic_ctx* c) { return c->k2; }
 inline const double* tab_filt(pmpic_ctx* c) { return c->filt; }
-inline const double* tab_diffz(pmpic_ctx* c, int which) { return c->sscratch + c->g.nspec + which * 3 * c->g.nzp; }
-inline void zero_mode_prepare(pmpic_ctx*) {}
-// the mean flow from the columns kx = ky = 0 of the filtered a and b
-// (vort2vel.F90:230-241); a, b are the unfiltered spectra
-inline int zero_mode_launch(pmpic_ctx* ctx, const double* a, const double* b) {
-  const Geom& g = ctx->g;
-  k_zmode<<<1, 256, sizeof(double) * 4 * g.nzp, ctx->stream>>>(g, a, b, (int64_t)g.sx * g.sy, ctx->filt, ctx->zmode); ++ctx->nlaunch;
-  return 0;
+inline const double* diffz_tab(pmpic_ctx* c, int which) { return c->sscratch + c->g.nspec + which * 3 * c->g.nzp; }
+// ctx->zrec: per diffz form, then per laplinv form, rh and rl
+inline ZTab<double> dz_tab(pmpic_ctx* c, int which) {
+  const int nz = c->g.nzp;
+  const double* r = c->zrec + which * 2 * nz;
+  return {r, r + nz, diffz_tab(c, which) + 2 * nz};
 }
+inline ZTab<double> lap_tab(pmpic_ctx* c, int form) {
+  const int64_t n = (int64_t)(c->g.sx >> 1) * (c->g.sy >> 1) * c->g.nzp;
+  const double* r = c->zrec + 4 * c->g.nzp + form * 2 * n;
+  return {r, r + n, c->lapcp + (2 * form + 1) * n};
+}
+// the mean flow (vort2vel.F90:230-241) comes from the zero modes of the
+// corrected spectra, inside k_invert
+inline int zero_mode(pmpic_ctx*) { return 0; }
 #include "spectral_impl.cuh"
 }  // namespace f64
 
@@ -241,17 +469,24 @@ inline const float* tab_kx(pmpic_ctx* c) { return c->wn32; }
 inline const float* tab_ky(pmpic_ctx* c) { return c->wn32 + (size_t)c->g.sx * c->g.sy; }
 inline const float* tab_k2(pmpic_ctx* c) { return c->wn32 + 2 * (size_t)c->g.sx * c->g.sy; }
 inline const float* tab_filt(pmpic_ctx* c) { return c->wn32 + 3 * (size_t)c->g.sx * c->g.sy; }
-inline const float* tab_diffz(pmpic_ctx* c, int which) { return c->wn32 + 4 * (size_t)c->g.sx * c->g.sy + which * 3 * c->g.nzp; }
+inline ZTab<float> dz_tab(pmpic_ctx* c, int which) {
+  const int nz = c->g.nzp;
+  const float* t = c->wn32 + 4 * (size_t)c->g.sx * c->g.sy + which * 3 * nz;
+  return {t + nz, nullptr, t + 2 * nz};
+}
+inline ZTab<float> lap_tab(pmpic_ctx* c, int form) {
+  const int64_t n = (int64_t)(c->g.sx >> 1) * (c->g.sy >> 1) * c->g.nzp;
+  const float* t = (const float*)c->lapcp + 2 * form * n;
+  return {t, nullptr, t + n};
+}
 // the zero mode stays FP64: horizontal sums of the gridded p and q taken in
 // FP64 before the FP32 transforms, then the FP64 mean-flow integral
-inline void zero_mode_prepare(pmpic_ctx* ctx) {
+inline int zero_mode(pmpic_ctx* ctx) {
   const Geom& g = ctx->g;
   k_hsum2<<<g.nzp, 256, 0, ctx->stream>>>(g, (const float*)ctx->grid[PMPIC_GRID_P], (const float*)ctx->grid[PMPIC_GRID_Q],
                                           ctx->hsum); ++ctx->nlaunch;
-}
-inline int zero_mode_launch(pmpic_ctx* ctx, const float*, const float*) {
-  const Geom& g = ctx->g;
   k_zmode<<<1, 256, sizeof(double) * 4 * g.nzp, ctx->stream>>>(g, ctx->hsum, ctx->hsum + g.nzp, 1, nullptr, ctx->zmode); ++ctx->nlaunch;
+  PMPIC_CUDA(cudaGetLastError());
   return 0;
 }
 #include "spectral_impl.cuh"
@@ -286,16 +521,52 @@ int spectral_init(pmpic_ctx* ctx) {
   PMPIC_CUDA(cudaMalloc(&ctx->wn32, sizeof(float) * t32.size()));
   PMPIC_CUDA(cudaMemcpy(ctx->wn32, t32.data(), sizeof(float) * t32.size(), cudaMemcpyHostToDevice));
   PMPIC_CUDA(cudaMalloc(&ctx->hsum, sizeof(double) * 2 * g.nzp));
-  return laplinv_tables(ctx, tabs.data() + 2 * cols);
+  if ((rc = laplinv_tables(ctx, tabs.data() + 2 * cols))) return rc;
+  if (ctx->mixed) return f32::invert_init(ctx);
+  // the FP64 inversion's reciprocal pivots, from the pivots of both solvers
+  const int64_t n = (int64_t)(g.sx >> 1) * (g.sy >> 1) * nz;
+  PMPIC_CUDA(cudaMalloc(&ctx->zrec, sizeof(double) * (4 * nz + 4 * n)));
+  for (int v = 0; v < 2; ++v) {
+    double* r = ctx->zrec + v * 2 * nz;
+    k_recip<<<nblk(nz, 256), 256, 0, ctx->stream>>>(nz, f64::diffz_tab(ctx, v) + nz, r, r + nz);
+    r = ctx->zrec + 4 * nz + v * 2 * n;
+    k_recip<<<nblk(n, 256), 256, 0, ctx->stream>>>(n, ctx->lapcp + 2 * v * n, r, r + n);
+    ctx->nlaunch += 2;
+  }
+  PMPIC_CUDA(cudaStreamSynchronize(ctx->stream));
+  return f64::invert_init(ctx);
 }
 
-int spec_diffx(pmpic_ctx* ctx, const double* in, double* out) { return f64::spec_diffx_impl(ctx, in, out); }
-int spec_diffy(pmpic_ctx* ctx, const double* in, double* out) { return f64::spec_diffy_impl(ctx, in, out); }
-int spec_filter(pmpic_ctx* ctx, const double* in, double* out) { return f64::spec_filter_impl(ctx, in, out); }
-int spec_diffz(pmpic_ctx* ctx, const double* in, double* out, const double* bot, const double* top) {
-  return f64::spec_diffz_impl(ctx, in, out, bot, top);
+int spec_diffx(pmpic_ctx* ctx, const double* in, double* out) {
+  k_diffx<<<nblk(ctx->g.nspec, 256), 256, 0, ctx->stream>>>(ctx->g, in, out, ctx->kx); ++ctx->nlaunch;
+  PMPIC_CUDA(cudaGetLastError());
+  return 0;
 }
-int spec_laplinv(pmpic_ctx* ctx, double* inout, bool df0) { return f64::spec_laplinv_impl(ctx, inout, df0); }
+int spec_diffy(pmpic_ctx* ctx, const double* in, double* out) {
+  k_diffy<<<nblk(ctx->g.nspec, 256), 256, 0, ctx->stream>>>(ctx->g, in, out, ctx->ky); ++ctx->nlaunch;
+  PMPIC_CUDA(cudaGetLastError());
+  return 0;
+}
+int spec_filter(pmpic_ctx* ctx, const double* in, double* out) {
+  k_filter<<<nblk(ctx->g.nspec, 256), 256, 0, ctx->stream>>>(ctx->g, in, out, ctx->filt); ++ctx->nlaunch;
+  PMPIC_CUDA(cudaGetLastError());
+  return 0;
+}
+int spec_diffz(pmpic_ctx* ctx, const double* in, double* out, const double* bot, const double* top) {
+  TimerScope ts(ctx, T_DIFFZ);
+  const Geom& g = ctx->g;
+  k_diffz<<<nblk((int64_t)g.sx * g.sy, 128), 128, 0, ctx->stream>>>(g, in, out, bot, top, f64::diffz_tab(ctx, bot ? 1 : 0),
+                                                                    f4div(1.f, 6.f)); ++ctx->nlaunch;
+  PMPIC_CUDA(cudaGetLastError());
+  return 0;
+}
+int spec_laplinv(pmpic_ctx* ctx, double* inout, bool df0) {
+  TimerScope ts(ctx, T_LAPLINV);
+  const Geom& g = ctx->g;
+  k_laplinv<<<nblk((int64_t)g.sx * g.sy, 128), 128, 0, ctx->stream>>>(g, inout, df0 ? 1 : 0, ctx->lapcp, ctx->k2); ++ctx->nlaunch;
+  PMPIC_CUDA(cudaGetLastError());
+  return 0;
+}
 
 // vort2vel.F90:139-320 and vorticity_tendency.F90:147-265 in the context's precision
 int vort2vel_spectral(pmpic_ctx* ctx) {

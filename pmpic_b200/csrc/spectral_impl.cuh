@@ -3,316 +3,468 @@
 // scalar type `real` and included by spectral.cu into one namespace per
 // precision (FP64 plain path, FP32 mixed-precision form).  The namespace
 // provides the tables of its precision (tab_kx, tab_ky, tab_k2, tab_filt,
-// tab_diffz) and the zero-mode hooks (zero_mode_prepare, zero_mode_launch).
-// Not a standalone header.
+// lap_tab, dz_tab) and zero_mode.  Not a standalone header.
 
 template <class P>
 inline real* RP(P* p) { return reinterpret_cast<real*>(p); }
 
-// ---- elementwise spectral operators --------------------------------------------
-// The wavenumber tables are laid out like a spectral level, but kx depends on
-// the x index ip alone and ky on the row jp alone: kx is read from row 0
-// (kx[ip]) and ky from column 0 (ky[jp * sx]), the same values.
-// diffx (fft_ops.F90:266-295): out(i) = -in(i+1) kx, out(i+1) = in(i) kx
-__device__ __forceinline__ real dx_of(const real* in, int64_t e, int ip, const real* kx) {
-  return (ip & 1) == 0 ? (real(-1) * in[e + 1]) * kx[ip] : in[e - 1] * kx[ip];
-}
-// diffy (fft_ops.F90:366-394)
-__device__ __forceinline__ real dy_of(const real* in, int64_t e, int jp, int sx, const real* ky) {
-  return (jp & 1) == 0 ? (real(-1) * in[e + sx]) * ky[jp * sx] : in[e - sx] * ky[jp * sx];
-}
-
-struct EwIdx {
-  int64_t e;
-  int col, ip, jp, k;
+// ---- the inversion's spectral part (vort2vel.F90:139-320) -----------------------------
+// One kernel from the transformed vorticity a, b, c to the corrected, filtered
+// vorticity and the velocity spectra.  Every operator on the way acts on a
+// column over all levels (the compact z solves, fft_ops.F90:419-601, and d/dz)
+// or on a mode's four columns (2i, 2i+1) x (2j, 2j+1) (diffx, diffy, the
+// filter).  So a CTA takes a tile of NC columns, NC / 2 of two neighbouring
+// rows, keeps three arrays of its columns in shared memory and touches global
+// memory to read a, b, c (twice: c's array has to serve lambda first) and to
+// write its results once, where separate operators would each stream whole
+// spectra.  The recurrences are sequential in z, one thread a column, one
+// warp an array; right-hand sides and everything else run on all threads, in
+// runs of levels.  What bounds it is the recurrences' latency: four chains of
+// nz levels, two dependent operations a level on the FP32 form; on the FP64
+// path the quotient by the pivot is n rh + n rl with the two-term reciprocal
+// (the division's rounding but for ties that the second term cannot decide),
+// four.  Their factors are tables, [mode][level].
+// Arithmetic and its order are the separate operators'.
+// Measured, ms per step for all that lies between the transforms (ten kernels
+// before, and the velocity spectra formed by the inverse x pass): 32^3 FP64
+// 0.60 -> 0.11, 96^3 FP32 0.85 -> 0.33, 128^3 FP64 2.0 -> 0.85; 256^3 FP32
+// 3.25 -> 3.26, but its inverse transforms 5.0 instead of 6.5.
+struct InvArgs {
+  real *a, *b, *c;           // in: the spectra; out: corrected and filtered
+  real *u, *v, *w;           // out: velocity spectra
+  real *us, *vs, *ws;        // and their filtered copies
+  const real *kx, *ky, *k2, *filt;
+  ZTab<real> lap[2], dz[2];  // per boundary form: laplinv (f0, df0), diffz (without, with boundary values)
+  double* zbar;              // mean flow ubar, vbar (FP64 path: written here)
+  real* work;                // the columns of the tiles, when they exceed shared memory
+  real hdzi;                 // 0.5 / dz (vort2vel.F90:158)
+  real rdz, rdzl;            // 1 / dz, two terms (FP64)
+  double rdz64;              // 1 / (FP32 dz)
+  int nxt;                   // tiles per row pair
 };
-__device__ __forceinline__ bool ew_index(const Geom& g, EwIdx& x) {
-  int64_t e = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
-  if (e >= g.nspec) return false;
-  int cols = g.sx * g.sy;
-  x.e = e;
-  x.k = (int)(e / cols);
-  x.col = (int)(e - (int64_t)x.k * cols);
-  x.jp = x.col / g.sx;
-  x.ip = x.col - x.jp * g.sx;
-  return true;
+// n / den with the reciprocal pivot
+__device__ __forceinline__ real zquot(real n, real r, real rl) {
+  if constexpr (sizeof(real) == 8) return __fma_rn(n, r, __dmul_rn(n, rl));
+  else return n * r;
 }
-
-__global__ void k_diffx(Geom g, const real* __restrict__ in, real* __restrict__ out, const real* __restrict__ kx) {
-  EwIdx x;
-  if (!ew_index(g, x)) return;
-  out[x.e] = dx_of(in, x.e, x.ip, kx);
-}
-__global__ void k_diffy(Geom g, const real* __restrict__ in, real* __restrict__ out, const real* __restrict__ ky) {
-  EwIdx x;
-  if (!ew_index(g, x)) return;
-  out[x.e] = dy_of(in, x.e, x.jp, g.sx, ky);
-}
-__global__ void k_filter(Geom g, const real* __restrict__ in, real* __restrict__ out,
-                         const real* __restrict__ filt) {
-  EwIdx x;
-  if (!ew_index(g, x)) return;
-  out[x.e] = in[x.e] * filt[x.col];
-}
-
-// vort2vel.F90:158-173: f = diffx(a) + diffy(b) + (dc/dz, 2nd order with
-// one-sided ends); f(:,1,1) = 0
-__global__ void k_div(Geom g, const real* __restrict__ a, const real* __restrict__ b,
-                      const real* __restrict__ c, real* __restrict__ f, const real* __restrict__ kx,
-                      const real* __restrict__ ky, real hdzi) {
-  EwIdx x;
-  if (!ew_index(g, x)) return;
-  const int64_t cs = (int64_t)g.sx * g.sy;
-  const int nz = g.nzp;
-  real d = dx_of(a, x.e, x.ip, kx);
-  real e = dy_of(b, x.e, x.jp, g.sx, ky);
-  real fz;
-  if (x.k == 0) {
-    fz = hdzi * (real(4) * c[x.e + cs] - c[x.e + 2 * cs] - real(3) * c[x.e]);
-  } else if (x.k == nz - 1) {
-    fz = hdzi * (c[x.e - 2 * cs] + real(3) * c[x.e] - real(4) * c[x.e - cs]);
-  } else {
-    fz = (c[x.e + cs] - c[x.e - cs]) * hdzi;
-  }
-  real v = d + e + fz;
-  if (x.col == 0) v = real(0);
-  f[x.e] = v;
-}
-
-// The filter and both subtractions of vort2vel.F90:179-194 in one pass:
-// fo = filter(f) and a = a - diffx(fo), b = b - diffy(fo), the neighbours'
-// filtered values formed as the filter forms them (f is left unfiltered; fo
-// is a separate array, so no thread reads a value another one rewrote)
-__global__ void k_filter_sub2(Geom g, const real* __restrict__ f, real* __restrict__ fo, real* __restrict__ a,
-                              real* __restrict__ b, const real* __restrict__ kx, const real* __restrict__ ky,
-                              const real* __restrict__ filt) {
-  EwIdx x;
-  if (!ew_index(g, x)) return;
-  fo[x.e] = f[x.e] * filt[x.col];
-  const real kxv = kx[x.ip], kyv = ky[x.jp * g.sx];  // (row 0, column 0: the same values)
-  const real dxf = (x.ip & 1) == 0 ? (real(-1) * (f[x.e + 1] * filt[x.col + 1])) * kxv
-                                   : (f[x.e - 1] * filt[x.col - 1]) * kxv;
-  const real dyf = (x.jp & 1) == 0 ? (real(-1) * (f[x.e + g.sx] * filt[x.col + g.sx])) * kyv
-                                   : (f[x.e - g.sx] * filt[x.col - g.sx]) * kyv;
-  a[x.e] = a[x.e] - dxf;
-  b[x.e] = b[x.e] - dyf;
-}
-
-// the top and bottom planes of a and b, unfiltered (vort2vel.F90:213-218)
-__global__ void k_bt_planes(Geom g, const real* __restrict__ a, const real* __restrict__ b, real* __restrict__ bt) {
-  const int col = blockIdx.x * blockDim.x + threadIdx.x;
-  const int cols = g.sx * g.sy;
-  if (col >= cols) return;
-  const size_t top = (size_t)(g.nzp - 1) * cols + col;
-  bt[0 * cols + col] = a[top];  // atop
-  bt[1 * cols + col] = a[col];  // abot
-  bt[2 * cols + col] = b[top];  // btop
-  bt[3 * cols + col] = b[col];  // bbot
-}
-
-// ---- compact z operators ----------------------------------------------------------
-// The z recurrences run one thread per spectral column, so only about 14 warps
-// per SM are resident at 256^2 columns and a level costs the latency of its
-// dependent instructions.  The Thomas factors (pivots den and ratios cp of
-// fft_ops.F90:620-656) depend only on the level and, for laplinv, on the
-// column's wavenumber: they are tables built once at set-up.  The FP64 path
-// keeps the reference's operations bit for bit (its tables repeat the
-// sequential recurrence exactly; the right-hand side is still divided by the
-// pivot); the FP32 form multiplies by the reciprocal pivot (taken from the FP64
-// recurrence and rounded once) and fuses the multiply-adds, so a level is two
-// dependent operations.
-__device__ __forceinline__ real zstep(real d, real a, real prev, real den_or_rden) {
-  if constexpr (sizeof(real) == 8) return (d - a * prev) / den_or_rden;
-  else return __fmaf_rn(-a, prev, d) * den_or_rden;
+__device__ __forceinline__ real zstep(real d, real a, real prev, real r, real rl) {
+  if constexpr (sizeof(real) == 8) return zquot(d - a * prev, r, rl);
+  else return __fmaf_rn(-a, prev, d) * r;
 }
 __device__ __forceinline__ real zback(real f, real cp, real nxt) {
   if constexpr (sizeof(real) == 8) return f - cp * nxt;
   else return __fmaf_rn(-cp, nxt, f);
 }
-__device__ __forceinline__ real zfirst(real d, real den_or_rden) {
-  if constexpr (sizeof(real) == 8) return d / den_or_rden;
-  else return d * den_or_rden;
+// The Thomas recurrence (fft_ops.F90:620-656) of a warp's columns in place:
+// right-hand side in, solution out.  X is the lane's column (level stride NC),
+// active false for a lane without one; ai the sub-diagonal of the inner
+// levels, an the last one's.  The factors of the warp's nm modes (mode m at
+// T.x + off + m * nz; only the first nmv exist) come through a ring in shared
+// memory, ZCH levels a chunk, three chunks ahead: read as they are needed,
+// their latency would bound the recurrence.
+constexpr int ZCH = 16, ZRING = 4;
+__device__ __forceinline__ void cp_async_z(real* smem, const real* gmem) {
+  const unsigned d = (unsigned)__cvta_generic_to_shared(smem);
+  if constexpr (sizeof(real) == 8) asm volatile("cp.async.ca.shared.global [%0], [%1], 8;\n" ::"r"(d), "l"(gmem) : "memory");
+  else asm volatile("cp.async.ca.shared.global [%0], [%1], 4;\n" ::"r"(d), "l"(gmem) : "memory");
+}
+template <int NC, int NM>
+__device__ __forceinline__ void thomas(real* X, bool active, int m, int nz, real ai, real an, const ZTab<real>& T,
+                                       int64_t off, int nmv, real* ring) {
+  constexpr bool D = sizeof(real) == 8;
+  constexpr int ZB = 8, SL = ZCH * NM;  // values of a table per chunk
+  const int lane = threadIdx.x & 31, nch = (nz + ZCH - 1) / ZCH;
+  real* ring2 = ring + ZRING * SL;
+  // chunk c of a table (and of the second) into its slot; one group either way
+  auto issue = [&](int c, const real* t, const real* t2) {
+    if (c >= 0 && c < nch) {
+      for (int e = lane; e < SL; e += 32) {
+        const int mm = e / ZCH, l = e % ZCH, k = c * ZCH + l;
+        if (mm < nmv && k < nz) {
+          cp_async_z(ring + (c % ZRING) * SL + l * NM + mm, t + off + (int64_t)mm * nz + k);
+          if (D && t2) cp_async_z(ring2 + (c % ZRING) * SL + l * NM + mm, t2 + off + (int64_t)mm * nz + k);
+        }
+      }
+    }
+    asm volatile("cp.async.commit_group;\n" ::: "memory");
+  };
+  auto ready = [&]() {
+    asm volatile("cp.async.wait_group 3;\n" ::: "memory");
+    __syncwarp();
+  };
+  // levels 0 .. nz-2 in whole chunks (constant offsets, no bounds: a level is
+  // little more than its loads, its two or four dependent operations and its
+  // store), then the rest one by one, the last with an
+  const int nfull = (nz - 1) / ZCH;
+  for (int c = 0; c < 3; ++c) issue(c, T.r, T.rl);
+  real prev = real(0);
+  for (int c = 0; c < nch; ++c) {
+    __syncwarp();  // the slot's last chunk has been read
+    issue(c + 3, T.r, T.rl);
+    ready();
+    const real* r = ring + (c % ZRING) * SL + m;
+    const real* rl = ring2 + (c % ZRING) * SL + m;
+    real* Xc = X + c * ZCH * NC;
+    if (!active) continue;
+    if (c < nfull) {
+#pragma unroll
+      for (int h = 0; h < ZCH; h += ZB) {
+        real d[ZB], rr[ZB], ll[ZB];
+#pragma unroll
+        for (int u = 0; u < ZB; ++u) {
+          rr[u] = r[(h + u) * NM];
+          ll[u] = D ? rl[(h + u) * NM] : real(0);
+          d[u] = Xc[(h + u) * NC];
+        }
+#pragma unroll
+        for (int u = 0; u < ZB; ++u) {  // (level 0: prev is zero)
+          prev = zstep(d[u], ai, prev, rr[u], ll[u]);
+          Xc[(h + u) * NC] = prev;
+        }
+      }
+    } else {
+      for (int l = 0; c * ZCH + l < nz; ++l) {
+        prev = zstep(Xc[l * NC], c * ZCH + l == nz - 1 ? an : ai, prev, r[l * NM], D ? rl[l * NM] : real(0));
+        Xc[l * NC] = prev;
+      }
+    }
+  }
+  // back substitution from level nz-2: f(k) = f(k) - cp(k+1) f(k+1)
+  __syncwarp();
+  for (int c = nch - 1; c > nch - 4; --c) issue(c, T.cp, nullptr);
+  real hi = real(0);  // cp of the level above
+  for (int c = nch - 1; c >= 0; --c) {
+    __syncwarp();
+    issue(c - 3, T.cp, nullptr);
+    ready();
+    const real* cp = ring + (c % ZRING) * SL + m;
+    real* Xc = X + c * ZCH * NC;
+    if (!active) continue;
+    if (c < nfull) {
+#pragma unroll
+      for (int h = ZCH - ZB; h >= 0; h -= ZB) {
+        real f[ZB], cc[ZB];
+#pragma unroll
+        for (int u = 0; u < ZB; ++u) {
+          cc[u] = cp[(h + u) * NM];
+          f[u] = Xc[(h + u) * NC];
+        }
+#pragma unroll
+        for (int u = ZB - 1; u >= 0; --u) {
+          prev = zback(f[u], u == ZB - 1 ? hi : cc[u + 1], prev);
+          Xc[(h + u) * NC] = prev;
+        }
+        hi = cc[0];
+      }
+    } else {
+      for (int l = nz - 1 - c * ZCH; l >= 0; --l) {
+        if (c * ZCH + l < nz - 1) {
+          prev = zback(Xc[l * NC], hi, prev);
+          Xc[l * NC] = prev;
+        }
+        hi = cp[l * NM];
+      }
+    }
+  }
+}
+// X[k] = f(k, X[k-1], X[k], X[k+1]) for this thread's run of levels k0 .. k1-1,
+// in place, given the values either side of the run
+template <int NC, class F>
+__device__ __forceinline__ void zwalk(real* X, int k0, int k1, real below, real above, F f) {
+  if (k0 >= k1) return;
+  real fm = below, f0 = X[k0 * NC];
+#pragma unroll 4
+  for (int k = k0; k < k1; ++k) {
+    const real fp = k + 1 < k1 ? X[(k + 1) * NC] : above;
+    X[k * NC] = f(k, fm, f0, fp);
+    fm = f0;
+    f0 = fp;
+  }
 }
 
-// diffz (fft_ops.F90:419-483).  The tridiagonal coefficients are the same for
-// every column, so the Thomas factors (cp and the pivots; the reciprocal
-// pivots on the FP32 form) are computed once on the host with the reference's
-// arithmetic and passed in.
-// blockIdx.y selects one of up to two independent solves in the same launch.
-struct DzBatch {
-  const real* f[2];
-  real* out[2];
-  const real* bot[2];  // both null: no boundary values (df0 form)
-  const real* top[2];
-  real* sub;           // solve 0 only: c = c - diffz(f), c(1,:,:) = 0 (vort2vel.F90:196-205) in
-                       // place of the final values in out
-};
-__global__ void k_diffz(Geom g, DzBatch zb, const real* __restrict__ coef /* a[nz], den[nz] (FP32: 1/den), cp[nz] */,
-                        real a1) {
-  const int col = blockIdx.x * blockDim.x + threadIdx.x;
-  const int cols = g.sx * g.sy;
-  if (col >= cols) return;
-  const int q = blockIdx.y;  // selected without indexing the parameter arrays (no local copy)
-  const real* __restrict__ f = q == 0 ? zb.f[0] : zb.f[1];
-  real* __restrict__ out = q == 0 ? zb.out[0] : zb.out[1];
-  const real* __restrict__ bot = q == 0 ? zb.bot[0] : zb.bot[1];
-  const real* __restrict__ top = q == 0 ? zb.top[0] : zb.top[1];
-  const int nz = g.nzp;
-  const uint32_t cs = (uint32_t)cols;  // level offsets fit 32 bits (the spectral grid is < 2^31)
-  const real* A = coef;
-  const real* DEN = coef + nz;
-  const real* CP = coef + 2 * nz;
+constexpr int INV_T = 256;
+// values of the rings of the three chain warps
+template <int NC>
+__host__ __device__ constexpr int inv_ring() {
+  return 3 * ZRING * ZCH * (NC / 4) * (sizeof(real) == 8 ? 2 : 1);
+}
+template <int NC, bool GM>
+__global__ void __launch_bounds__(INV_T, 2) k_invert(Geom g, const __grid_constant__ InvArgs S) {
+  constexpr int W = NC / 2, NG = INV_T / NC;
+  extern __shared__ __align__(16) unsigned char zsm[];
+  const int nz = g.nzp, sx = g.sx;
+  const int64_t cs = (int64_t)sx * g.sy;
+  const int col = threadIdx.x % NC, grp = threadIdx.x / NC, warp = threadIdx.x >> 5;
+  const int ip = (blockIdx.x % S.nxt) * W + col % W, jp = 2 * (blockIdx.x / S.nxt) + col / W;
+  const bool in = ip < sx;
+  const int gc = jp * sx + (in ? ip : 0);                 // spectral column
+  const int sgx = in ? ((ip & 1) ? -1 : 1) : 0, sgy = (jp & 1) ? -sx : sx;  // to the mode's neighbour columns
+  const int cx = col ^ 1, cy = col ^ W;                   // the same in the tile
+  constexpr int NM = NC / 4, RING = inv_ring<NC>() / 3;
+  real* ring = (real*)zsm + (warp < 3 ? warp : 0) * RING;
+  real* F = GM ? S.work + (size_t)blockIdx.x * 3 * nz * NC : (real*)zsm + 3 * RING;  // lambda, then c
+  real *A = F + nz * NC, *B = A + nz * NC;
+  const real kx = S.kx[in ? ip : 0], ky = S.ky[jp * sx], kk = S.k2[gc];
+  const real fl = S.filt[gc], flx = S.filt[gc + sgx], fly = S.filt[gc + sgy];
+  const bool solve = in && kk != 0;  // columns with k2 == 0 keep their input (fft_ops.F90:567)
+  const int L = (nz + NG - 1) / NG, k0 = min(grp * L, nz), k1 = min(k0 + L, nz);
   const real dz = (real)g.dz;
-  const bool bt = bot != nullptr;
-  // forward sweep: f'(1) = d(1)/den(1); f'(i) = (d(i) - a(i) f'(i-1)) / den(i).
-  // The loads of each batch of ZB levels are issued before its recurrence, so
-  // the loop waits on one memory latency per batch, not per level.
-  constexpr int ZB = 8;
-  real fm = f[col], f0 = f[cs + col];
-  real d1 = bt ? f0 / dz - a1 * bot[col] * dz : real(0);
-  real prev = zfirst(d1, DEN[0]);
-  out[col] = prev;
-  for (int kb = 1; kb < nz - 1; kb += ZB) {
-    real fb[ZB];
-#pragma unroll
-    for (int u = 0; u < ZB; ++u)
-      if (kb + u < nz - 1) fb[u] = f[(uint32_t)(kb + u + 1) * cs + col];
-#pragma unroll
-    for (int u = 0; u < ZB; ++u) {
-      const int k = kb + u;
-      if (k >= nz - 1) break;
-      real d = (fb[u] - fm) / real(2) / dz;
-      prev = zstep(d, A[k], prev, DEN[k]);
-      out[(uint32_t)k * cs + col] = prev;
-      fm = f0;
-      f0 = fb[u];
-    }
-  }
-  real* __restrict__ sub = q == 0 ? zb.sub : nullptr;
-  {
-    int k = nz - 1;
-    real dn = bt ? -fm / dz + a1 * top[col] * dz : real(0);  // fm = f(nz-1)
-    prev = zstep(dn, A[k], prev, DEN[k]);
-    if (sub) sub[(uint32_t)k * cs + col] = sub[(uint32_t)k * cs + col] - prev;
-    else out[(uint32_t)k * cs + col] = prev;
-  }
-  // back substitution: f(i) = f(i) - cp(i+1) f(i+1)
-  real nxt = prev;
-  for (int kb = nz - 2; kb >= 0; kb -= ZB) {
-    real ob[ZB], sb[ZB];
-#pragma unroll
-    for (int u = 0; u < ZB; ++u)
-      if (kb - u >= 0) {
-        ob[u] = out[(uint32_t)(kb - u) * cs + col];
-        if (sub) sb[u] = sub[(uint32_t)(kb - u) * cs + col];  // loaded with the batch, off the chain
-      }
-#pragma unroll
-    for (int u = 0; u < ZB; ++u) {
-      const int k = kb - u;
-      if (k < 0) break;
-      real v = zback(ob[u], CP[k + 1], nxt);
-      if (sub) {
-        sub[(uint32_t)k * cs + col] = k == 0 ? real(0) : sb[u] - v;
-      } else {
-        out[(uint32_t)k * cs + col] = v;
-      }
-      nxt = v;
-    }
-  }
-}
-
-// laplinv (fft_ops.F90:505-601), in place, one thread per column; columns with
-// k2 == 0 keep their input (:567).  The Thomas factors of a column depend on
-// its wavenumber only, shared by the four columns (2a-1..2a, 2b-1..2b) of one
-// mode (a, b): tab holds, per boundary form (f0, df0), the pivots (FP32: their
-// reciprocals) and then the ratios cp, each [level][mode], built at set-up
-// (laplinv_tables).
-// blockIdx.y selects one of up to three arrays solved in the same launch
-struct LapBatch {
-  real* f[3];
-  int df0[3];
-};
-__global__ void k_laplinv(Geom g, LapBatch lb, const real* __restrict__ tab, const real* __restrict__ k2) {
-  int col = blockIdx.x * blockDim.x + threadIdx.x;
-  const int cols = g.sx * g.sy;
-  if (col >= cols) return;
-  const int q = blockIdx.y;  // selected without indexing the parameter arrays (no local copy)
-  real* __restrict__ f = q == 0 ? lb.f[0] : (q == 1 ? lb.f[1] : lb.f[2]);
-  const int df0 = q == 0 ? lb.df0[0] : (q == 1 ? lb.df0[1] : lb.df0[2]);
-  const real kk = k2[col];
-  if (kk == 0) return;
-  const int nz = g.nzp;
-  const int64_t cs = cols;
-  const int nmode = (g.sx >> 1) * (g.sy >> 1);
-  const int jp = col / g.sx, ip = col - jp * g.sx;
-  const real* __restrict__ DEN = tab + (size_t)(2 * df0) * nz * nmode + (jp >> 1) * (g.sx >> 1) + (ip >> 1);
-  const real* __restrict__ CP = DEN + (size_t)nz * nmode;
   const real f16 = (real)f4div(1.f, 6.f), f13 = (real)f4div(1.f, 3.f), f112 = (real)f4div(1.f, 12.f), f56 = (real)f4div(5.f, 6.f);
-  const real dz = (real)g.dz;
   const real idz2 = real(1) / dz / dz;
-  const real ai = idz2 - f112 * kk;
-  real an;
-  real fm, f0, fp;
-  f0 = f[col];
-  fp = f[cs + col];
-  real d;
-  if (!df0) {
-    d = real(0);
-    an = real(0);
-  } else {
-    d = f13 * f0 + f16 * fp;
-    an = idz2 - f16 * kk;
-  }
-  // tridiagonal (fft_ops.F90:620-656) with the tabulated factors
-  real prev = zfirst(d, DEN[0]);
-  f[col] = prev;
-  // loads of each batch of ZB levels first, then its recurrence (one memory
-  // latency per batch); the batch reads f above the levels it overwrites
-  constexpr int ZB = sizeof(real) == 8 ? 4 : 8;  // FP64: fewer registers for the batch
-  for (int kb = 1; kb < nz; kb += ZB) {
-    real fb[ZB], db[ZB];
+  const real lai = idz2 - f112 * kk, lan = idz2 - f16 * kk;
+  // the tile's modes: the first one's factors in the tables, how many exist, and this column's
+  const int tx = blockIdx.x % S.nxt;
+  const int64_t mode0 = ((int64_t)(blockIdx.x / S.nxt) * (sx >> 1) + tx * (W / 2)) * nz;
+  const int nmv = min(NM, (sx >> 1) - tx * (W / 2)), mcol = (col % W) >> 1;
+  const bool lanecol = (threadIdx.x & 31) < NC;  // (a chain warp's lane is its column)
+  auto dxs = [&](real nb) { return (ip & 1) == 0 ? (real(-1) * nb) * kx : nb * kx; };  // diffx from the neighbour
+  auto dys = [&](real nb) { return (jp & 1) == 0 ? (real(-1) * nb) * ky : nb * ky; };
+  auto qdz = [&](real n) {  // n / dz
+    if constexpr (sizeof(real) == 8) return zquot(n, S.rdz, S.rdzl);
+    // FP32: a quotient of two FP32 values is no nearer to a rounding boundary
+    // than 2^-49 of itself, so the FP64 product with 1 / dz, off by 2^-52,
+    // rounds to the bits of n / dz
+    else return (real)((double)n * S.rdz64);
+  };
+  auto at = [&](int k) { return (int64_t)k * cs + gc; };
+  constexpr int LB = 8;  // levels loaded together
+
+  // lambda's right-hand side f = diffx(a) + diffy(b) + dc/dz (2nd order, one-
+  // sided at the walls), f(:,1,1) = 0 (vort2vel.F90:158-173)
+  if (in) {
+    real cm = k0 > 0 ? S.c[at(k0 - 1)] : real(0), c0 = S.c[at(min(k0, nz - 1))];
+    for (int kb = k0; kb < k1; kb += LB) {
+      real av[LB], bv[LB], cv[LB];
 #pragma unroll
-    for (int u = 0; u < ZB; ++u) {
-      if (kb + u < nz - 1) fb[u] = f[(int64_t)(kb + u + 1) * cs + col];
-      if (kb + u < nz) db[u] = DEN[(size_t)(kb + u) * nmode];
-    }
-#pragma unroll
-    for (int u = 0; u < ZB; ++u) {
-      const int k = kb + u;
-      if (k >= nz) break;
-      fm = f0;
-      f0 = fp;
-      real a;
-      if (k < nz - 1) {
-        fp = fb[u];
-        a = ai;
-        d = f112 * fm + f56 * f0 + f112 * fp;
-      } else {
-        a = an;
-        d = df0 ? f13 * f0 + f16 * fm : real(0);
-      }
-      prev = zstep(d, a, prev, db[u]);
-      f[(int64_t)k * cs + col] = prev;
-    }
-  }
-  real nxt = prev;
-  for (int kb = nz - 2; kb >= 0; kb -= ZB) {
-    real fb[ZB], cb[ZB];
-#pragma unroll
-    for (int u = 0; u < ZB; ++u)
-      if (kb - u >= 0) {
-        fb[u] = f[(int64_t)(kb - u) * cs + col];
-        cb[u] = CP[(size_t)(kb - u + 1) * nmode];
+      for (int u = 0; u < LB; ++u) {
+        const int k = min(kb + u, nz - 1);
+        av[u] = S.a[at(k) + sgx];
+        bv[u] = S.b[at(k) + sgy];
+        cv[u] = S.c[at(min(k + 1, nz - 1))];
       }
 #pragma unroll
-    for (int u = 0; u < ZB; ++u) {
-      const int k = kb - u;
-      if (k < 0) break;
-      real v = zback(fb[u], cb[u], nxt);
-      f[(int64_t)k * cs + col] = v;
-      nxt = v;
+      for (int u = 0; u < LB; ++u) {
+        const int k = kb + u;
+        if (k >= k1) break;
+        real fz;
+        if (k == 0) fz = S.hdzi * (real(4) * cv[u] - S.c[at(2)] - real(3) * c0);
+        else if (k == nz - 1) fz = S.hdzi * (S.c[at(nz - 3)] + real(3) * c0 - real(4) * cm);
+        else fz = (cv[u] - cm) * S.hdzi;
+        real v = dxs(av[u]) + dys(bv[u]) + fz;
+        if (gc == 0) v = real(0);
+        F[k * NC + col] = v;
+        cm = c0;
+        c0 = cv[u];
+      }
     }
   }
+  __syncthreads();
+  // laplinv's right-hand sides and solves, in place (fft_ops.F90:505-601)
+  auto edge = [&](const real* X, real& lo, real& hi) {
+    lo = k0 > 0 && k0 < k1 ? X[(k0 - 1) * NC + col] : real(0);
+    hi = k1 < nz && k0 < k1 ? X[k1 * NC + col] : real(0);
+  };
+  auto lap_rhs = [&](real* X, bool df0, real lo, real hi) {
+    zwalk<NC>(X + col, k0, k1, lo, hi, [&](int k, real fm, real f0, real fp) {
+      if (k == 0) return df0 ? f13 * f0 + f16 * fp : real(0);
+      if (k == nz - 1) return df0 ? f13 * f0 + f16 * fm : real(0);
+      return f112 * fm + f56 * f0 + f112 * fp;
+    });
+  };
+  real lo, hi;
+  edge(F, lo, hi);
+  __syncthreads();
+  if (solve) lap_rhs(F, true, lo, hi);
+  __syncthreads();
+  if (warp == 0) thomas<NC, NM>(F + col, lanecol && solve, mcol, nz, lai, lan, S.lap[1], mode0, nmv, ring);
+  __syncthreads();
+  // lambda filtered; a = a - diffx(lambda), b = b - diffy(lambda) (:179-194)
+  if (in) {
+    for (int kb = k0; kb < k1; kb += LB) {
+      real av[LB], bv[LB];
+#pragma unroll
+      for (int u = 0; u < LB; ++u) {
+        const int64_t e = at(min(kb + u, nz - 1));
+        av[u] = S.a[e];
+        bv[u] = S.b[e];
+      }
+#pragma unroll
+      for (int u = 0; u < LB; ++u) {
+        const int k = kb + u;
+        if (k >= k1) break;
+        A[k * NC + col] = av[u] - dxs(F[k * NC + cx] * flx);
+        B[k * NC + col] = bv[u] - dys(F[k * NC + cy] * fly);
+      }
+    }
+  }
+  edge(F, lo, hi);
+  __syncthreads();
+  // c = c - diffz(lambda), c(1,:,:) = 0 (:196-205); meanwhile a and b go out, filtered (:207-218)
+  zwalk<NC>(F + col, k0, k1, lo, hi, [&](int k, real fm, real, real fp) {
+    return k == 0 || k == nz - 1 ? real(0) : qdz((fp * fl - fm * fl) / real(2));
+  });
+  __syncthreads();
+  if (threadIdx.x < 32) {
+    thomas<NC, 1>(F + col, lanecol && in, 0, nz, f16, real(0), S.dz[0], 0, 1, ring);
+  } else if (in) {
+    for (int k = (threadIdx.x - 32) / NC; k < nz; k += (INV_T - 32) / NC) {
+      S.a[at(k)] = A[k * NC + col] * fl;
+      S.b[at(k)] = B[k * NC + col] * fl;
+    }
+  }
+  __syncthreads();
+  const real abot = A[col], atop = A[(nz - 1) * NC + col], bbot = B[col], btop = B[(nz - 1) * NC + col];
+  if (in) {
+    for (int kb = k0; kb < k1; kb += LB) {
+      real cv[LB];
+#pragma unroll
+      for (int u = 0; u < LB; ++u) cv[u] = S.c[at(min(kb + u, nz - 1))];
+#pragma unroll
+      for (int u = 0; u < LB; ++u) {
+        const int k = kb + u;
+        if (k >= k1) break;
+        const real c = k == 0 ? real(0) : cv[u] - F[k * NC + col];
+        F[k * NC + col] = c;
+        S.c[at(k)] = c * fl;
+      }
+    }
+  }
+  __syncthreads();
+  // the vector potential: laplinv of a, b (f0) and c (df0) (:243-249)
+  real loa, hia, lob, hib;
+  edge(A, loa, hia);
+  edge(B, lob, hib);
+  edge(F, lo, hi);
+  __syncthreads();
+  if (solve) {
+    lap_rhs(A, false, loa, hia);
+    lap_rhs(B, false, lob, hib);
+    lap_rhs(F, true, lo, hi);
+  }
+  __syncthreads();
+  if (warp < 3) {
+    thomas<NC, NM>((warp == 0 ? A : (warp == 1 ? B : F)) + col, lanecol && solve, mcol, nz, lai,
+                   warp == 2 ? lan : real(0), S.lap[warp == 2], mode0, nmv, ring);
+  } else if (sizeof(real) == 8 && blockIdx.x == 0 && threadIdx.x == 96) {
+    // mean flow of the zero mode (vort2vel.F90:230-241; k_zmode) from column
+    // 0 of the filtered a and b (it keeps its values: k2 == 0)
+    const double f0 = S.filt[0], dzd = g.dz;
+    double u = 0, v = 0;
+    double *ub = S.zbar, *vb = S.zbar + nz;
+    ub[0] = vb[0] = 0;
+    for (int k = 0; k < nz - 1; ++k) {
+      u = u + dzd / 2. * (B[k * NC] * f0 + B[(k + 1) * NC] * f0);
+      v = v - dzd / 2. * (A[k * NC] * f0 + A[(k + 1) * NC] * f0);
+      ub[k + 1] = u;
+      vb[k + 1] = v;
+    }
+    const double inz = (double)(1.0f / (float)nz);
+    double su = 0.0, sv = 0.0;
+    for (int k = 0; k < nz - 1; ++k) {
+      su = su + (ub[k] + f4(0.5f) * u);
+      sv = sv + (vb[k] + f4(0.5f) * v);
+    }
+    for (int k = 0; k < nz; ++k) {
+      ub[k] = ub[k] - inz * su;
+      vb[k] = vb[k] - inz * sv;
+    }
+  }
+  __syncthreads();
+  // w = dA/dy - dB/dx and its filtered copy (:306-320)
+  if (in) {
+#pragma unroll 4
+    for (int k = k0; k < k1; ++k) {
+      const real w = dys(A[k * NC + cy]) - dxs(B[k * NC + cx]);
+      S.w[at(k)] = w;
+      S.ws[at(k)] = w * fl;
+    }
+  }
+  edge(A, loa, hia);
+  edge(B, lob, hib);
+  __syncthreads();
+  // dA/dz and dB/dz with boundary values (:255, :284)
+  auto dz_rhs = [&](real* X, real lo, real hi, real bot, real top) {
+    zwalk<NC>(X + col, k0, k1, lo, hi, [&](int k, real fm, real, real fp) {
+      if (k == 0) return qdz(fp) - f16 * bot * dz;
+      if (k == nz - 1) return qdz(-fm) + f16 * top * dz;
+      return qdz((fp - fm) / real(2));
+    });
+  };
+  dz_rhs(A, loa, hia, abot, atop);
+  dz_rhs(B, lob, hib, bbot, btop);
+  __syncthreads();
+  if (warp < 2) thomas<NC, 1>((warp == 0 ? A : B) + col, lanecol && in, 0, nz, f16, f13, S.dz[1], 0, 1, ring);
+  __syncthreads();
+  // u = dB/dz - dC/dy, v = dC/dx - dA/dz, the mean flow in mode (0, 0) (:251-302)
+  if (in) {
+#pragma unroll 4
+    for (int k = k0; k < k1; ++k) {
+      real u = B[k * NC + col] - dys(F[k * NC + cy]), v = dxs(F[k * NC + cx]) - A[k * NC + col];
+      if (gc == 0) {
+        u = (real)S.zbar[k];
+        v = (real)S.zbar[nz + k];
+      }
+      S.u[at(k)] = u;
+      S.us[at(k)] = u * fl;
+      S.v[at(k)] = v;
+      S.vs[at(k)] = v * fl;
+    }
+  }
+}
+
+// Columns per tile: as many as let two CTAs share an SM's 227 KB, fewer while
+// the grid has not a tile per SM; one CTA per SM, and then global memory in
+// place of shared memory, only for more levels than 8 columns can hold.
+struct InvPlan {
+  int nc;
+  bool gm;
+  size_t bytes;  // of shared memory
+};
+InvPlan invert_plan(const Geom& g) {
+  auto ring = [&](int nc) { return (size_t)3 * ZRING * ZCH * (nc / 4) * (sizeof(real) == 8 ? 2 : 1); };
+  auto bytes = [&](int nc) { return ((size_t)3 * g.nzp * nc + ring(nc)) * sizeof(real); };
+  auto tiles = [&](int nc) { return (int64_t)(g.sy / 2) * ((g.sx + nc / 2 - 1) / (nc / 2)); };
+  int nc = 32;
+  while (nc > 8 && (bytes(nc) > 112 * 1024 || tiles(nc) < 148)) nc /= 2;
+  const bool gm = bytes(nc) > 224 * 1024;
+  return InvPlan{nc, gm, gm ? ring(nc) * sizeof(real) : bytes(nc)};
+}
+template <class F>
+void invert_kernel(const InvPlan& p, F&& f) {
+  if (p.gm) f(k_invert<8, true>);
+  else if (p.nc == 32) f(k_invert<32, false>);
+  else if (p.nc == 16) f(k_invert<16, false>);
+  else f(k_invert<8, false>);
+}
+int invert_init(pmpic_ctx* ctx) {
+  const Geom& g = ctx->g;
+  const InvPlan p = invert_plan(g);
+  if (p.gm) {
+    const int64_t tiles = (int64_t)(g.sy / 2) * ((g.sx + p.nc / 2 - 1) / (p.nc / 2));
+    PMPIC_CUDA(cudaMalloc(&ctx->zwork, sizeof(real) * 3 * (size_t)g.nzp * p.nc * tiles));
+    return 0;
+  }
+  cudaError_t e = cudaSuccess;
+  invert_kernel(p, [&](auto k) { e = cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, 225 * 1024); });
+  PMPIC_CUDA(e);
+  return 0;
+}
+int invert_launch(pmpic_ctx* ctx, real* a, real* b, real* c, real* u, real* v, real* w) {
+  TimerScope ts(ctx, T_LAPLINV);
+  const Geom& g = ctx->g;
+  const InvPlan p = invert_plan(g);
+  InvArgs S{a, b, c, u, v, w, RP(ctx->spec[PMPIC_SPEC_U]), RP(ctx->spec[PMPIC_SPEC_V]), RP(ctx->spec[PMPIC_SPEC_W]),
+            tab_kx(ctx), tab_ky(ctx), tab_k2(ctx), tab_filt(ctx), {lap_tab(ctx, 0), lap_tab(ctx, 1)},
+            {dz_tab(ctx, 0), dz_tab(ctx, 1)}, ctx->zmode, (real*)ctx->zwork, (real)(f4div(1.f, 2.f) / g.dz)};
+  const double r = 1.0 / g.dz;
+  S.rdz = (real)r;
+  S.rdzl = (real)(std::fma(-g.dz, r, 1.0) * r);
+  S.rdz64 = 1.0 / (double)(real)g.dz;
+  S.nxt = (g.sx + p.nc / 2 - 1) / (p.nc / 2);
+  invert_kernel(p, [&](auto k) { k<<<(unsigned)(S.nxt * (g.sy / 2)), INV_T, p.bytes, ctx->stream>>>(g, S); });
+  ++ctx->nlaunch;
+  PMPIC_CUDA(cudaGetLastError());
+  return 0;
 }
 
 // max of squares over the interior (vort2vel.F90:331-338,
@@ -348,147 +500,32 @@ __global__ void k_max_vort(int64_t n, const real* __restrict__ p, const real* __
   if ((threadIdx.x & 31) == 0) atomicMax((unsigned long long*)out, __double_as_longlong((double)m));
 }
 
-// nb (1 or 2) diffz solves of one boundary kind (all with or all without
-// boundary values) in one launch
-int diffz_batch_impl(pmpic_ctx* ctx, int nb, const real* const* in, real* const* out, const real* const* bot,
-                     const real* const* top, real* sub = nullptr) {
-  TimerScope ts(ctx, T_DIFFZ);
-  const Geom& g = ctx->g;
-  DzBatch zb{};
-  zb.sub = sub;
-  for (int q = 0; q < nb; ++q) {
-    zb.f[q] = in[q];
-    zb.out[q] = out[q];
-    zb.bot[q] = bot ? bot[q] : nullptr;
-    zb.top[q] = top ? top[q] : nullptr;
-  }
-  const real* coef = tab_diffz(ctx, bot ? 1 : 0);
-  k_diffz<<<dim3(nblk((int64_t)g.sx * g.sy, 128), nb), 128, 0, ctx->stream>>>(g, zb, coef, (real)f4div(1.f, 6.f)); ++ctx->nlaunch;
-  PMPIC_CUDA(cudaGetLastError());
-  return 0;
-}
-int diffz_launch_impl(pmpic_ctx* ctx, const real* in, real* out, const real* bot, const real* top) {
-  return diffz_batch_impl(ctx, 1, &in, &out, bot ? &bot : nullptr, top ? &top : nullptr);
-}
-
-
-int spec_diffx_impl(pmpic_ctx* ctx, const real* in, real* out) {
-  k_diffx<<<nblk(ctx->g.nspec, 256), 256, 0, ctx->stream>>>(ctx->g, in, out, tab_kx(ctx)); ++ctx->nlaunch;
-  PMPIC_CUDA(cudaGetLastError());
-  return 0;
-}
-int spec_diffy_impl(pmpic_ctx* ctx, const real* in, real* out) {
-  k_diffy<<<nblk(ctx->g.nspec, 256), 256, 0, ctx->stream>>>(ctx->g, in, out, tab_ky(ctx)); ++ctx->nlaunch;
-  PMPIC_CUDA(cudaGetLastError());
-  return 0;
-}
-int spec_filter_impl(pmpic_ctx* ctx, const real* in, real* out) {
-  k_filter<<<nblk(ctx->g.nspec, 256), 256, 0, ctx->stream>>>(ctx->g, in, out, tab_filt(ctx)); ++ctx->nlaunch;
-  PMPIC_CUDA(cudaGetLastError());
-  return 0;
-}
-int spec_diffz_impl(pmpic_ctx* ctx, const real* in, real* out, const real* bot, const real* top) {
-  return diffz_launch_impl(ctx, in, out, bot, top);
-}
-// laplinv of na (1..3) arrays in one launch, the Thomas factors from the tables
-int spec_laplinv_batch(pmpic_ctx* ctx, int na, real* const* fs, const bool* df0) {
-  TimerScope ts(ctx, T_LAPLINV);
-  const Geom& g = ctx->g;
-  LapBatch lb{};
-  for (int q = 0; q < na; ++q) {
-    lb.f[q] = fs[q];
-    lb.df0[q] = df0[q] ? 1 : 0;
-  }
-  k_laplinv<<<dim3(nblk((int64_t)g.sx * g.sy, 128), na), 128, 0, ctx->stream>>>(g, lb, RP(ctx->lapcp), tab_k2(ctx)); ++ctx->nlaunch;
-  PMPIC_CUDA(cudaGetLastError());
-  return 0;
-}
-int spec_laplinv_impl(pmpic_ctx* ctx, real* inout, bool df0) { return spec_laplinv_batch(ctx, 1, &inout, &df0); }
-
 // vort2vel.F90:139-320 after the three par2grid calls (grids P, Q, R hold the
 // gridded vorticity on entry; on exit they hold the corrected, filtered
 // vorticity, U, V, W the velocity and u_s, v_s, w_s its filtered spectra).
 int vort2vel_spectral_impl(pmpic_ctx* ctx) {
   const Geom& g = ctx->g;
   int rc;
-  real *a = RP(ctx->sa), *b = RP(ctx->sb), *c = RP(ctx->sc), *d = RP(ctx->sd), *e = RP(ctx->se), *f = RP(ctx->sf);
+  real *a = RP(ctx->sa), *b = RP(ctx->sb), *c = RP(ctx->sc), *u = RP(ctx->sd), *v = RP(ctx->se), *w = RP(ctx->sf);
   real* const* G = (real* const*)ctx->grid;
-  zero_mode_prepare(ctx);
-  const unsigned nb = nblk(g.nspec, 256);
-  const int cols = g.sx * g.sy;
-  // scratch of the transforms: these spectral arrays hold nothing the inversion reads
-  real* mids[3] = {RP(ctx->fftmid), RP(ctx->sas), RP(ctx->sbs)};
+  if ((rc = zero_mode(ctx))) return rc;
+  // scratch of the transforms: these arrays hold nothing that the inversion
+  // reads (the packed gather grids are made afresh before they are used)
+  const size_t nmid = (size_t)g.nzp * g.sy * g.Nx;
+  real* pk = RP(ctx->gpack);
+  real* mids[6] = {RP(ctx->fftmid), RP(ctx->sas), RP(ctx->sbs), pk, pk + nmid, pk + 2 * nmid};
   {
     const real* in[3] = {G[PMPIC_GRID_P], G[PMPIC_GRID_Q], G[PMPIC_GRID_R]};
     real* out[3] = {a, b, c};
     if ((rc = fft_forward(ctx, 3, in, out, mids))) return rc;
   }
-  const real hdzi = (real)(f4div(1.f, 2.f) / g.dz);
-  k_div<<<nb, 256, 0, ctx->stream>>>(g, a, b, c, f, tab_kx(ctx), tab_ky(ctx), hdzi); ++ctx->nlaunch;
-  if ((rc = spec_laplinv_impl(ctx, f, true))) return rc;
-  // :179-205: the filtered f (into e), a and b corrected, then c = c - diffz(filtered f)
-  k_filter_sub2<<<nb, 256, 0, ctx->stream>>>(g, f, e, a, b, tab_kx(ctx), tab_ky(ctx), tab_filt(ctx)); ++ctx->nlaunch;
-  {
-    const real* zin[1] = {e};
-    real* zout[1] = {d};
-    if ((rc = diffz_batch_impl(ctx, 1, zin, zout, nullptr, nullptr, c))) return rc;
-  }
-  // :207-226: the top and bottom planes of a and b, then the filtered a, b, c
-  // transformed back (the filter applied as the transform reads them)
-  k_bt_planes<<<nblk(cols, 256), 256, 0, ctx->stream>>>(g, a, b, RP(ctx->bt)); ++ctx->nlaunch;
-  {
-    SpecIn<real> F;
-    F.op = SPEC_FILT;
-    F.filt = tab_filt(ctx);
-    F.x[0] = a;
-    F.x[1] = b;
-    F.x[2] = c;
-    real* out[3] = {G[PMPIC_GRID_P], G[PMPIC_GRID_Q], G[PMPIC_GRID_R]};
-    if ((rc = fft_inverse(ctx, 3, F, out, mids))) return rc;
-  }
-  if ((rc = zero_mode_launch(ctx, a, b))) return rc;
-  {
-    real* abc[3] = {a, b, c};
-    const bool df[3] = {false, false, true};
-    if ((rc = spec_laplinv_batch(ctx, 3, abc, df))) return rc;
-  }
-  const real* atop = RP(ctx->bt);
-  const real* abot = RP(ctx->bt) + cols;
-  const real* btop = RP(ctx->bt) + 2 * cols;
-  const real* bbot = RP(ctx->bt) + 3 * cols;
-  // dB/dz into e and dA/dz into d (:255, :284), in one launch
-  {
-    const real* zin[2] = {b, a};
-    real* zout[2] = {e, d};
-    const real* zbot[2] = {bbot, abot};
-    const real* ztop[2] = {btop, atop};
-    if ((rc = diffz_batch_impl(ctx, 2, zin, zout, zbot, ztop))) return rc;
-  }
-  // u = dB/dz - dC/dy (:251-276), v = dC/dx - dA/dz (:280-302) and
-  // w = dA/dy - dB/dx (:306-320): each velocity spectrum is formed as its
-  // inverse transform reads it, which also stores the filtered copy (u_s, v_s, w_s)
-  {
-    SpecIn<real> V;
-    V.op = SPEC_VEL;
-    V.x[0] = e;
-    V.y[0] = c;
-    V.x[1] = d;
-    V.y[1] = c;
-    V.x[2] = a;
-    V.y[2] = b;
-    V.fs[0] = RP(ctx->spec[PMPIC_SPEC_U]);
-    V.fs[1] = RP(ctx->spec[PMPIC_SPEC_V]);
-    V.fs[2] = RP(ctx->spec[PMPIC_SPEC_W]);
-    V.zbar[0] = ctx->zmode;
-    V.zbar[1] = ctx->zmode + g.nzp;
-    V.kx = tab_kx(ctx);
-    V.ky = tab_ky(ctx);
-    V.filt = tab_filt(ctx);
-    real* out[3] = {G[PMPIC_GRID_U], G[PMPIC_GRID_V], G[PMPIC_GRID_W]};
-    if ((rc = fft_inverse(ctx, 3, V, out, mids))) return rc;
-  }
-  PMPIC_CUDA(cudaGetLastError());
-  return 0;
+  if ((rc = invert_launch(ctx, a, b, c, u, v, w))) return rc;
+  // the corrected, filtered vorticity (:207-226) and the velocity (:251-320)
+  SpecIn<real> S;
+  const real* in[6] = {a, b, c, u, v, w};
+  real* out[6] = {G[PMPIC_GRID_P], G[PMPIC_GRID_Q], G[PMPIC_GRID_R], G[PMPIC_GRID_U], G[PMPIC_GRID_V], G[PMPIC_GRID_W]};
+  for (int q = 0; q < 6; ++q) S.x[q] = in[q];
+  return fft_inverse(ctx, 6, S, out, mids);
 }
 
 // vorticity_tendency.F90:147-265 (grid B holds par2grid(btot) on entry).  The
