@@ -320,8 +320,8 @@ struct pmpic_ctx {
   // physical grids (dense (Nz+1) x Ny x Nx)
   double* grid[PMPIC_NGRID];
   double* gwork[5];          // dudx, dwdx, dvdy, dwdy, ap
-  double* mixres[6];         // residual grids vres..rres
-  int32_t* npercell;         // ncell
+  double* mixres[6];         // residual grids vres..rres (one allocation)
+  int32_t* npercell;         // ncell (mixing): kept parcels, by cell id
   int32_t* newslot;          // ncell: slot of the new parcel of a cell or -1
   uint8_t* near;             // ncell (mixing): cell within one of a cell with a removed or a
                              // new parcel (its corners may hold residuals)

@@ -14,7 +14,6 @@
 namespace pmpic {
 
 int spectral_init(pmpic_ctx* ctx);
-int scan_excl(pmpic_ctx* ctx, const int32_t* in, int64_t n, int32_t* out);
 
 int cuda_fail(pmpic_ctx* ctx, cudaError_t e, const char* what, int line) {
   char buf[256];
@@ -129,8 +128,7 @@ void free_all(pmpic_ctx* c) {
     if (c->grid[i]) cudaFree(c->grid[i]);
   for (int i = 0; i < 5; ++i)
     if (c->gwork[i]) cudaFree(c->gwork[i]);
-  for (int i = 0; i < 6; ++i)
-    if (c->mixres[i]) cudaFree(c->mixres[i]);
+  if (c->mixres[0]) cudaFree(c->mixres[0]);
   for (int i = 0; i < PMPIC_NSPEC; ++i)
     if (c->spec[i]) cudaFree(c->spec[i]);
   if (c->hinfo) cudaFreeHost(c->hinfo);
@@ -275,7 +273,8 @@ int pmpic_create(const pmpic_config* cfg, pmpic_ctx** out) {
   if (!rc) rc = dalloc(ctx, (int32_t**)&ctx->scan_tmp, (size_t)(std::max<int64_t>(std::max<int64_t>(g.ncell, ctx->cap), ctx->nbmax) / 4096 + 64));
   for (int i = 0; i < PMPIC_NGRID && !rc; ++i) rc = dalloc(ctx, &ctx->grid[i], (size_t)g.nphys);
   for (int i = 0; i < 5 && !rc; ++i) rc = dalloc(ctx, &ctx->gwork[i], (size_t)g.nphys);
-  for (int i = 0; i < 6 && !rc; ++i) rc = dalloc(ctx, &ctx->mixres[i], (size_t)g.nphys);
+  if (!rc) rc = dalloc(ctx, &ctx->mixres[0], 6 * (size_t)g.nphys);
+  for (int i = 1; i < 6 && !rc; ++i) ctx->mixres[i] = ctx->mixres[0] + i * g.nphys;
   if (!rc) rc = dalloc(ctx, &ctx->npercell, (size_t)g.ncell);
   if (!rc) rc = dalloc(ctx, &ctx->newslot, (size_t)g.ncell);
   if (!rc) rc = dalloc(ctx, &ctx->near, (size_t)g.ncell);

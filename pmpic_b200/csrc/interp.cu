@@ -89,11 +89,6 @@ __global__ void k_bin_count_m(Geom g, int64_t n, const int32_t* __restrict__ cel
 // coalesced load each, mostly L1 hits) and the run's extent there is read off
 // two ballots; only a run reaching past them is followed further slot by slot.
 constexpr int SC_ITEMS = 4;
-// the total of counts kept current by other kernels against the parcel count
-// (a mismatch would leave the cell index inconsistent: reported as an error)
-__global__ void k_check_total(const int32_t* __restrict__ total, int64_t n, DevInfo* info) {
-  if (*total != n) atomicCAS(&info->error, 0, PMPIC_ERR_STATE);
-}
 __global__ void __launch_bounds__(256) k_bin_scatter(int64_t n, const int32_t* __restrict__ cell,
                                                      const int32_t* __restrict__ count,
                                                      const int32_t* __restrict__ start, int32_t* __restrict__ fill,
@@ -208,7 +203,10 @@ __global__ void __launch_bounds__(SORT_CELLS) k_sort_segments(int64_t ncell, con
   }
 }
 
-// ---- exclusive scan of int32 counts (three-phase) ----------------------------
+// ---- exclusive scan of int32 counts ---------------------------------------------
+// Up to SCAN_DIRECT tiles in one launch, every CTA summing the tiles before its
+// own itself (at most 1 MB out of L2, less than two more launches take: 9 -> 4
+// us at 32^3 cells); three phases beyond.
 constexpr int SCAN_BLOCK = 1024;
 constexpr int SCAN_ITEMS = 4;
 constexpr int SCAN_TILE = SCAN_BLOCK * SCAN_ITEMS;
@@ -251,7 +249,50 @@ __global__ void k_scan_tiles(const int32_t* __restrict__ in, int64_t n, int32_t*
   if (threadIdx.x == 0) tile_sums[blockIdx.x] = total;
 }
 
-__global__ void k_scan_sums(int32_t* __restrict__ sums, int64_t ntiles, int32_t* __restrict__ grand) {
+// the grand total against the expected one (expect >= 0): counts kept current by
+// other kernels must add up to the parcels, or the cell index would be
+// inconsistent
+__device__ __forceinline__ void check_total(int total, int64_t expect, DevInfo* info) {
+  if (expect >= 0 && total != expect) atomicCAS(&info->error, 0, PMPIC_ERR_STATE);
+}
+constexpr int SCAN_DIRECT = 64;
+// (zero: an array of n values cleared on the way, or null)
+__global__ void __launch_bounds__(SCAN_BLOCK) k_scan_direct(const int32_t* __restrict__ in, int64_t n,
+                                                            int32_t* __restrict__ out, int32_t* __restrict__ zero,
+                                                            int64_t expect, DevInfo* info) {
+  __shared__ int sh[32];
+  const int64_t b0 = (int64_t)blockIdx.x * SCAN_TILE;
+  int s = 0, before, total;
+  for (int64_t i = threadIdx.x; i < b0 / 4; i += SCAN_BLOCK) {
+    const int4 v = reinterpret_cast<const int4*>(in)[i];  // (device allocations are 256-byte aligned)
+    s += v.x + v.y + v.z + v.w;
+  }
+  block_excl_scan(s, sh, before);
+  const int64_t base = b0 + (int64_t)threadIdx.x * SCAN_ITEMS;
+  int v[SCAN_ITEMS];
+  s = 0;
+#pragma unroll
+  for (int q = 0; q < SCAN_ITEMS; ++q) {
+    v[q] = (base + q < n) ? in[base + q] : 0;
+    s += v[q];
+  }
+  int ex = block_excl_scan(s, sh, total) + before;
+#pragma unroll
+  for (int q = 0; q < SCAN_ITEMS; ++q) {
+    if (base + q < n) {
+      out[base + q] = ex;
+      if (zero) zero[base + q] = 0;
+    }
+    ex += v[q];
+  }
+  if (blockIdx.x == gridDim.x - 1 && threadIdx.x == 0) {
+    out[n] = before + total;
+    check_total(before + total, expect, info);
+  }
+}
+
+__global__ void k_scan_sums(int32_t* __restrict__ sums, int64_t ntiles, int32_t* __restrict__ grand, int64_t expect,
+                            DevInfo* info) {
   __shared__ int sh[32];
   int carry = 0;
   for (int64_t b0 = 0; b0 < ntiles; b0 += blockDim.x) {
@@ -262,11 +303,14 @@ __global__ void k_scan_sums(int32_t* __restrict__ sums, int64_t ntiles, int32_t*
     if (i < ntiles) sums[i] = carry + ex;
     carry += total;
   }
-  if (threadIdx.x == 0 && grand) *grand = carry;
+  if (threadIdx.x == 0) {
+    *grand = carry;
+    check_total(carry, expect, info);
+  }
 }
 
 __global__ void k_scan_apply(const int32_t* __restrict__ in, int64_t n, const int32_t* __restrict__ tile_off,
-                             int32_t* __restrict__ out) {
+                             int32_t* __restrict__ out, int32_t* __restrict__ zero) {
   __shared__ int sh[32];
   int64_t base = (int64_t)blockIdx.x * SCAN_TILE + (int64_t)threadIdx.x * SCAN_ITEMS;
   int v[SCAN_ITEMS];
@@ -280,9 +324,25 @@ __global__ void k_scan_apply(const int32_t* __restrict__ in, int64_t n, const in
   int ex = block_excl_scan(s, sh, total) + tile_off[blockIdx.x];
 #pragma unroll
   for (int q = 0; q < SCAN_ITEMS; ++q) {
-    if (base + q < n) out[base + q] = ex;
+    if (base + q < n) {
+      out[base + q] = ex;
+      if (zero) zero[base + q] = 0;
+    }
     ex += v[q];
   }
+}
+void scan_launch(const int32_t* in, int64_t n, int32_t* out, int32_t* zero, int64_t expect, DevInfo* info,
+                 int32_t* sums, cudaStream_t st, int64_t& nlaunch) {
+  const int64_t ntiles = (n + SCAN_TILE - 1) / SCAN_TILE;
+  if (ntiles <= SCAN_DIRECT) {
+    k_scan_direct<<<(unsigned)std::max<int64_t>(ntiles, 1), SCAN_BLOCK, 0, st>>>(in, n, out, zero, expect, info);
+    ++nlaunch;
+    return;
+  }
+  k_scan_tiles<<<(unsigned)ntiles, SCAN_BLOCK, 0, st>>>(in, n, sums);
+  k_scan_sums<<<1, SCAN_BLOCK, 0, st>>>(sums, ntiles, out + n, expect, info);
+  k_scan_apply<<<(unsigned)ntiles, SCAN_BLOCK, 0, st>>>(in, n, sums, out, zero);
+  nlaunch += 3;
 }
 
 // ---- par2grid reduction ----------------------------------------------------------
@@ -539,7 +599,7 @@ __global__ void __launch_bounds__(32 * RW, sizeof(R) == 4 ? 6 : 4) k_p2g_rows(Ge
 #pragma unroll
           for (int q = 0; q < NA; ++q) dst[b * half + q * NLV] = C[b][q] + acc[2 * b][q];
       }
-      if (MODE == 1 && cz == 0 && has_cell) a.npercell[((int64_t)(k0 + kk) * g.Ny + cy) * g.Nx + cx] = nkept;
+      if (MODE == 1 && cz == 0 && has_cell) a.npercell[((int64_t)cx * g.Ny + cy) * g.Nz + k0 + kk] = nkept;
     }
 #pragma unroll
     for (int b = 0; b < 2; ++b)
@@ -828,27 +888,11 @@ __global__ void k_grid2par(Geom g, int64_t n, const int32_t* __restrict__ cell, 
 
 }  // namespace
 
-// exclusive scan of n int32 values; out[n] receives the total
-int scan_excl(pmpic_ctx* ctx, const int32_t* in, int64_t n, int32_t* out) {
-  int64_t ntiles = (n + SCAN_TILE - 1) / SCAN_TILE;
-  int32_t* sums = (int32_t*)ctx->scan_tmp;
-  if (ntiles > 0) {
-    k_scan_tiles<<<(unsigned)ntiles, SCAN_BLOCK, 0, ctx->stream>>>(in, n, sums); ++ctx->nlaunch;
-  }
-  k_scan_sums<<<1, SCAN_BLOCK, 0, ctx->stream>>>(sums, ntiles, out + n); ++ctx->nlaunch;
-  if (ntiles > 0) {
-    k_scan_apply<<<(unsigned)ntiles, SCAN_BLOCK, 0, ctx->stream>>>(in, n, sums, out); ++ctx->nlaunch;
-  }
-  PMPIC_CUDA(cudaGetLastError());
-  return 0;
-}
-
 // cache_parcel_interp_weights + the cell-ordered index: valid until positions change
 int bin_and_sort(pmpic_ctx* ctx) {
   TimerScope ts(ctx, T_CACHE);
   const Geom& g = ctx->g;
   const int64_t n = ctx->n;
-  PMPIC_CUDA(cudaMemsetAsync(ctx->cell_fill, 0, sizeof(int32_t) * g.ncell, ctx->stream));
   // on the mixed form, after an RK4 stage and its haloswap, a split or
   // mixing, the cell ids and counts are current already (kept by the kernels
   // that moved, added or removed parcels)
@@ -866,11 +910,8 @@ int bin_and_sort(pmpic_ctx* ctx) {
     }
   }
   ctx->count_ready = false;
-  int rc = scan_excl(ctx, ctx->cell_count, g.ncell, ctx->cell_start);
-  if (rc) return rc;
-  if (counted) {  // the maintained counts must add up to the parcels
-    k_check_total<<<1, 1, 0, ctx->stream>>>(ctx->cell_start + g.ncell, n, ctx->dinfo); ++ctx->nlaunch;
-  }
+  scan_launch(ctx->cell_count, g.ncell, ctx->cell_start, ctx->cell_fill, counted ? n : -1, ctx->dinfo,
+              (int32_t*)ctx->scan_tmp, ctx->stream, ctx->nlaunch);
   if (n > 0) {
     k_bin_scatter<<<nblk(n, 256 * SC_ITEMS), 256, 0, ctx->stream>>>(n, ctx->cell, ctx->cell_count, ctx->cell_start,
                                                                     ctx->cell_fill, ctx->sorted, ctx->cap); ++ctx->nlaunch;
@@ -998,8 +1039,7 @@ size_t rowpart_bytes(const Geom& g) {
 // kept grids into VOL, B, HG, P, Q, R (as the reference reuses state%vol,
 // state%b, state%hg, state%p, ...), residual grids into mixres, npercell.
 // With no parcel in the removed class (any_removed false) its sums are all
-// +0.0, which a memset gives without a pass over the parcels, and the kept
-// volume grid (and npercell) is made in full, the five other kept grids only
+// +0.0, left to a memset where they are read, and the kept volume grid (and npercell) is made in full, the five other kept grids only
 // where mixing reads them (launch_kept_corners).
 int launch_mix_grids(pmpic_ctx* ctx, bool any_removed) {
   if (ctx->mixed) {
@@ -1013,9 +1053,7 @@ int launch_mix_grids(pmpic_ctx* ctx, bool any_removed) {
     float* res[6];
     for (int q = 0; q < 6; ++q) res[q] = (float*)ctx->mixres[q];
     if (any_removed) return launch_p2g_m<6, 2>(ctx, f, res);
-    for (int q = 0; q < 6; ++q)
-      PMPIC_CUDA(cudaMemsetAsync(res[q], 0, sizeof(float) * ctx->g.nphys, ctx->stream));
-    return 0;
+    return 0;  // (the residual grids are cleared once an event is known)
   }
   const double* f[6] = {nullptr, prop(ctx, PMPIC_PROP_B), prop(ctx, PMPIC_PROP_H),
                         prop(ctx, PMPIC_PROP_P), prop(ctx, PMPIC_PROP_Q), prop(ctx, PMPIC_PROP_R)};
@@ -1024,8 +1062,6 @@ int launch_mix_grids(pmpic_ctx* ctx, bool any_removed) {
   int rc = any_removed ? launch_p2g<6, 1, false>(ctx, f, kept) : launch_p2g<1, 1, false>(ctx, f, kept);
   if (rc) return rc;
   if (any_removed) return launch_p2g<6, 2, false>(ctx, f, ctx->mixres);
-  for (int q = 0; q < 6; ++q)
-    PMPIC_CUDA(cudaMemsetAsync(ctx->mixres[q], 0, sizeof(double) * ctx->g.nphys, ctx->stream));
   return 0;
 }
 
@@ -1270,14 +1306,11 @@ extern "C" int pmpic_par2grid_static(int32_t nx, int32_t ny, int32_t nz, double 
 
   // the counters and the error word must start at zero: cleared on every call
   if (cudaMemsetAsync(count, 0, sizeof(int32_t) * (ncell + 1), st) != cudaSuccess) return PMPIC_ERR_CUDA;
-  if (cudaMemsetAsync(fill, 0, sizeof(int32_t) * ncell, st) != cudaSuccess) return PMPIC_ERR_CUDA;
   if (cudaMemsetAsync(info, 0, sizeof(DevInfo), st) != cudaSuccess) return PMPIC_ERR_CUDA;
   if (n > 0)
     k_bin_count<<<nblk(n, 256), 256, 0, st>>>(g, n, x, y, z, cell, del, SP_MAX_PARCELS, count, info);
-  const int64_t ntiles = (ncell + SCAN_TILE - 1) / SCAN_TILE;
-  k_scan_tiles<<<(unsigned)ntiles, SCAN_BLOCK, 0, st>>>(count, ncell, tiles);
-  k_scan_sums<<<1, SCAN_BLOCK, 0, st>>>(tiles, ntiles, cstart + ncell);
-  k_scan_apply<<<(unsigned)ntiles, SCAN_BLOCK, 0, st>>>(count, ncell, tiles, cstart);
+  int64_t nl = 0;
+  scan_launch(count, ncell, cstart, fill, -1, info, tiles, st, nl);
   if (n > 0) {
     k_bin_scatter<<<nblk(n, 256 * SC_ITEMS), 256, 0, st>>>(n, cell, count, cstart, fill, sorted, SP_MAX_PARCELS);
     k_sort_segments<<<nblk(ncell, SORT_CELLS), SORT_CELLS, 0, st>>>(ncell, cstart, fill, sorted);

@@ -12,7 +12,6 @@
 
 namespace pmpic {
 
-int scan_excl(pmpic_ctx* ctx, const int32_t* in, int64_t n, int32_t* out);
 int launch_mix_grids(pmpic_ctx* ctx, bool any_removed);
 int launch_kept_corners(pmpic_ctx* ctx, const int32_t* olist, const int32_t* nnew, int64_t hnew);
 
@@ -55,13 +54,48 @@ __global__ void __launch_bounds__(256) k_count(Pred pr, int64_t n, int32_t* __re
     blockcnt[blockIdx.x] = t;
   }
 }
+// sum of m counts over a CTA of 256 threads
+__device__ __forceinline__ int cta_sum(const int32_t* __restrict__ c, int64_t m, int* ws) {
+  int s = 0;
+  for (int64_t i = threadIdx.x; i < m; i += 256) s += c[i];
+#pragma unroll
+  for (int o = 16; o > 0; o >>= 1) s += __shfl_down_sync(0xffffffffu, s, o);
+  __syncthreads();
+  if ((threadIdx.x & 31) == 0) ws[threadIdx.x >> 5] = s;
+  __syncthreads();
+  s = 0;
+  for (int w = 0; w < 8; ++w) s += ws[w];
+  return s;
+}
+// what a haloswap's list needs besides its count: the count clamped to the
+// staging capacity (beyond it nothing is moved and the call reports the error)
+struct SwapCheck {
+  int32_t* nclamped = nullptr;  // null: no haloswap
+  int64_t swapcap = 0;
+  DevInfo* info = nullptr;
+};
+// The list from the per-CTA counts.  A CTA with a true item sums the counts
+// before its own itself (no scan between the two passes), CTA 0 the total.
 template <class Pred>
-__global__ void __launch_bounds__(256) k_write(Pred pr, int64_t n, const int32_t* __restrict__ blockoff,
-                                               int32_t* __restrict__ list) {
+__global__ void __launch_bounds__(256) k_write(Pred pr, int64_t n, const int32_t* __restrict__ blockcnt,
+                                               int32_t* __restrict__ list, int32_t* __restrict__ dcount, SwapCheck sc) {
   __shared__ int wc[CCH * 8];  // per (chunk, warp): count, then exclusive offset within the CTA
+  __shared__ int ws[8];
+  if (blockIdx.x == 0) {
+    const int total = cta_sum(blockcnt, gridDim.x, ws);
+    if (threadIdx.x == 0) {
+      *dcount = total;
+      if (sc.nclamped) {
+        if (total > sc.swapcap) atomicCAS(&sc.info->error, 0, PMPIC_ERR_CAPACITY);
+        *sc.nclamped = total > sc.swapcap ? 0 : total;
+        sc.info->n_migrated = total;
+      }
+    }
+  }
   // the lists are sparse (movers, splits, removals, under-populated cells):
-  // a CTA whose range holds none leaves at once (blockoff has nb + 1 entries)
-  if (blockoff[blockIdx.x + 1] == blockoff[blockIdx.x]) return;
+  // a CTA whose range holds none leaves at once
+  if (blockcnt[blockIdx.x] == 0) return;
+  const int32_t off = cta_sum(blockcnt, blockIdx.x, ws);
   const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
   const int64_t base = (int64_t)blockIdx.x * CITEMS + threadIdx.x;
   uint32_t mask = 0;
@@ -95,7 +129,6 @@ __global__ void __launch_bounds__(256) k_write(Pred pr, int64_t n, const int32_t
     }
   }
   __syncthreads();
-  const int32_t off = blockoff[blockIdx.x];
   const unsigned lt = (1u << lane) - 1;
 #pragma unroll 8
   for (int j = 0; j < CCH; ++j) {
@@ -130,16 +163,11 @@ struct PredStretchM {
   const float* s;
   __device__ bool operator()(int64_t i) const { return s[i] > 4.f; }
 };
-// cell in the reference's loop order o = (i*Ny + j)*Nz + k (parcel_mixing.F90:160-162)
+// a cell with fewer than three kept parcels; the cell id is the reference's loop
+// order o = (i*Ny + j)*Nz + k (parcel_mixing.F90:160-162)
 struct PredNewCell {
   const int32_t* npc;
-  int Nx, Ny, Nz;
-  __device__ bool operator()(int64_t o) const {
-    int k = (int)(o % Nz);
-    int j = (int)((o / Nz) % Ny);
-    int i = (int)(o / ((int64_t)Nz * Ny));
-    return npc[((int64_t)k * Ny + j) * Nx + i] < 3;
-  }
+  __device__ bool operator()(int64_t o) const { return npc[o] < 3; }
 };
 
 // ---- packed gather grids ------------------------------------------------------------
@@ -148,46 +176,79 @@ struct PredNewCell {
 // repacks the six into G6[i][j][k][6] (z fastest, fields interleaved): a cell's
 // four xy corners then hold their two levels and six fields in 12 consecutive
 // values, and the cells of a warp (consecutive in z) share lines.
-// x extent of a tile: 64 values (256-byte row segments) on the FP32 form, 32
-// on the FP64 path (its tile would not fit the static shared memory)
-template <class R>
-struct PkT {
-  static constexpr int value = sizeof(R) == 4 ? 64 : 32;
+// A CTA turns a tile of 32 x by 16 levels of the six fields round in shared
+// memory, reading and writing pairs of values (nx is even, and a record is
+// three pairs): bound by HBM, 1.6 GB at 256^3 FP32.  Before the stage kernel
+// that follows it also clears two arrays of counters (null: none).
+constexpr int PK_T = 32, PK_K = 16;
+struct Zero2 {
+  int32_t* p[2];
+  int64_t n[2];
 };
-constexpr int PK_K = 16;  // z extent of a tile
 template <class R>
-__global__ void __launch_bounds__(256) k_pack(Geom g, const R* __restrict__ G0, const R* __restrict__ G1,
-                                              const R* __restrict__ G2, const R* __restrict__ G3,
-                                              const R* __restrict__ G4, const R* __restrict__ G5,
-                                              R* __restrict__ out) {
-  constexpr int NF = 6;
-  constexpr int PK_T = PkT<R>::value;
-  constexpr int TS = PK_K * (PK_T + 1) + 1;  // per-field tile stride, odd
+struct Pair;
+template <>
+struct Pair<float> {
+  using T = float2;
+};
+template <>
+struct Pair<double> {
+  using T = double2;
+};
+template <class R>
+struct Six {
+  const R* g[6];
+};
+template <class R>
+__global__ void __launch_bounds__(256) k_pack(Geom g, Six<R> S, R* __restrict__ out, Zero2 z) {
+  using R2 = typename Pair<R>::T;
+  constexpr int NF = 6, KS = PK_T + 1;
+  constexpr int TS = PK_K * KS + 1;  // per-field tile stride
   __shared__ R tile[NF * TS];
-  const int i0 = blockIdx.x * PK_T, k0 = blockIdx.y * PK_K, j = blockIdx.z;
-  const R* G[NF] = {G0, G1, G2, G3, G4, G5};
-  const int ni = min(PK_T, g.Nx - i0), nk = min(PK_K, g.nzp - k0);
+  {
+    const int64_t b = ((int64_t)blockIdx.z * gridDim.y + blockIdx.y) * gridDim.x + blockIdx.x;
+    const int64_t step = (int64_t)gridDim.x * gridDim.y * gridDim.z * 256;
 #pragma unroll
-  for (int f = 0; f < NF; ++f) {
-    for (int e = threadIdx.x; e < PK_K * PK_T; e += blockDim.x) {
-      const int kk = e / PK_T, ii = e - kk * PK_T;
-      if (kk < nk && ii < ni) tile[f * TS + kk * (PK_T + 1) + ii] = G[f][((size_t)(k0 + kk) * g.Ny + j) * g.Nx + i0 + ii];
+    for (int q = 0; q < 2; ++q)
+      for (int64_t i = b * 256 + threadIdx.x; i < z.n[q]; i += step) z.p[q][i] = 0;
+  }
+  const int i0 = blockIdx.x * PK_T, k0 = blockIdx.y * PK_K, j = blockIdx.z;
+  const int ni = min(PK_T, g.Nx - i0), nk = min(PK_K, g.nzp - k0);
+  const int t = threadIdx.x;
+  {
+    const int ii = 2 * (t % 16), kk = t / 16;  // 16 pairs by 16 levels
+    if (ii < ni && kk < nk) {
+      const size_t o = ((size_t)(k0 + kk) * g.Ny + j) * g.Nx + i0 + ii;
+      R2 v[NF];
+#pragma unroll
+      for (int f = 0; f < NF; ++f) v[f] = *reinterpret_cast<const R2*>(S.g[f] + o);
+#pragma unroll
+      for (int f = 0; f < NF; ++f) {
+        tile[f * TS + kk * KS + ii] = v[f].x;
+        tile[f * TS + kk * KS + ii + 1] = v[f].y;
+      }
     }
   }
   __syncthreads();
-  for (int e = threadIdx.x; e < NF * PK_K * PK_T; e += blockDim.x) {
-    const int ii = e / (NF * PK_K), r = e - ii * NF * PK_K;
-    const int kk = r / NF, f = r - kk * NF;
-    if (kk < nk && ii < ni)
-      out[(((size_t)(i0 + ii) * g.Ny + j) * g.nzp + k0 + kk) * NF + f] = tile[f * TS + kk * (PK_T + 1) + ii];
+  constexpr int RP = PK_K * NF / 2;  // pairs of an x's run of levels
+#pragma unroll
+  for (int u = 0; u < PK_T * RP / 256; ++u) {
+    const int e = t + 256 * u, ii = e / RP, r = e - ii * RP, kk = r / 3, f = 2 * (r - 3 * kk);
+    if (kk < nk && ii < ni) {
+      R2 v;
+      v.x = tile[f * TS + kk * KS + ii];
+      v.y = tile[(f + 1) * TS + kk * KS + ii];
+      *reinterpret_cast<R2*>(out + (((size_t)(i0 + ii) * g.Ny + j) * g.nzp + k0 + kk) * NF + f) = v;
+    }
   }
 }
 template <class R>
-static void pack6(pmpic_ctx* ctx, const R* const* grids, R* out) {
+static void pack6(pmpic_ctx* ctx, const R* const* grids, R* out, const Zero2& z) {
   const Geom& g = ctx->g;
-  constexpr int PK_T = PkT<R>::value;
   dim3 gr((g.Nx + PK_T - 1) / PK_T, (g.nzp + PK_K - 1) / PK_K, g.Ny);
-  k_pack<R><<<gr, 256, 0, ctx->stream>>>(g, grids[0], grids[1], grids[2], grids[3], grids[4], grids[5], out);
+  Six<R> S;
+  for (int f = 0; f < 6; ++f) S.g[f] = grids[f];
+  k_pack<R><<<gr, 256, 0, ctx->stream>>>(g, S, out, z);
   ++ctx->nlaunch;
 }
 // the six fields at the two levels of xy corner (ci, cj) of a cell of level ck:
@@ -634,16 +695,6 @@ __global__ void k_swap_scatter(const int32_t* __restrict__ nmov, const int32_t* 
     parcels[(size_t)c_swap_props[q] * cap + V[t]] = buf[e];
   }
 }
-__global__ void k_check_swapcap(const int32_t* nmov, int32_t* nclamped, int64_t swapcap, DevInfo* info) {
-  int nm = *nmov;
-  if (nm > swapcap) {
-    atomicCAS(&info->error, 0, PMPIC_ERR_CAPACITY);
-    nm = 0;  // nothing is moved; the call reports the capacity error
-  }
-  *nclamped = nm;
-  info->n_migrated = *nmov;
-}
-
 // ---- parcel splitting (parcel_splitting.F90:64-133) -----------------------------------
 __global__ void k_split_flag(int64_t n, double* __restrict__ parcels, int64_t cap, const double* __restrict__ dtp,
                              int32_t* __restrict__ flag) {
@@ -1580,40 +1631,22 @@ __global__ void k_prescribed_velocity(int64_t n, double* __restrict__ parcels, i
 
 }  // namespace
 
-// list of i in [0,n) with pred(i), ascending; count written to *dcount (device)
+// list of i in [0,n) with pred(i), ascending; count written to *dcount (device).
+// counted: the per-CTA counts are in ctx->aux2 already (written by the kernel
+// that computed the predicate's input).
 template <class Pred>
-static int compact(pmpic_ctx* ctx, Pred pr, int64_t n, int32_t* list, int32_t* dcount) {
+static int compact(pmpic_ctx* ctx, Pred pr, int64_t n, int32_t* list, int32_t* dcount, bool counted = false,
+                   const SwapCheck& sc = SwapCheck{}) {
   int64_t nb = (n + CITEMS - 1) / CITEMS;
   if (nb == 0) {
     PMPIC_CUDA(cudaMemsetAsync(dcount, 0, sizeof(int32_t), ctx->stream));
     return 0;
   }
-  int32_t* cnt = ctx->aux2;            // nb + 1 (nb + 1 <= nbmax)
-  int32_t* off = ctx->aux2 + ctx->nbmax;
-  k_count<<<(unsigned)nb, 256, 0, ctx->stream>>>(pr, n, cnt); ++ctx->nlaunch;
-  int rc = scan_excl(ctx, cnt, nb, off);
-  if (rc) return rc;
-  k_write<<<(unsigned)nb, 256, 0, ctx->stream>>>(pr, n, off, list); ++ctx->nlaunch;
-  PMPIC_CUDA(cudaMemcpyAsync(dcount, off + nb, sizeof(int32_t), cudaMemcpyDeviceToDevice, ctx->stream));
-  PMPIC_CUDA(cudaGetLastError());
-  return 0;
-}
-
-// the same with the per-CTA counts already in ctx->aux2 (written by the
-// kernel that computed the predicate's input)
-template <class Pred>
-static int compact_counted(pmpic_ctx* ctx, Pred pr, int64_t n, int32_t* list, int32_t* dcount) {
-  int64_t nb = (n + CITEMS - 1) / CITEMS;
-  if (nb == 0) {
-    PMPIC_CUDA(cudaMemsetAsync(dcount, 0, sizeof(int32_t), ctx->stream));
-    return 0;
+  int32_t* cnt = ctx->aux2;  // nb <= nbmax
+  if (!counted) {
+    k_count<<<(unsigned)nb, 256, 0, ctx->stream>>>(pr, n, cnt); ++ctx->nlaunch;
   }
-  int32_t* cnt = ctx->aux2;
-  int32_t* off = ctx->aux2 + ctx->nbmax;
-  int rc = scan_excl(ctx, cnt, nb, off);
-  if (rc) return rc;
-  k_write<<<(unsigned)nb, 256, 0, ctx->stream>>>(pr, n, off, list); ++ctx->nlaunch;
-  PMPIC_CUDA(cudaMemcpyAsync(dcount, off + nb, sizeof(int32_t), cudaMemcpyDeviceToDevice, ctx->stream));
+  k_write<<<(unsigned)nb, 256, 0, ctx->stream>>>(pr, n, cnt, list, dcount, sc); ++ctx->nlaunch;
   PMPIC_CUDA(cudaGetLastError());
   return 0;
 }
@@ -1715,10 +1748,14 @@ int rk4_stage(pmpic_ctx* ctx, int stage) {
     P.inv[2] = (float)(1.0 / ctx->g.dz);
     P.g6 = (const float*)ctx->gpack;
     P.whint = ctx->whint;
-    if (gu && gp) pack6<float>(ctx, P.grid, (float*)ctx->gpack);
+    // the next binning's cell counts and the mover counts start at zero
+    const Zero2 z{{ctx->cell_count, ctx->aux2}, {ctx->g.ncell + 1, ctx->nbmax}};
+    if (gu && gp) {
+      pack6<float>(ctx, P.grid, (float*)ctx->gpack, z);
+    } else {
+      for (int q = 0; q < 2; ++q) PMPIC_CUDA(cudaMemsetAsync(z.p[q], 0, sizeof(int32_t) * z.n[q], ctx->stream));
+    }
     auto kern = gu ? (gp ? k_rk4_m<true, true> : k_rk4_m<true, false>) : (gp ? k_rk4_m<false, true> : k_rk4_m<false, false>);
-    PMPIC_CUDA(cudaMemsetAsync(ctx->cell_count, 0, sizeof(int32_t) * (ctx->g.ncell + 1), ctx->stream));
-    PMPIC_CUDA(cudaMemsetAsync(ctx->aux2, 0, sizeof(int32_t) * ctx->nbmax, ctx->stream));  // mover counts
     // within pmpic_step the last stage also advances the stretch of the split
     // that follows (the haloswap in between moves it with its parcel)
     const bool adv = ctx->split_follows && stage == 4;
@@ -1753,12 +1790,13 @@ int rk4_stage(pmpic_ctx* ctx, int stage) {
   if ((gu || gp) && !ctx->sorted_valid) return set_error(ctx, PMPIC_ERR_STATE, "deferred gather without binning");
   P.g6 = ctx->gpack;
   P.whint = ctx->whint;
-  if (gu && gp) pack6<double>(ctx, P.grid, ctx->gpack);
+  const Zero2 z{{ctx->aux2, nullptr}, {ctx->nbmax, 0}};  // the mover counts
+  if (gu && gp) pack6<double>(ctx, P.grid, ctx->gpack, z);
+  else PMPIC_CUDA(cudaMemsetAsync(z.p[0], 0, sizeof(int32_t) * z.n[0], ctx->stream));
   auto kern = gu ? (gp ? k_rk4<true, true> : k_rk4<true, false>) : (gp ? k_rk4<false, true> : k_rk4<false, false>);
   // the next binning stays a separate pass on this path: its six IEEE
   // divisions per parcel cost the HBM-bound stage kernel more than the
   // position reads they would save
-  PMPIC_CUDA(cudaMemsetAsync(ctx->aux2, 0, sizeof(int32_t) * ctx->nbmax, ctx->stream));  // mover counts
   kern<<<nblk(ctx->n, 256), 256, 0, ctx->stream>>>(ctx->g, ctx->n, P, stage, &ctx->dinfo->dtm, ctx->cell, ctx->del,
                                                    ctx->cap, ctx->dir, store_tendencies(ctx, stage), ctx->aux2); ++ctx->nlaunch;
   ctx->pending_uvw = ctx->pending_pqr = false;
@@ -1799,13 +1837,12 @@ int parcel_haloswap(pmpic_ctx* ctx) {
   int32_t* M = ctx->keep;                // moved parcels in send order (keep is free outside mixing)
   int32_t* nm = dcounter(ctx, 0);
   // after an RK4 stage or a split, the kernel that classified counted the movers
-  int rc = ready ? compact_counted(ctx, PredDirNZ{ctx->dir}, n, V, nm) : compact(ctx, PredDirNZ{ctx->dir}, n, V, nm);
-  if (rc) return rc;
-  k_partition_dirs<<<1, 1024, 0, ctx->stream>>>(V, nm, ctx->dir, M); ++ctx->nlaunch;
   // the staging buffer is bounded: on overflow nothing moves and the call
   // reports PMPIC_ERR_CAPACITY
   int32_t* nmc = dcounter(ctx, 1);
-  k_check_swapcap<<<1, 1, 0, ctx->stream>>>(nm, nmc, ctx->swapcap, ctx->dinfo); ++ctx->nlaunch;
+  int rc = compact(ctx, PredDirNZ{ctx->dir}, n, V, nm, ready, SwapCheck{nmc, ctx->swapcap, ctx->dinfo});
+  if (rc) return rc;
+  k_partition_dirs<<<1, 1024, 0, ctx->stream>>>(V, nm, ctx->dir, M); ++ctx->nlaunch;
   if (ctx->mixed) {
     k_swap_gather_m<<<592, 256, 0, ctx->stream>>>(ctx->g, nmc, M, ctx->dir, ctx->parcels, ctx->cap, ctx->cell,
                                                    ctx->swapbuf); ++ctx->nlaunch;
@@ -1829,7 +1866,6 @@ int splitting(pmpic_ctx* ctx) {
   int32_t* ns = dcounter(ctx, 2);
   const bool advanced = ctx->stretch_advanced;
   ctx->stretch_advanced = false;
-  bool split_counted = false;
   if (n > 0) {
     int rc;
     if (advanced) {  // the RK4 stage advanced the stretch: only the criterion is left
@@ -1843,17 +1879,37 @@ int splitting(pmpic_ctx* ctx) {
       rc = compact(ctx, PredFlag{flag}, n, list, ns);
     }
     if (rc) return rc;
-    // after a haloswap only the split parcels can be outside the domain: the
-    // haloswap that follows needs no pass over all parcels to find them.  The
-    // mixed form's positions are always inside (kept wrapped and reflected).
+  } else {
+    PMPIC_CUDA(cudaMemsetAsync(ns, 0, sizeof(int32_t), ctx->stream));
+  }
+  int32_t hns = 0;
+  PMPIC_CUDA(cudaMemcpyAsync(&hns, ns, sizeof(int32_t), cudaMemcpyDeviceToHost, ctx->stream));
+  PMPIC_CUDA(cudaStreamSynchronize(ctx->stream));
+  const int64_t nn = n + hns;
+  // after a haloswap only the split parcels can be outside the domain: the
+  // haloswap that follows needs no pass over all parcels to find them.  The
+  // mixed form's positions are always inside (kept wrapped and reflected).
+  const bool inside = ctx->in_domain || ctx->mixed;
+  // on the mixed form the binning counts stay current through the split
+  const bool keep_counts = n > 0 && ctx->mixed && ctx->count_ready;
+  ctx->count_ready = keep_counts;  // else split parents move and children are added uncounted
+  if (n > 0 && hns == 0 && inside) {
+    // nothing split: nothing moves either, and the haloswap (:134) would find no parcel
+    PMPIC_CUDA(cudaMemsetAsync(&ctx->dinfo->n_migrated, 0, sizeof(long long), ctx->stream));
+    ctx->sorted_valid = false;
+    ctx->btot_grid_ready = false;
+    ctx->dir_ready = false;
+    ctx->in_domain = true;
+    ctx->info.n_split = 0;
+    return 0;
+  }
+  if (n > 0) {
     int8_t* dsplit = nullptr;
-    if (ctx->in_domain || ctx->mixed) {
+    if (inside) {
       PMPIC_CUDA(cudaMemsetAsync(ctx->dir, 0, (size_t)n, ctx->stream));
       PMPIC_CUDA(cudaMemsetAsync(ctx->aux2, 0, sizeof(int32_t) * ctx->nbmax, ctx->stream));  // mover counts
       dsplit = ctx->dir;
     }
-    // on the mixed form the binning counts stay current through the split
-    const bool keep_counts = ctx->mixed && ctx->count_ready;
     if (ctx->mixed)
       k_split_apply_m<<<592, 256, 0, ctx->stream>>>(ctx->g, n, list, ns, ctx->parcels, ctx->cap, ctx->dinfo, dsplit,
                                                     ctx->aux2, ctx->cell, keep_counts ? ctx->cell_count : nullptr);
@@ -1862,15 +1918,7 @@ int splitting(pmpic_ctx* ctx) {
                                                   ctx->aux2);
     ++ctx->nlaunch;
     ctx->dir_ready = dsplit != nullptr;
-    split_counted = keep_counts;
-  } else {
-    PMPIC_CUDA(cudaMemsetAsync(ns, 0, sizeof(int32_t), ctx->stream));
   }
-  int32_t hns = 0;
-  PMPIC_CUDA(cudaMemcpyAsync(&hns, ns, sizeof(int32_t), cudaMemcpyDeviceToHost, ctx->stream));
-  PMPIC_CUDA(cudaStreamSynchronize(ctx->stream));
-  int64_t nn = n + hns;
-  ctx->count_ready = split_counted;  // else split parents moved and children were added uncounted
   if (nn > ctx->cap) return set_error(ctx, PMPIC_ERR_CAPACITY, "maxparcels reached (parcel splitting)");
   ctx->n = nn;
   ctx->info.n_split = hns;
@@ -1964,7 +2012,7 @@ int mixing(pmpic_ctx* ctx) {
   // under-populated cells in loop order
   int32_t* olist = ctx->cell_fill;  // ncell entries; free after bin_and_sort
   int32_t* nnew = dcounter(ctx, 4);
-  if ((rc = compact(ctx, PredNewCell{ctx->npercell, g.Nx, g.Ny, g.Nz}, g.ncell, olist, nnew))) return rc;
+  if ((rc = compact(ctx, PredNewCell{ctx->npercell}, g.ncell, olist, nnew))) return rc;
   int32_t hnew = 0;
   PMPIC_CUDA(cudaMemcpyAsync(&hnew, nnew, sizeof(int32_t), cudaMemcpyDeviceToHost, ctx->stream));
   PMPIC_CUDA(cudaStreamSynchronize(ctx->stream));
@@ -1986,6 +2034,8 @@ int mixing(pmpic_ctx* ctx) {
     return 0;
   }
   PMPIC_CUDA(cudaMemsetAsync(ctx->newslot, 0xff, sizeof(int32_t) * g.ncell, ctx->stream));
+  if (hz0 == 0)  // the empty removed class's sums (launch_mix_grids)
+    PMPIC_CUDA(cudaMemsetAsync(ctx->mixres[0], 0, sizeof(double) * 6 * g.nphys, ctx->stream));
   double* K[6] = {ctx->grid[PMPIC_GRID_VOL], ctx->grid[PMPIC_GRID_B], ctx->grid[PMPIC_GRID_HG],
                   ctx->grid[PMPIC_GRID_P],   ctx->grid[PMPIC_GRID_Q], ctx->grid[PMPIC_GRID_R]};
   if (ctx->mixed) {

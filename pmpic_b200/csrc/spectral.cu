@@ -29,18 +29,15 @@ inline unsigned nblk(int64_t n, int b) { return (unsigned)((n + b - 1) / b); }
 // mean flow of the zero mode (vort2vel.F90:230-241), one thread: the trapezoid
 // integral and the reference's average (`1./nz` in REAL(4), 0.5*ubar(nz) added
 // to every element before the sum).
-// d, e: the zero-mode values of level k at d[k * stride], e[k * stride],
-// multiplied by the filter's zero-mode factor *filt when filt is given (the
-// filtered d = filter(a), e = filter(b) of vort2vel.F90:208-209)
-__global__ void k_zmode(Geom g, const double* __restrict__ d, const double* __restrict__ e, int64_t stride,
-                        const double* __restrict__ filt, double* __restrict__ zb) {
+// d, e: the zero-mode values of each level
+__global__ void k_zmode(Geom g, const double* __restrict__ d, const double* __restrict__ e, double* __restrict__ zb) {
   extern __shared__ double zs[];  // e(:,1,1), d(:,1,1), then ubar, vbar
   const int nz = g.nzp;
   double* es = zs;
   double* ds = zs + nz;
   for (int k = threadIdx.x; k < nz; k += blockDim.x) {  // stage the zero-mode columns
-    es[k] = filt ? e[k * stride] * filt[0] : e[k * stride];
-    ds[k] = filt ? d[k * stride] * filt[0] : d[k * stride];
+    es[k] = e[k];
+    ds[k] = d[k];
   }
   __syncthreads();
   if (threadIdx.x != 0) return;
@@ -82,9 +79,22 @@ __global__ void __launch_bounds__(256) k_hsum2(Geom g, const float* __restrict__
   const float* P = p + (size_t)k * m;
   const float* Q = q + (size_t)k * m;
   double a = 0.0, b = 0.0;
-  for (int64_t e = threadIdx.x; e < m; e += 256) {
-    a += (double)P[e];
-    b += (double)Q[e];
+  // (loads of eight terms in flight, added in the one order)
+  constexpr int U = 8;
+  for (int64_t e0 = threadIdx.x; e0 < m; e0 += 256 * U) {
+    float pv[U], qv[U];
+#pragma unroll
+    for (int u = 0; u < U; ++u) {
+      const int64_t e = e0 + 256 * u;
+      pv[u] = e < m ? P[e] : 0.f;
+      qv[u] = e < m ? Q[e] : 0.f;
+    }
+#pragma unroll
+    for (int u = 0; u < U; ++u)
+      if (e0 + 256 * u < m) {
+        a += (double)pv[u];
+        b += (double)qv[u];
+      }
   }
   sp[threadIdx.x] = a;
   sq[threadIdx.x] = b;
@@ -485,7 +495,7 @@ inline int zero_mode(pmpic_ctx* ctx) {
   const Geom& g = ctx->g;
   k_hsum2<<<g.nzp, 256, 0, ctx->stream>>>(g, (const float*)ctx->grid[PMPIC_GRID_P], (const float*)ctx->grid[PMPIC_GRID_Q],
                                           ctx->hsum); ++ctx->nlaunch;
-  k_zmode<<<1, 256, sizeof(double) * 4 * g.nzp, ctx->stream>>>(g, ctx->hsum, ctx->hsum + g.nzp, 1, nullptr, ctx->zmode); ++ctx->nlaunch;
+  k_zmode<<<1, 256, sizeof(double) * 4 * g.nzp, ctx->stream>>>(g, ctx->hsum, ctx->hsum + g.nzp, ctx->zmode); ++ctx->nlaunch;
   PMPIC_CUDA(cudaGetLastError());
   return 0;
 }
@@ -522,7 +532,12 @@ int spectral_init(pmpic_ctx* ctx) {
   PMPIC_CUDA(cudaMemcpy(ctx->wn32, t32.data(), sizeof(float) * t32.size(), cudaMemcpyHostToDevice));
   PMPIC_CUDA(cudaMalloc(&ctx->hsum, sizeof(double) * 2 * g.nzp));
   if ((rc = laplinv_tables(ctx, tabs.data() + 2 * cols))) return rc;
-  if (ctx->mixed) return f32::invert_init(ctx);
+  if (ctx->mixed) {
+    const size_t zs = sizeof(double) * 4 * (size_t)nz;  // k_zmode's columns
+    if (zs > 48 * 1024)
+      PMPIC_CUDA(cudaFuncSetAttribute(k_zmode, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)zs));
+    return f32::invert_init(ctx);
+  }
   // the FP64 inversion's reciprocal pivots, from the pivots of both solvers
   const int64_t n = (int64_t)(g.sx >> 1) * (g.sy >> 1) * nz;
   PMPIC_CUDA(cudaMalloc(&ctx->zrec, sizeof(double) * (4 * nz + 4 * n)));

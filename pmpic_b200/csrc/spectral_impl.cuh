@@ -467,6 +467,18 @@ int invert_launch(pmpic_ctx* ctx, real* a, real* b, real* c, real* u, real* v, r
   return 0;
 }
 
+// a CTA's maximum into *out (one atomic per CTA)
+__device__ __forceinline__ void cta_max(real m, double* __restrict__ out) {
+  __shared__ real sh[8];
+  for (int o = 16; o > 0; o >>= 1) m = fmax(m, __shfl_down_sync(0xffffffffu, m, o));
+  __syncthreads();
+  if ((threadIdx.x & 31) == 0) sh[threadIdx.x >> 5] = m;
+  __syncthreads();
+  if (threadIdx.x == 0) {
+    for (int w = 1; w < 8; ++w) m = fmax(m, sh[w]);
+    atomicMax((unsigned long long*)out, __double_as_longlong((double)m));
+  }
+}
 // max of squares over the interior (vort2vel.F90:331-338,
 // vorticity_tendency.F90:279-282); non-negative doubles order like their bits
 __global__ void k_max_sq3(int64_t n, const real* __restrict__ u, const real* __restrict__ v,
@@ -478,16 +490,9 @@ __global__ void k_max_sq3(int64_t n, const real* __restrict__ u, const real* __r
     mv = fmax(mv, b * b);
     mw = fmax(mw, c * c);
   }
-  for (int o = 16; o > 0; o >>= 1) {
-    mu = fmax(mu, __shfl_down_sync(0xffffffffu, mu, o));
-    mv = fmax(mv, __shfl_down_sync(0xffffffffu, mv, o));
-    mw = fmax(mw, __shfl_down_sync(0xffffffffu, mw, o));
-  }
-  if ((threadIdx.x & 31) == 0) {
-    atomicMax((unsigned long long*)&out3[0], __double_as_longlong((double)mu));
-    atomicMax((unsigned long long*)&out3[1], __double_as_longlong((double)mv));
-    atomicMax((unsigned long long*)&out3[2], __double_as_longlong((double)mw));
-  }
+  cta_max(mu, &out3[0]);
+  cta_max(mv, &out3[1]);
+  cta_max(mw, &out3[2]);
 }
 __global__ void k_max_vort(int64_t n, const real* __restrict__ p, const real* __restrict__ q,
                            const real* __restrict__ r, double* __restrict__ out) {
@@ -496,8 +501,7 @@ __global__ void k_max_vort(int64_t n, const real* __restrict__ p, const real* __
     real a = p[e], b = q[e], c = r[e];
     m = fmax(m, a * a + b * b + c * c);
   }
-  for (int o = 16; o > 0; o >>= 1) m = fmax(m, __shfl_down_sync(0xffffffffu, m, o));
-  if ((threadIdx.x & 31) == 0) atomicMax((unsigned long long*)out, __double_as_longlong((double)m));
+  cta_max(m, out);
 }
 
 // vort2vel.F90:139-320 after the three par2grid calls (grids P, Q, R hold the
