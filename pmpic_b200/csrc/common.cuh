@@ -5,6 +5,7 @@
 #include <stdint.h>
 
 #include <string>
+#include <utility>
 #include <vector>
 
 #include "../../include/pmpic_gpu.h"
@@ -16,6 +17,37 @@
   } while (0)
 
 namespace pmpic {
+
+// Programmatic dependent launch: a kernel is set up while the one before it on
+// the stream still runs, and waits for its end and for what it wrote in
+// PDL_WAIT, the first statement of every kernel here.  On small grids a step
+// is a chain of about a hundred kernels of a few microseconds, whose gaps this
+// shortens: 0.83 -> 0.63 ms a step at 32^3 FP64, 2.87 -> 2.64 at 96^3 FP32,
+// 38.7 -> 38.4 at 256^3 FP32.  (Letting the next kernel's CTAs in as soon as
+// the last ones of this kernel have begun was slower: 0.65, 2.69, 41.0.)
+// The branch that is never taken (the compiler cannot know it) ends the entry
+// block after the wait, so that no load, not even one of constant data, is
+// moved up before it.
+#define PDL_WAIT()                                                                     \
+  do {                                                                                 \
+    int never_;                                                                        \
+    asm volatile("griddepcontrol.wait;\n\tmov.u32 %0, 0;" : "=r"(never_)::"memory"); \
+    if (never_) return;                                                                \
+  } while (0)
+template <class... P, class... A>
+inline void launch(cudaStream_t st, dim3 grid, dim3 block, size_t smem, void (*kern)(P...), A&&... args) {
+  cudaLaunchConfig_t c{};
+  c.gridDim = grid;
+  c.blockDim = block;
+  c.dynamicSmemBytes = smem;
+  c.stream = st;
+  cudaLaunchAttribute at{};
+  at.id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  at.val.programmaticStreamSerializationAllowed = 1;
+  c.attrs = &at;
+  c.numAttrs = 1;
+  cudaLaunchKernelEx(&c, kern, std::forward<A>(args)...);
+}
 
 // Fortran single-precision literals promoted to double (fft_ops.F90:427-429,
 // :512-513, parcel_splitting.F90:71,79, vort2vel.F90:237-238).
@@ -294,6 +326,7 @@ struct pmpic_ctx {
                              // (parcel_splitting.F90:64-73) for the split that follows
   bool in_domain;            // every parcel is inside the domain (set by the parcel haloswap,
                              // cleared by any change of positions): a split moves only its own
+  bool count_zero;           // cell_count is zero (cleared by the last RK4 stage's packing)
   bool count_ready;          // mixed form: cell ids and per-cell counts were written by the
                              // last RK4 stage and haloswap, so binning starts at the scan
   bool btot_grid_ready;      // gspare holds par2grid(btot) of the current substep

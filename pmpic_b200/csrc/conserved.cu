@@ -52,6 +52,7 @@ __device__ __forceinline__ DD dd_add_prod(DD acc, double a, double b) {
 template <class R>
 __global__ void __launch_bounds__(CS_THREADS) k_sums(int64_t n, const R* __restrict__ vol, const R* __restrict__ h,
                                                       const R* __restrict__ b, double* __restrict__ part) {
+  PDL_WAIT();
   DD s0{0.0, 0.0}, s1{0.0, 0.0}, s2{0.0, 0.0};
   const int64_t stride = (int64_t)gridDim.x * CS_THREADS;
   for (int64_t i = (int64_t)blockIdx.x * CS_THREADS + threadIdx.x; i < n; i += stride) {
@@ -80,6 +81,7 @@ __global__ void __launch_bounds__(CS_THREADS) k_sums(int64_t n, const R* __restr
 // one warp per quantity: lane l sums the partials of blocks l, l + 32, ... in
 // order, then a fixed butterfly over the lanes
 __global__ void k_sums_final(int nblocks, const double* __restrict__ part, DevInfo* info) {
+  PDL_WAIT();
   const int q = threadIdx.x >> 5, lane = threadIdx.x & 31;
   if (q >= 3) return;
   DD s{0.0, 0.0};
@@ -97,13 +99,13 @@ int conserved_sums(pmpic_ctx* ctx) {
   const int64_t n = ctx->n;
   const int nb = (int)std::min<int64_t>(CS_BLOCKS, std::max<int64_t>(1, (n + CS_THREADS - 1) / CS_THREADS));
   if (ctx->mixed) {
-    k_sums<float><<<nb, CS_THREADS, 0, ctx->stream>>>(n, propf(ctx, PMPIC_PROP_VOL), propf(ctx, PMPIC_PROP_H),
-                                                       propf(ctx, PMPIC_PROP_B), ctx->csum);
+    launch(ctx->stream, nb, CS_THREADS, 0, k_sums<float>, n, propf(ctx, PMPIC_PROP_VOL), propf(ctx, PMPIC_PROP_H),
+           propf(ctx, PMPIC_PROP_B), ctx->csum);
   } else {
-    k_sums<double><<<nb, CS_THREADS, 0, ctx->stream>>>(n, prop(ctx, PMPIC_PROP_VOL), prop(ctx, PMPIC_PROP_H),
-                                                        prop(ctx, PMPIC_PROP_B), ctx->csum);
+    launch(ctx->stream, nb, CS_THREADS, 0, k_sums<double>, n, prop(ctx, PMPIC_PROP_VOL), prop(ctx, PMPIC_PROP_H),
+           prop(ctx, PMPIC_PROP_B), ctx->csum);
   }
-  k_sums_final<<<1, 96, 0, ctx->stream>>>(nb, ctx->csum, ctx->dinfo);
+  launch(ctx->stream, 1, 96, 0, k_sums_final, nb, ctx->csum, ctx->dinfo);
   ctx->nlaunch += 2;
   PMPIC_CUDA(cudaGetLastError());
   return 0;

@@ -233,7 +233,7 @@ int pmpic_create(const pmpic_config* cfg, pmpic_ctx** out) {
   ctx->cap = cfg->max_parcels;
   ctx->n = 0;
   ctx->sorted_valid = false;
-  ctx->count_ready = false;
+  ctx->count_ready = ctx->count_zero = false;
   ctx->in_domain = false;
   ctx->btot_grid_ready = false;
   ctx->pending_uvw = ctx->pending_pqr = ctx->dir_ready = false;
@@ -368,6 +368,7 @@ struct ConvIn {
   DevInfo* info;
 };
 __global__ void k_conv_in(Geom g, int64_t n, const double* __restrict__ src, void* __restrict__ dst, ConvIn c) {
+  PDL_WAIT();
   const int64_t t = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
   if (t >= n) return;
   const double v = src ? src[t] : 0.0;
@@ -407,6 +408,7 @@ struct ConvOut {
   const int32_t* cell;   // MK_CUR
 };
 __global__ void k_conv_out(Geom g, int64_t n, const void* __restrict__ src, double* __restrict__ dst, ConvOut c) {
+  PDL_WAIT();
   const int64_t t = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
   if (t >= n) return;
   switch (c.kind) {
@@ -430,10 +432,12 @@ __global__ void k_conv_out(Geom g, int64_t n, const void* __restrict__ src, doub
   }
 }
 __global__ void k_f2d(int64_t n, const float* __restrict__ src, double* __restrict__ dst) {
+  PDL_WAIT();
   const int64_t t = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
   if (t < n) dst[t] = (double)src[t];
 }
 __global__ void k_d2f(int64_t n, const double* __restrict__ src, float* __restrict__ dst) {
+  PDL_WAIT();
   const int64_t t = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
   if (t < n) dst[t] = (float)src[t];
 }
@@ -484,7 +488,7 @@ int pmpic::prop_upload(pmpic_ctx* ctx, int pid, int64_t off, int64_t n, const do
       PMPIC_CUDA(cudaEventRecord(ctx->xfull[i & 1], ctx->xstream));
       PMPIC_CUDA(cudaStreamWaitEvent(ctx->stream, ctx->xfull[i & 1], 0));
     }
-    k_conv_in<<<cblk(len), 256, 0, ctx->stream>>>(ctx->g, len, src ? buf : nullptr, base + es * c0, c);
+    launch(ctx->stream, cblk(len), 256, 0, k_conv_in, ctx->g, len, src ? buf : nullptr, base + es * c0, c);
     ++ctx->nlaunch;
     if (src) PMPIC_CUDA(cudaEventRecord(ctx->xfree[i & 1], ctx->stream));
   }
@@ -513,7 +517,7 @@ int pmpic::prop_download(pmpic_ctx* ctx, int pid, int64_t off, int64_t n, double
     c.base = propc(ctx, PMPIC_PROP_XO + c.axis) + off + c0;
     c.cell = ctx->cell + off + c0;
     PMPIC_CUDA(cudaStreamWaitEvent(ctx->stream, ctx->xfree[i & 1], 0));  // its last copy is done
-    k_conv_out<<<cblk(len), 256, 0, ctx->stream>>>(ctx->g, len, base + es * c0, buf, c);
+    launch(ctx->stream, cblk(len), 256, 0, k_conv_out, ctx->g, len, base + es * c0, buf, c);
     ++ctx->nlaunch;
     PMPIC_CUDA(cudaEventRecord(ctx->xfull[i & 1], ctx->stream));
     PMPIC_CUDA(cudaStreamWaitEvent(ctx->xstream, ctx->xfull[i & 1], 0));
@@ -638,7 +642,7 @@ int pmpic_download_grid(pmpic_ctx* ctx, int grid, double* dst) {
   if (!ctx || grid < 0 || grid >= PMPIC_NGRID || !dst) return PMPIC_ERR_ARG;
   cudaSetDevice(ctx->device);
   if (ctx->mixed) {  // FP32 grid widened into the spare grid first
-    k_f2d<<<cblk(ctx->g.nphys), 256, 0, ctx->stream>>>(ctx->g.nphys, (const float*)ctx->grid[grid], ctx->gspare);
+    launch(ctx->stream, cblk(ctx->g.nphys), 256, 0, k_f2d, ctx->g.nphys, (const float*)ctx->grid[grid], ctx->gspare);
     ++ctx->nlaunch;
     ctx->btot_grid_ready = false;  // gspare is overwritten
     PMPIC_CUDA(cudaMemcpyAsync(dst, ctx->gspare, sizeof(double) * ctx->g.nphys, cudaMemcpyDeviceToHost, ctx->stream));
@@ -653,7 +657,7 @@ int pmpic_upload_grid(pmpic_ctx* ctx, int grid, const double* src) {
   cudaSetDevice(ctx->device);
   if (ctx->mixed) {
     PMPIC_CUDA(cudaMemcpyAsync(ctx->gspare, src, sizeof(double) * ctx->g.nphys, cudaMemcpyHostToDevice, ctx->stream));
-    k_d2f<<<cblk(ctx->g.nphys), 256, 0, ctx->stream>>>(ctx->g.nphys, ctx->gspare, (float*)ctx->grid[grid]);
+    launch(ctx->stream, cblk(ctx->g.nphys), 256, 0, k_d2f, ctx->g.nphys, ctx->gspare, (float*)ctx->grid[grid]);
     ++ctx->nlaunch;
     ctx->btot_grid_ready = false;
   } else {
@@ -666,7 +670,7 @@ int pmpic_download_spectral(pmpic_ctx* ctx, int spec, double* dst) {
   if (!ctx || spec < 0 || spec >= PMPIC_NSPEC || !dst) return PMPIC_ERR_ARG;
   cudaSetDevice(ctx->device);
   if (ctx->mixed) {
-    k_f2d<<<cblk(ctx->g.nspec), 256, 0, ctx->stream>>>(ctx->g.nspec, (const float*)ctx->spec[spec], ctx->sscratch);
+    launch(ctx->stream, cblk(ctx->g.nspec), 256, 0, k_f2d, ctx->g.nspec, (const float*)ctx->spec[spec], ctx->sscratch);
     ++ctx->nlaunch;
     PMPIC_CUDA(cudaMemcpyAsync(dst, ctx->sscratch, sizeof(double) * ctx->g.nspec, cudaMemcpyDeviceToHost, ctx->stream));
   } else {
@@ -1065,6 +1069,7 @@ int pmpic_op_grid2par_multi(pmpic_ctx* ctx, int ng, const int* grids, const int*
 namespace {
 __global__ void k_permute(int64_t n, const int32_t* __restrict__ perm, const void* __restrict__ src,
                           void* __restrict__ dst, int es) {
+  PDL_WAIT();
   const int64_t q = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
   if (q >= n) return;
   if (es == 8) ((double*)dst)[q] = ((const double*)src)[perm[q]];
@@ -1088,7 +1093,7 @@ int pmpic_sort_parcels(pmpic_ctx* ctx) {
     if (p == PMPIC_NPROP && !ctx->mixed) break;
     void* col = p < PMPIC_NPROP ? (void*)prop(ctx, p) : (void*)ctx->cell;
     const int es = p == PMPIC_NPROP ? 4 : (ctx->mixed ? mixed_elem_bytes(p) : 8);
-    k_permute<<<cblk(n), 256, 0, ctx->stream>>>(n, ctx->sorted, col, tmp, es);
+    launch(ctx->stream, cblk(n), 256, 0, k_permute, n, ctx->sorted, col, tmp, es);
     ++ctx->nlaunch;
     cudaError_t e = cudaMemcpyAsync(col, tmp, (size_t)es * n, cudaMemcpyDeviceToDevice, ctx->stream);
     if (e != cudaSuccess) rc = cuda_fail(ctx, e, "cudaMemcpyAsync", __LINE__);

@@ -57,6 +57,7 @@ struct File {
 template <class R>
 __global__ void k_dump_field(Geom g, const R* __restrict__ src, const R* __restrict__ h, int mode,
                              double* __restrict__ dst) {
+  PDL_WAIT();
   const int64_t e = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
   if (e >= g.nphys) return;
   const int k = (int)(e % g.nzp);
@@ -107,9 +108,9 @@ int dump_grid_fields(pmpic_ctx* ctx, Emit&& emit) {
   const unsigned nb = (unsigned)((g.nphys + 255) / 256);
   for (int q = 0; q < 10; ++q) {
     if (ctx->mixed)
-      k_dump_field<float><<<nb, 256, 0, ctx->stream>>>(g, (const float*)src[q], (const float*)W[4], mode[q], stage);
+      launch(ctx->stream, nb, 256, 0, k_dump_field<float>, g, (const float*)src[q], (const float*)W[4], mode[q], stage);
     else
-      k_dump_field<double><<<nb, 256, 0, ctx->stream>>>(g, src[q], W[4], mode[q], stage);
+      launch(ctx->stream, nb, 256, 0, k_dump_field<double>, g, src[q], W[4], mode[q], stage);
     ++ctx->nlaunch;
     PMPIC_CUDA(cudaGetLastError());
     PMPIC_CUDA(cudaMemcpyAsync(host.data(), stage, sizeof(double) * g.nphys, cudaMemcpyDeviceToHost, ctx->stream));

@@ -98,6 +98,7 @@ __device__ real2* fft_rows(real2* buf0, real2* buf1, int nrows, int stride_row, 
 // CTA: one z level, TXF consecutive x columns (TXF/2 complex rows of length Ny).
 __global__ void __launch_bounds__(FFT_THREADS) k_fwd_y(Geom g, int TXF, FftPlan pl, const real2* __restrict__ tw,
                                                        const real* __restrict__ phys, real* __restrict__ mid) {
+  PDL_WAIT();
   extern __shared__ real2 sm[];
   const int Ny = g.Ny, Nx = g.Nx;
   const int nr = TXF / 2;
@@ -138,6 +139,7 @@ __global__ void __launch_bounds__(FFT_THREADS) k_fwd_y(Geom g, int TXF, FftPlan 
 __global__ void __launch_bounds__(FFT_THREADS) k_fwd_x(Geom g, int RP, int64_t nrows_total, FftPlan pl,
                                                        const real2* __restrict__ tw, const real* __restrict__ mid,
                                                        real* __restrict__ spec) {
+  PDL_WAIT();
   extern __shared__ real2 sm[];
   const int Nx = g.Nx;
   real2* b0 = sm;
@@ -276,6 +278,7 @@ template <int OP>
 __global__ void __launch_bounds__(FFT_THREADS) k_inv_x(Geom g, int RP, int64_t nrows_total, FftPlan pl,
                                                        const real2* __restrict__ tw, real* __restrict__ mid,
                                                        SpecIn<real> S, int q) {
+  PDL_WAIT();
   extern __shared__ real2 sm[];
   const int Nx = g.Nx;
   real2* b0 = sm;
@@ -311,6 +314,7 @@ __global__ void __launch_bounds__(FFT_THREADS) k_inv_x(Geom g, int RP, int64_t n
 __global__ void __launch_bounds__(FFT_THREADS) k_inv_y(Geom g, int TXF, FftPlan pl,
                                                        const real2* __restrict__ tw, const real* __restrict__ mid,
                                                        real* __restrict__ phys, PhysOut<real> E) {
+  PDL_WAIT();
   extern __shared__ real2 sm[];
   const int Ny = g.Ny, Nx = g.Nx;
   const int nr = TXF / 2;
@@ -550,6 +554,7 @@ template <int N1c, int N2c, bool ST>
 __global__ void __launch_bounds__(FS_THREADS) k4_fwd_x(Geom g, int n1, int n2_, int64_t nrows,
                                                        const real2* __restrict__ tw4, Arr6<const real> mids,
                                                        Arr6<real> specs) {
+  PDL_WAIT();
   const int N1 = N1c ? N1c : n1, N2 = N2c ? N2c : n2_, N = N1 * N2;
   const int RP = FS_THREADS / (N1 > N2 ? N1 : N2), YS = N1 * (N2 + 1);
   __shared__ real2 Y[fs_xvals(N1c, N2c)];
@@ -607,6 +612,7 @@ template <int N1c, int N2c, bool ST, int OP>
 __global__ void __launch_bounds__(FS_THREADS, sizeof(real) == 4 ? 5 : 3) k4_inv_x(Geom g, int n1, int n2_, int64_t nrows,
                                                        const real2* __restrict__ tw4, SpecIn<real> S,
                                                        Arr6<real> mids, Arr6<real> ymids) {
+  PDL_WAIT();
   const int N1 = N1c ? N1c : n1, N2 = N2c ? N2c : n2_, N = N1 * N2;
   const int RP = FS_THREADS / (N1 > N2 ? N1 : N2), YS = N1 * (N2 + 1);
   extern __shared__ real2 sm[];
@@ -679,6 +685,7 @@ template <int N1c, int N2c, bool ST>
 __global__ void __launch_bounds__(FS_YT) k4_fwd_y(Geom g, int n1, int n2_,
                                                        const real2* __restrict__ tw4, Arr6<const real> physs,
                                                        Arr6<real> mids) {
+  PDL_WAIT();
   const int N1 = N1c ? N1c : n1, N2 = N2c ? N2c : n2_, N = N1 * N2;
   constexpr int RP = FS_YV;
   const int YS = N1 * (N2 + 1) + 1, XS = N + 1;
@@ -766,6 +773,7 @@ template <int N1c, int N2c, bool ST>
 __global__ void __launch_bounds__(FS_YT) k4_inv_y(Geom g, int n1, int n2_,
                                                        const real2* __restrict__ tw4, Arr6<const real> mids,
                                                        Arr6<real> physs) {
+  PDL_WAIT();
   const int N1 = N1c ? N1c : n1, N2 = N2c ? N2c : n2_, N = N1 * N2;
   constexpr int RP = FS_YV;
   const int YS = N1 * (N2 + 1) + 1;
@@ -812,6 +820,7 @@ struct VtArgs {
 template <int N1c, int N2c, bool ST>
 __global__ void __launch_bounds__(FS_YT, sizeof(real) == 4 ? 2 : 4) k4_vt_y(Geom g, int n1, int n2_,
                                                       const real2* __restrict__ tw4, const __grid_constant__ VtArgs V) {
+  PDL_WAIT();
   const int N1 = N1c ? N1c : n1, N2 = N2c ? N2c : n2_, N = N1 * N2;
   constexpr int RP = FS_YV;
   constexpr bool MEM = sizeof(real) == 8;  // the sums wait in memory
@@ -921,15 +930,15 @@ int fft_forward_impl(pmpic_ctx* ctx, int nb, const real* const* phys, real* cons
   if (py.n1) {
     const dim3 gr((g.Nx + 2 * FS_YV - 1) / (2 * FS_YV), g.nzp, nb);
     fs_dispatch(py.n1, py.n2, py.st, [&](auto a, auto b, auto c) {
-      k4_fwd_y<decltype(a)::value, decltype(b)::value, decltype(c)::value><<<gr, FS_YV * std::max(py.n1, py.n2), 0, st>>>(g, py.n1, py.n2, twy + py.tw4_off,
-                                                                                     P, M);
+      launch(st, gr, FS_YV * std::max(py.n1, py.n2), 0, k4_fwd_y<decltype(a)::value, decltype(b)::value,
+             decltype(c)::value>, g, py.n1, py.n2, twy + py.tw4_off, P, M);
     });
     ++ctx->nlaunch;
   } else {
     const int txf = pick_txf(g.Nx);
     const size_t sm_y = sizeof(real2) * (size_t)(txf / 2) * g.Ny * 2;
     for (int b = 0; b < nb; ++b) {
-      k_fwd_y<<<dim3(g.Nx / txf, g.nzp), FFT_THREADS, sm_y, st>>>(g, txf, py, twy, phys[b], mids[b]);
+      launch(st, dim3(g.Nx / txf, g.nzp), FFT_THREADS, sm_y, k_fwd_y, g, txf, py, twy, phys[b], mids[b]);
       ++ctx->nlaunch;
     }
   }
@@ -937,16 +946,16 @@ int fft_forward_impl(pmpic_ctx* ctx, int nb, const real* const* phys, real* cons
     const int rp = fs_rows(px.n1, px.n2);
     const dim3 gr((unsigned)((nrows + 2 * rp - 1) / (2 * rp)), nb);
     fs_dispatch(px.n1, px.n2, px.st, [&](auto a, auto b, auto c) {
-      k4_fwd_x<decltype(a)::value, decltype(b)::value, decltype(c)::value><<<gr, FS_THREADS, 0, st>>>(g, px.n1, px.n2, nrows,
-                                                                                  tw + px.tw4_off, MC, Sp);
+      launch(st, gr, FS_THREADS, 0, k4_fwd_x<decltype(a)::value, decltype(b)::value, decltype(c)::value>, g, px.n1,
+             px.n2, nrows, tw + px.tw4_off, MC, Sp);
     });
     ++ctx->nlaunch;
   } else {
     const int rp = pick_rp(g.Nx);
     const size_t sm_x = sizeof(real2) * (size_t)rp * g.Nx * 2;
     for (int b = 0; b < nb; ++b) {
-      k_fwd_x<<<(unsigned)((nrows + 2 * rp - 1) / (2 * rp)), FFT_THREADS, sm_x, st>>>(g, rp, nrows, px, tw, mids[b],
-                                                                                       spec[b]);
+      launch(st, (unsigned)((nrows + 2 * rp - 1) / (2 * rp)), FFT_THREADS, sm_x, k_fwd_x, g, rp, nrows, px, tw,
+             mids[b], spec[b]);
       ++ctx->nlaunch;
     }
   }
@@ -975,7 +984,7 @@ void inv_x_pass(pmpic_ctx* ctx, int nb, const SpecIn<real>& S, real* const* mids
       constexpr int A = decltype(a)::value, B = decltype(b)::value;
       constexpr bool C = decltype(c)::value;
       auto go = [&](auto kern) {
-        kern<<<gr, FS_THREADS, sm, st>>>(g, px.n1, px.n2, nrows, tw + px.tw4_off, S, M, D);
+        launch(st, gr, FS_THREADS, sm, kern, g, px.n1, px.n2, nrows, tw + px.tw4_off, S, M, D);
       };
       switch (S.op) {
         case SPEC_PAIR: go(k4_inv_x<A, B, C, SPEC_PAIR>); break;
@@ -990,7 +999,7 @@ void inv_x_pass(pmpic_ctx* ctx, int nb, const SpecIn<real>& S, real* const* mids
   const unsigned nblk = (unsigned)((nrows + 2 * rp - 1) / (2 * rp));
   for (int b = 0; b < nb; ++b) {
     auto go = [&](auto kern, real* mid) {
-      kern<<<nblk, FFT_THREADS, sm, st>>>(g, rp, nrows, px, tw, mid, S, b);
+      launch(st, nblk, FFT_THREADS, sm, kern, g, rp, nrows, px, tw, mid, S, b);
       ++ctx->nlaunch;
     };
     switch (S.op) {
@@ -1009,7 +1018,7 @@ void inv_y_generic(pmpic_ctx* ctx, const real* mid, real* phys, const real2* twy
   const int txf = pick_txf(g.Nx);
   const size_t half = (size_t)g.Ny / 2 + 1;
   const size_t sm = sizeof(real2) * std::max((size_t)(txf / 2) * g.Ny * 2, (size_t)(txf / 2) * g.Ny + txf * half);
-  k_inv_y<<<dim3(g.Nx / txf, g.nzp), FFT_THREADS, sm, ctx->stream>>>(g, txf, ctx->plan_y, twy, mid, phys, E);
+  launch(ctx->stream, dim3(g.Nx / txf, g.nzp), FFT_THREADS, sm, k_inv_y, g, txf, ctx->plan_y, twy, mid, phys, E);
   ++ctx->nlaunch;
 }
 
@@ -1030,8 +1039,8 @@ int fft_inverse_impl(pmpic_ctx* ctx, int nb, const SpecIn<real>& S, real* const*
   if (py.n1) {
     const dim3 gr((g.Nx + 2 * FS_YV - 1) / (2 * FS_YV), g.nzp, nb);
     fs_dispatch(py.n1, py.n2, py.st, [&](auto a, auto b, auto c) {
-      k4_inv_y<decltype(a)::value, decltype(b)::value, decltype(c)::value><<<gr, FS_YV * std::max(py.n1, py.n2), 0, ctx->stream>>>(g, py.n1, py.n2,
-                                                                                              twy + py.tw4_off, M, P);
+      launch(ctx->stream, gr, FS_YV * std::max(py.n1, py.n2), 0, k4_inv_y<decltype(a)::value, decltype(b)::value,
+             decltype(c)::value>, g, py.n1, py.n2, twy + py.tw4_off, M, P);
     });
     ++ctx->nlaunch;
   } else {
@@ -1058,8 +1067,8 @@ int fft_tendency_impl(pmpic_ctx* ctx, const SpecIn<real>& S, const real* const* 
     const dim3 gr((g.Nx + 2 * FS_YV - 1) / (2 * FS_YV), g.nzp);
     const size_t sm = sizeof(real2) * 2 * FS_YV * (size_t)(py.n1 * (py.n2 + 1) + 1);
     fs_dispatch(py.n1, py.n2, py.st, [&](auto a, auto b, auto c) {
-      k4_vt_y<decltype(a)::value, decltype(b)::value, decltype(c)::value><<<gr, FS_YV * std::max(py.n1, py.n2), sm, ctx->stream>>>(
-          g, py.n1, py.n2, twy + py.tw4_off, V);
+      launch(ctx->stream, gr, FS_YV * std::max(py.n1, py.n2), sm, k4_vt_y<decltype(a)::value, decltype(b)::value,
+             decltype(c)::value>,  g, py.n1, py.n2, twy + py.tw4_off, V);
     });
     ++ctx->nlaunch;
     PMPIC_CUDA(cudaGetLastError());

@@ -40,6 +40,7 @@ __global__ void k_bin_count(Geom g, int64_t n, const double* __restrict__ X, con
                             const double* __restrict__ Z, int32_t* __restrict__ cell, double* __restrict__ del,
                             int64_t cap, int32_t* __restrict__ count, DevInfo* info,
                             int32_t* __restrict__ whint = nullptr) {
+  PDL_WAIT();
   int64_t t = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
   if (t >= n) return;
   int ci, cj, ck;
@@ -63,6 +64,7 @@ __global__ void k_bin_count(Geom g, int64_t n, const double* __restrict__ X, con
 __global__ void k_bin_count_m(Geom g, int64_t n, const int32_t* __restrict__ cell, const float* __restrict__ FX,
                               const float* __restrict__ FY, const float* __restrict__ FZ,
                               int32_t* __restrict__ count, DevInfo* info) {
+  PDL_WAIT();
   int64_t t = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
   if (t >= n) return;
   const int32_t id = cell[t];
@@ -93,6 +95,7 @@ __global__ void __launch_bounds__(256) k_bin_scatter(int64_t n, const int32_t* _
                                                      const int32_t* __restrict__ count,
                                                      const int32_t* __restrict__ start, int32_t* __restrict__ fill,
                                                      int32_t* __restrict__ sorted, int64_t lim) {
+  PDL_WAIT();
   constexpr unsigned FULL = 0xffffffffu;
   const int lane = threadIdx.x & 31;
   const int64_t t0 = (int64_t)blockIdx.x * 256 * SC_ITEMS + threadIdx.x;
@@ -172,6 +175,7 @@ constexpr int SORT_RANK = 16, SORT_RANK_MAX = 512;  // entries of a cell that is
 __global__ void __launch_bounds__(SORT_CELLS) k_sort_segments(int64_t ncell, const int32_t* __restrict__ start,
                                                               const int32_t* __restrict__ fill,
                                                               int32_t* __restrict__ sorted) {
+  PDL_WAIT();
   // staged position e sits at e + e/8: segments (~8 parcels each) start in
   // different banks for neighbouring threads
   __shared__ int32_t buf[SORT_CAP + SORT_CAP / 8];
@@ -256,6 +260,7 @@ __device__ __forceinline__ int block_excl_scan(int v, int* sh, int& total) {
 }
 
 __global__ void k_scan_tiles(const int32_t* __restrict__ in, int64_t n, int32_t* __restrict__ tile_sums) {
+  PDL_WAIT();
   __shared__ int sh[32];
   int64_t base = (int64_t)blockIdx.x * SCAN_TILE + (int64_t)threadIdx.x * SCAN_ITEMS;
   int s = 0;
@@ -278,6 +283,7 @@ constexpr int SCAN_DIRECT = 64;
 __global__ void __launch_bounds__(SCAN_BLOCK) k_scan_direct(const int32_t* __restrict__ in, int64_t n,
                                                             int32_t* __restrict__ out, int32_t* __restrict__ zero,
                                                             int64_t expect, DevInfo* info) {
+  PDL_WAIT();
   __shared__ int sh[32];
   const int64_t b0 = (int64_t)blockIdx.x * SCAN_TILE;
   int s = 0, before, total;
@@ -311,6 +317,7 @@ __global__ void __launch_bounds__(SCAN_BLOCK) k_scan_direct(const int32_t* __res
 
 __global__ void k_scan_sums(int32_t* __restrict__ sums, int64_t ntiles, int32_t* __restrict__ grand, int64_t expect,
                             DevInfo* info) {
+  PDL_WAIT();
   __shared__ int sh[32];
   int carry = 0;
   for (int64_t b0 = 0; b0 < ntiles; b0 += blockDim.x) {
@@ -329,6 +336,7 @@ __global__ void k_scan_sums(int32_t* __restrict__ sums, int64_t ntiles, int32_t*
 
 __global__ void k_scan_apply(const int32_t* __restrict__ in, int64_t n, const int32_t* __restrict__ tile_off,
                              int32_t* __restrict__ out, int32_t* __restrict__ zero) {
+  PDL_WAIT();
   __shared__ int sh[32];
   int64_t base = (int64_t)blockIdx.x * SCAN_TILE + (int64_t)threadIdx.x * SCAN_ITEMS;
   int v[SCAN_ITEMS];
@@ -353,13 +361,13 @@ void scan_launch(const int32_t* in, int64_t n, int32_t* out, int32_t* zero, int6
                  int32_t* sums, cudaStream_t st, int64_t& nlaunch) {
   const int64_t ntiles = (n + SCAN_TILE - 1) / SCAN_TILE;
   if (ntiles <= SCAN_DIRECT) {
-    k_scan_direct<<<(unsigned)std::max<int64_t>(ntiles, 1), SCAN_BLOCK, 0, st>>>(in, n, out, zero, expect, info);
+    launch(st, (unsigned)std::max<int64_t>(ntiles, 1), SCAN_BLOCK, 0, k_scan_direct, in, n, out, zero, expect, info);
     ++nlaunch;
     return;
   }
-  k_scan_tiles<<<(unsigned)ntiles, SCAN_BLOCK, 0, st>>>(in, n, sums);
-  k_scan_sums<<<1, SCAN_BLOCK, 0, st>>>(sums, ntiles, out + n, expect, info);
-  k_scan_apply<<<(unsigned)ntiles, SCAN_BLOCK, 0, st>>>(in, n, sums, out, zero);
+  launch(st, (unsigned)ntiles, SCAN_BLOCK, 0, k_scan_tiles, in, n, sums);
+  launch(st, 1, SCAN_BLOCK, 0, k_scan_sums, sums, ntiles, out + n, expect, info);
+  launch(st, (unsigned)ntiles, SCAN_BLOCK, 0, k_scan_apply, in, n, sums, out, zero);
   nlaunch += 3;
 }
 
@@ -458,6 +466,7 @@ __global__ void __launch_bounds__(32 * RW, sizeof(R) == 4 ? 6 : 4) k_p2g_rows(Ge
                                                      const R* __restrict__ DY, const R* __restrict__ DZ, int ds,
                                                      const R* __restrict__ VOL, P2GArgs<NQ, R> a,
                                                      R* __restrict__ rowpart) {
+  PDL_WAIT();
   using Lay = P2GLayout<NQ, MODE, BT>;
   constexpr int NA = Lay::NA, NS = Lay::NS;
   constexpr unsigned FULL = 0xffffffffu;
@@ -692,6 +701,7 @@ __global__ void __launch_bounds__(32 * RW, sizeof(R) == 4 ? 6 : 4) k_p2g_rows(Ge
 template <int NQ, int MODE, class R = double>
 __global__ void __launch_bounds__(256) k_p2g_combine(Geom g, int nzc, const R* __restrict__ rowpart,
                                                     P2GArgs<NQ, R> a) {
+  PDL_WAIT();
   constexpr int NA = MODE == 0 ? NQ + 1 : NQ;
   constexpr int SEG = NA * NLV;
   constexpr int TS = SEG | 1;  // odd stride: conflict-free reads by consecutive points
@@ -799,6 +809,7 @@ __global__ void __launch_bounds__(256) k_kept_corners(Geom g, const int32_t* __r
                                                       const int32_t* __restrict__ sorted, const R* __restrict__ DX,
                                                       const R* __restrict__ DY, const R* __restrict__ DZ,
                                                       const R* __restrict__ VOL, KeptCorners<R> a) {
+  PDL_WAIT();
   constexpr unsigned FULL = 0xffffffffu;
   const int lane = threadIdx.x & 31;
   const int u = threadIdx.x >> 5;  // the corner: x low/high, then y, then z
@@ -853,6 +864,7 @@ __global__ void __launch_bounds__(256) k_kept_corners(Geom g, const int32_t* __r
 
 // z-fastest cell id -> x-fastest id ((k*Ny + j)*Nx + i); -1 stays -1
 __global__ void k_cell_xfast(Geom g, int64_t n, const int32_t* __restrict__ cell, int32_t* __restrict__ out) {
+  PDL_WAIT();
   int64_t t = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
   if (t >= n) return;
   const int32_t id = cell[t];
@@ -874,6 +886,7 @@ struct G2PArgs {
 template <int NG>
 __global__ void k_grid2par(Geom g, int64_t n, const int32_t* __restrict__ cell, const double* __restrict__ del,
                            int64_t cap, G2PArgs<NG> a) {
+  PDL_WAIT();
   int64_t t = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
   if (t >= n) return;
   const int32_t id = cell[t];
@@ -916,25 +929,26 @@ int bin_and_sort(pmpic_ctx* ctx) {
   // that moved, added or removed parcels)
   const bool counted = ctx->count_ready;
   if (!counted) {
-    PMPIC_CUDA(cudaMemsetAsync(ctx->cell_count, 0, sizeof(int32_t) * (g.ncell + 1), ctx->stream));
+    if (!ctx->count_zero)
+      PMPIC_CUDA(cudaMemsetAsync(ctx->cell_count, 0, sizeof(int32_t) * (g.ncell + 1), ctx->stream));
     if (n > 0 && ctx->mixed) {
-      k_bin_count_m<<<nblk(n, 256), 256, 0, ctx->stream>>>(g, n, ctx->cell, curoff(ctx, 0), curoff(ctx, 1),
-                                                           curoff(ctx, 2), ctx->cell_count, ctx->dinfo);
+      launch(ctx->stream, nblk(n, 256), 256, 0, k_bin_count_m, g, n, ctx->cell, curoff(ctx, 0), curoff(ctx, 1),
+             curoff(ctx, 2), ctx->cell_count, ctx->dinfo);
       ++ctx->nlaunch;
     } else if (n > 0) {
-      k_bin_count<<<nblk(n, 256), 256, 0, ctx->stream>>>(g, n, prop(ctx, PMPIC_PROP_X), prop(ctx, PMPIC_PROP_Y),
-                                                         prop(ctx, PMPIC_PROP_Z), ctx->cell, ctx->del, ctx->cap,
-                                                         ctx->cell_count, ctx->dinfo, ctx->whint); ++ctx->nlaunch;
+      launch(ctx->stream, nblk(n, 256), 256, 0, k_bin_count, g, n, prop(ctx, PMPIC_PROP_X), prop(ctx, PMPIC_PROP_Y),
+             prop(ctx, PMPIC_PROP_Z), ctx->cell, ctx->del, ctx->cap, ctx->cell_count, ctx->dinfo,
+             ctx->whint); ++ctx->nlaunch;
     }
   }
-  ctx->count_ready = false;
+  ctx->count_ready = ctx->count_zero = false;
   scan_launch(ctx->cell_count, g.ncell, ctx->cell_start, ctx->cell_fill, counted ? n : -1, ctx->dinfo,
               (int32_t*)ctx->scan_tmp, ctx->stream, ctx->nlaunch);
   if (n > 0) {
-    k_bin_scatter<<<nblk(n, 256 * SC_ITEMS), 256, 0, ctx->stream>>>(n, ctx->cell, ctx->cell_count, ctx->cell_start,
-                                                                    ctx->cell_fill, ctx->sorted, ctx->cap); ++ctx->nlaunch;
-    k_sort_segments<<<nblk(g.ncell, SORT_CELLS), SORT_CELLS, 0, ctx->stream>>>(g.ncell, ctx->cell_start,
-                                                                               ctx->cell_fill, ctx->sorted);
+    launch(ctx->stream, nblk(n, 256 * SC_ITEMS), 256, 0, k_bin_scatter, n, ctx->cell, ctx->cell_count,
+           ctx->cell_start, ctx->cell_fill, ctx->sorted, ctx->cap); ++ctx->nlaunch;
+    launch(ctx->stream, nblk(g.ncell, SORT_CELLS), SORT_CELLS, 0, k_sort_segments, g.ncell, ctx->cell_start,
+           ctx->cell_fill, ctx->sorted);
     ++ctx->nlaunch;
   }
   PMPIC_CUDA(cudaGetLastError());
@@ -974,9 +988,9 @@ static cudaError_t run_p2g(const Geom& g, const int32_t* start, const int32_t* s
   cudaError_t e = cudaFuncSetAttribute(rows, cudaFuncAttributePreferredSharedMemoryCarveout,
                                        (int)cudaSharedmemCarveoutMaxShared);
   if (e != cudaSuccess) return e;
-  rows<<<nblk(nw, RW), 32 * RW, 0, st>>>(g, nzc, nxs, xseg, start, sorted, dx, dy, dz, ds, vol, a, rowpart);
+  launch(st, nblk(nw, RW), 32 * RW, 0, rows, g, nzc, nxs, xseg, start, sorted, dx, dy, dz, ds, vol, a, rowpart);
   dim3 gb((g.Nx + P2GPx<R>::value - 1) / P2GPx<R>::value, g.Ny, nzc);
-  k_p2g_combine<NQ, MODE, R><<<gb, 256, 0, st>>>(g, nzc, rowpart, a);
+  launch(st, gb, 256, 0, k_p2g_combine<NQ, MODE, R>, g, nzc, rowpart, a);
   return cudaGetLastError();
 }
 
@@ -1097,9 +1111,8 @@ int launch_kept_corners(pmpic_ctx* ctx, const int32_t* olist, const int32_t* nne
       k.out[q] = (float*)ctx->grid[pg[q]];
     }
     k.vmin = (double)(float)ctx->g.vmin;
-    k_kept_corners<float><<<(unsigned)hnew, 256, 0, ctx->stream>>>(ctx->g, olist, nnew, ctx->cell_start, ctx->sorted,
-                                                                  curoff(ctx, 0), curoff(ctx, 1), curoff(ctx, 2),
-                                                                  propf(ctx, PMPIC_PROP_VOL), k);
+    launch(ctx->stream, (unsigned)hnew, 256, 0, k_kept_corners<float>, ctx->g, olist, nnew, ctx->cell_start,
+           ctx->sorted, curoff(ctx, 0), curoff(ctx, 1), curoff(ctx, 2), propf(ctx, PMPIC_PROP_VOL), k);
   } else {
     KeptCorners<double> k;
     for (int q = 0; q < 5; ++q) {
@@ -1108,9 +1121,8 @@ int launch_kept_corners(pmpic_ctx* ctx, const int32_t* olist, const int32_t* nne
     }
     k.vmin = ctx->g.vmin;
     const double* del = ctx->del;  // the binning made at the start of mixing
-    k_kept_corners<double><<<(unsigned)hnew, 256, 0, ctx->stream>>>(ctx->g, olist, nnew, ctx->cell_start, ctx->sorted,
-                                                                   del, del + ctx->cap, del + 2 * ctx->cap,
-                                                                   prop(ctx, PMPIC_PROP_VOL), k);
+    launch(ctx->stream, (unsigned)hnew, 256, 0, k_kept_corners<double>, ctx->g, olist, nnew, ctx->cell_start,
+           ctx->sorted, del, del + ctx->cap, del + 2 * ctx->cap, prop(ctx, PMPIC_PROP_VOL), k);
   }
   ++ctx->nlaunch;
   PMPIC_CUDA(cudaGetLastError());
@@ -1145,7 +1157,7 @@ static int launch_g2p(pmpic_ctx* ctx, const double* const* grids, double* const*
     a.grid[q] = grids[q];
     a.out[q] = out[q];
   }
-  k_grid2par<NG><<<nblk(ctx->n, 256), 256, 0, ctx->stream>>>(g, ctx->n, ctx->cell, ctx->del, ctx->cap, a);
+  launch(ctx->stream, nblk(ctx->n, 256), 256, 0, k_grid2par<NG>, g, ctx->n, ctx->cell, ctx->del, ctx->cap, a);
   ++ctx->nlaunch;
   PMPIC_CUDA(cudaGetLastError());
   return 0;
@@ -1156,6 +1168,7 @@ template <int NG>
 __global__ void k_grid2par_mt(Geom g, int64_t n, const int32_t* __restrict__ cell, const float* __restrict__ FX,
                               const float* __restrict__ FY, const float* __restrict__ FZ, G2PArgs<NG> a,
                               DevInfo* info) {
+  PDL_WAIT();
   const int64_t t = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
   if (t >= n) return;
   const int32_t id = cell[t];
@@ -1193,8 +1206,8 @@ int grid2par_multi_m(pmpic_ctx* ctx, const float* const* grids, int ng, float* c
       a.grid[q] = (const double*)grids[q];
       a.out[q] = (double*)out[q];
     }
-    k_grid2par_mt<NG><<<nblk(ctx->n, 256), 256, 0, ctx->stream>>>(ctx->g, ctx->n, ctx->cell, curoff(ctx, 0),
-                                                                   curoff(ctx, 1), curoff(ctx, 2), a, ctx->dinfo);
+    launch(ctx->stream, nblk(ctx->n, 256), 256, 0, k_grid2par_mt<NG>, ctx->g, ctx->n, ctx->cell, curoff(ctx, 0),
+           curoff(ctx, 1), curoff(ctx, 2), a, ctx->dinfo);
     ++ctx->nlaunch;
   };
   switch (ng) {
@@ -1227,7 +1240,7 @@ int cell_ids(pmpic_ctx* ctx, int32_t* dcells) {
   int rc = bin_and_sort(ctx);
   if (rc) return rc;
   if (ctx->n > 0) {
-    k_cell_xfast<<<nblk(ctx->n, 256), 256, 0, ctx->stream>>>(ctx->g, ctx->n, ctx->cell, dcells); ++ctx->nlaunch;
+    launch(ctx->stream, nblk(ctx->n, 256), 256, 0, k_cell_xfast, ctx->g, ctx->n, ctx->cell, dcells); ++ctx->nlaunch;
   }
   PMPIC_CUDA(cudaGetLastError());
   return 0;
@@ -1326,12 +1339,13 @@ extern "C" int pmpic_par2grid_static(int32_t nx, int32_t ny, int32_t nz, double 
   if (cudaMemsetAsync(count, 0, sizeof(int32_t) * (ncell + 1), st) != cudaSuccess) return PMPIC_ERR_CUDA;
   if (cudaMemsetAsync(info, 0, sizeof(DevInfo), st) != cudaSuccess) return PMPIC_ERR_CUDA;
   if (n > 0)
-    k_bin_count<<<nblk(n, 256), 256, 0, st>>>(g, n, x, y, z, cell, del, SP_MAX_PARCELS, count, info);
+    launch(st, nblk(n, 256), 256, 0, k_bin_count, g, n, x, y, z, cell, del, SP_MAX_PARCELS, count, info,
+           (int32_t*)nullptr);
   int64_t nl = 0;
   scan_launch(count, ncell, cstart, fill, -1, info, tiles, st, nl);
   if (n > 0) {
-    k_bin_scatter<<<nblk(n, 256 * SC_ITEMS), 256, 0, st>>>(n, cell, count, cstart, fill, sorted, SP_MAX_PARCELS);
-    k_sort_segments<<<nblk(ncell, SORT_CELLS), SORT_CELLS, 0, st>>>(ncell, cstart, fill, sorted);
+    launch(st, nblk(n, 256 * SC_ITEMS), 256, 0, k_bin_scatter, n, cell, count, cstart, fill, sorted, SP_MAX_PARCELS);
+    launch(st, nblk(ncell, SORT_CELLS), SORT_CELLS, 0, k_sort_segments, ncell, cstart, fill, sorted);
   }
   P2GArgs<1> a{};
   a.f[0] = field;

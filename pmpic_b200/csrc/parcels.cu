@@ -36,6 +36,7 @@ __device__ __forceinline__ void count_mover(int64_t t, bool moves, int32_t* __re
 }
 template <class Pred>
 __global__ void __launch_bounds__(256) k_count(Pred pr, int64_t n, int32_t* __restrict__ blockcnt) {
+  PDL_WAIT();
   __shared__ int ws[8];
   const int64_t base = (int64_t)blockIdx.x * CITEMS + threadIdx.x;
   int c = 0;
@@ -79,6 +80,7 @@ struct SwapCheck {
 template <class Pred>
 __global__ void __launch_bounds__(256) k_write(Pred pr, int64_t n, const int32_t* __restrict__ blockcnt,
                                                int32_t* __restrict__ list, int32_t* __restrict__ dcount, SwapCheck sc) {
+  PDL_WAIT();
   __shared__ int wc[CCH * 8];  // per (chunk, warp): count, then exclusive offset within the CTA
   __shared__ int ws[8];
   if (blockIdx.x == 0) {
@@ -201,6 +203,7 @@ struct Six {
 };
 template <class R>
 __global__ void __launch_bounds__(256) k_pack(Geom g, Six<R> S, R* __restrict__ out, Zero2 z) {
+  PDL_WAIT();
   using R2 = typename Pair<R>::T;
   constexpr int NF = 6, KS = PK_T + 1;
   constexpr int TS = PK_K * KS + 1;  // per-field tile stride
@@ -248,7 +251,7 @@ static void pack6(pmpic_ctx* ctx, const R* const* grids, R* out, const Zero2& z)
   dim3 gr((g.Nx + PK_T - 1) / PK_T, (g.nzp + PK_K - 1) / PK_K, g.Ny);
   Six<R> S;
   for (int f = 0; f < 6; ++f) S.g[f] = grids[f];
-  k_pack<R><<<gr, 256, 0, ctx->stream>>>(g, S, out, z);
+  launch(ctx->stream, gr, 256, 0, k_pack<R>, g, S, out, z);
   ++ctx->nlaunch;
 }
 // the six fields at the two levels of xy corner (ci, cj) of a cell of level ck:
@@ -494,6 +497,7 @@ template <bool GU, bool GP>
 __global__ void __launch_bounds__(256, 4) k_rk4(Geom g, int64_t n, RkPtrs P, int stage, const double* __restrict__ dtp,
                       const int32_t* __restrict__ cell, const double* __restrict__ del, int64_t cap,
                       int8_t* __restrict__ dir, int store_d, int32_t* __restrict__ dircnt) {
+  PDL_WAIT();
   // the staged gather window, when both gathers are pending (the step's path)
   __shared__ __align__(16) double gws[(GU && GP) ? 4 * GWD_KW * 6 : 2];
   __shared__ __align__(8) uint64_t gwbar;
@@ -594,6 +598,7 @@ __global__ void __launch_bounds__(256, 4) k_rk4(Geom g, int64_t n, RkPtrs P, int
 // = 1..8 (:296-437) with the limits x_coords(3), x_coords(Nx+3) (:314-318).
 __global__ void k_reflect_classify(Geom g, int64_t n, const double* __restrict__ X, const double* __restrict__ Y,
                                    double* __restrict__ Z, int8_t* __restrict__ dir) {
+  PDL_WAIT();
   int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
   if (i >= n) return;
   double z = Z[i];
@@ -607,6 +612,7 @@ __global__ void k_reflect_classify(Geom g, int64_t n, const double* __restrict__
 // receives and unpacks the parcels (dir 1..8, ascending index within a dir).
 __global__ void k_partition_dirs(const int32_t* __restrict__ V, const int32_t* __restrict__ nmov,
                                  const int8_t* __restrict__ dir, int32_t* __restrict__ M) {
+  PDL_WAIT();
   __shared__ int base[9];
   __shared__ int cnt[9];
   __shared__ int wcnt[32][9];
@@ -667,6 +673,7 @@ __constant__ int c_swap_props[29] = {PMPIC_PROP_X,    PMPIC_PROP_Y,    PMPIC_PRO
 __global__ void k_swap_gather(Geom g, const int32_t* __restrict__ nmov, const int32_t* __restrict__ M,
                               const int8_t* __restrict__ dir, const double* __restrict__ parcels, int64_t cap,
                               double* __restrict__ buf) {
+  PDL_WAIT();
   const int nm = *nmov;
   for (int64_t e = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; e < (int64_t)nm * 29;
        e += (int64_t)gridDim.x * blockDim.x) {
@@ -688,6 +695,7 @@ __global__ void k_swap_gather(Geom g, const int32_t* __restrict__ nmov, const in
 // unpack into the vacated slots in ascending order (haloswap.F90:695-716)
 __global__ void k_swap_scatter(const int32_t* __restrict__ nmov, const int32_t* __restrict__ V,
                                const double* __restrict__ buf, double* __restrict__ parcels, int64_t cap) {
+  PDL_WAIT();
   const int nm = *nmov;
   for (int64_t e = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; e < (int64_t)nm * 29;
        e += (int64_t)gridDim.x * blockDim.x) {
@@ -698,6 +706,7 @@ __global__ void k_swap_scatter(const int32_t* __restrict__ nmov, const int32_t* 
 // ---- parcel splitting (parcel_splitting.F90:64-133) -----------------------------------
 __global__ void k_split_flag(int64_t n, double* __restrict__ parcels, int64_t cap, const double* __restrict__ dtp,
                              int32_t* __restrict__ flag) {
+  PDL_WAIT();
   int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
   if (i >= n) return;
   const double dt = *dtp;
@@ -720,6 +729,7 @@ __global__ void k_split_flag(int64_t n, double* __restrict__ parcels, int64_t ca
 __global__ void k_split_apply(Geom g, int64_t n, const int32_t* __restrict__ list, const int32_t* __restrict__ nsplit,
                               double* __restrict__ parcels, int64_t cap, DevInfo* info, int8_t* __restrict__ dir,
                               int32_t* __restrict__ dircnt) {
+  PDL_WAIT();
   const int ns = *nsplit;
   const double pi = 4. * atan(1.0);
   const double third = f4div(1.f, 3.f);
@@ -780,6 +790,7 @@ __global__ void k_split_apply(Geom g, int64_t n, const int32_t* __restrict__ lis
 // ---- btot (vorticity_tendency.F90:121-126) ------------------------------------------------
 __global__ void k_btot(int64_t n, const double* __restrict__ B, const double* __restrict__ H,
                        const double* __restrict__ Z, double* __restrict__ BT) {
+  PDL_WAIT();
   int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
   if (i >= n) return;
   BT[i] = B[i] + 12.5 * fmax(0.0, H[i] - exp(-Z[i]));
@@ -802,6 +813,7 @@ __device__ __forceinline__ void mark_near(const Geom& g, int32_t id, uint8_t* __
 // the removed parcels' cells (FP64 path; the mixed form marks them as it uncounts them)
 __global__ void k_mark_removed(Geom g, const int32_t* __restrict__ zlist, const int32_t* __restrict__ nz,
                                const int32_t* __restrict__ cell, uint8_t* __restrict__ near) {
+  PDL_WAIT();
   const int n = *nz;
   for (int t = blockIdx.x * blockDim.x + threadIdx.x; t < n; t += gridDim.x * blockDim.x) {
     const int32_t c = cell[zlist[t]];
@@ -809,6 +821,7 @@ __global__ void k_mark_removed(Geom g, const int32_t* __restrict__ zlist, const 
   }
 }
 __global__ void k_keep(int64_t n, const double* __restrict__ VOL, double vmin, int32_t* __restrict__ keep) {
+  PDL_WAIT();
   int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
   if (i >= n) return;
   keep[i] = VOL[i] < vmin ? 0 : 1;  // :488, :555
@@ -825,6 +838,7 @@ __global__ void k_new_parcels(Geom g, const int32_t* __restrict__ olist, const i
                               const double* __restrict__ KQ, const double* __restrict__ KR,
                               int32_t* __restrict__ newslot, double* __restrict__ portion,
                               uint8_t* __restrict__ near, DevInfo* info) {
+  PDL_WAIT();
   const int na = *nnew, nz0 = *nzero;
   for (int64_t a = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; a < na; a += (int64_t)gridDim.x * blockDim.x) {
     int64_t o = olist[a];
@@ -883,6 +897,7 @@ struct ResPtrs {
 // doubled or not), so it is left at once.
 __global__ void k_residual_update(Geom g, ResPtrs RP, const int32_t* __restrict__ newslot,
                                   const double* __restrict__ portion, const uint8_t* __restrict__ near) {
+  PDL_WAIT();
   int64_t e = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
   if (e >= g.nphys) return;
   int i = (int)(e % g.Nx);
@@ -932,6 +947,7 @@ __global__ void __launch_bounds__(256, 3) k_redistribute(Geom g, int64_t norig, 
                                                          const int32_t* __restrict__ cell,
                                                          const double* __restrict__ del,
                                                          const uint8_t* __restrict__ near, RedistGridsD RD) {
+  PDL_WAIT();
   int64_t m = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
   if (m >= norig) return;
   auto A = [&](int pid) -> double* { return parcels + (size_t)pid * cap; };
@@ -984,6 +1000,7 @@ __global__ void __launch_bounds__(256, 3) k_redistribute(Geom g, int64_t norig, 
 __global__ void k_backfill(const int32_t* __restrict__ zlist, const int32_t* __restrict__ nz,
                            const int32_t* __restrict__ olist, const int32_t* __restrict__ no,
                            double* __restrict__ parcels, int64_t cap, DevInfo* info) {
+  PDL_WAIT();
   const int nzero = *nz, nones = *no;
   if (blockIdx.x == 0 && threadIdx.x == 0 && nzero > nones) atomicCAS(&info->error, 0, PMPIC_ERR_BACKFILL);
   const int pids[11] = {PMPIC_PROP_X, PMPIC_PROP_Y, PMPIC_PROP_Z, PMPIC_PROP_P,   PMPIC_PROP_Q,      PMPIC_PROP_R,
@@ -1076,6 +1093,7 @@ template <bool GU, bool GP>
 __global__ void __launch_bounds__(256, 6) k_rk4_m(Geom g, int64_t n, MPtrs P, int stage, const double* __restrict__ dtp,
                         int8_t* __restrict__ dir, int32_t* __restrict__ count, DevInfo* info,
                         float* __restrict__ stretch, int store_d, int32_t* __restrict__ dircnt) {
+  PDL_WAIT();
   // the staged gather window, when both gathers are pending (the step's path)
   __shared__ __align__(16) float gws[(GU && GP) ? 4 * GW_KW * 6 : 4];
   __shared__ __align__(8) uint64_t gwbar;
@@ -1203,6 +1221,7 @@ constexpr int SWAP_M = 30;  // 29 properties + the cell id per staged parcel
 __global__ void k_swap_gather_m(Geom g, const int32_t* __restrict__ nmov, const int32_t* __restrict__ M,
                                 const int8_t* __restrict__ dir, const double* __restrict__ parcels, int64_t cap,
                                 const int32_t* __restrict__ cell, double* __restrict__ buf) {
+  PDL_WAIT();
   const int nm = *nmov;
   for (int64_t e = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; e < (int64_t)nm * SWAP_M;
        e += (int64_t)gridDim.x * blockDim.x) {
@@ -1239,6 +1258,7 @@ __global__ void k_swap_gather_m(Geom g, const int32_t* __restrict__ nmov, const 
 __global__ void k_swap_scatter_m(const int32_t* __restrict__ nmov, const int32_t* __restrict__ V,
                                  const double* __restrict__ buf, double* __restrict__ parcels, int64_t cap,
                                  int32_t* __restrict__ cell) {
+  PDL_WAIT();
   const int nm = *nmov;
   for (int64_t e = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; e < (int64_t)nm * SWAP_M;
        e += (int64_t)gridDim.x * blockDim.x) {
@@ -1257,6 +1277,7 @@ __global__ void k_swap_scatter_m(const int32_t* __restrict__ nmov, const int32_t
 // splitting (parcel_splitting.F90:64-133) in FP32
 __global__ void k_split_flag_m(int64_t n, double* __restrict__ parcels, int64_t cap, const double* __restrict__ dtp,
                                int32_t* __restrict__ flag) {
+  PDL_WAIT();
   const int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
   if (i >= n) return;
   const float dt = (float)*dtp;
@@ -1277,6 +1298,7 @@ __global__ void k_split_flag_m(int64_t n, double* __restrict__ parcels, int64_t 
 __global__ void k_split_apply_m(Geom g, int64_t n, const int32_t* __restrict__ list, const int32_t* __restrict__ nsplit,
                                 double* __restrict__ parcels, int64_t cap, DevInfo* info, int8_t* __restrict__ dir,
                                 int32_t* __restrict__ dircnt, int32_t* __restrict__ cell, int32_t* __restrict__ count) {
+  PDL_WAIT();
   const int ns = *nsplit;
   const float pi = 3.14159265358979f;
   const float inv[3] = {(float)(1.0 / g.dx), (float)(1.0 / g.dy), (float)(1.0 / g.dz)};
@@ -1340,6 +1362,7 @@ __global__ void k_split_apply_m(Geom g, int64_t n, const int32_t* __restrict__ l
 // btot (vorticity_tendency.F90:121-126) in FP32, z from the current cell layer and offset
 __global__ void k_btot_m(Geom g, int64_t n, const float* __restrict__ B, const float* __restrict__ H,
                          const int32_t* __restrict__ cell, const float* __restrict__ FZ, float* __restrict__ BT) {
+  PDL_WAIT();
   const int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
   if (i >= n) return;
   int ci, cj, ck;
@@ -1350,6 +1373,7 @@ __global__ void k_btot_m(Geom g, int64_t n, const float* __restrict__ B, const f
 
 // mixing (parcel_mixing.F90:68-431) in FP32
 __global__ void k_keep_m(int64_t n, const float* __restrict__ VOL, float vmin, int32_t* __restrict__ keep) {
+  PDL_WAIT();
   const int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
   if (i >= n) return;
   keep[i] = VOL[i] < vmin ? 0 : 1;
@@ -1362,6 +1386,7 @@ __global__ void k_new_parcels_m(Geom g, const int32_t* __restrict__ olist, const
                                 const float* __restrict__ KQ, const float* __restrict__ KR,
                                 int32_t* __restrict__ newslot, float* __restrict__ portion, float vmin,
                                 int32_t* __restrict__ cell, uint8_t* __restrict__ near, DevInfo* info) {
+  PDL_WAIT();
   const int na = *nnew, nz0 = *nzero;
   for (int64_t a = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; a < na; a += (int64_t)gridDim.x * blockDim.x) {
     const int64_t o = olist[a];
@@ -1414,6 +1439,7 @@ struct ResPtrsF {
 // residuals are zero and stay zero (doubled at a wall or not).
 __global__ void k_residual_update_m(Geom g, ResPtrsF RP, const int32_t* __restrict__ newslot,
                                     const float* __restrict__ portion, const uint8_t* __restrict__ near) {
+  PDL_WAIT();
   const int64_t e = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
   if (e >= g.nphys) return;
   const int i = (int)(e % g.Nx);
@@ -1457,6 +1483,7 @@ __global__ void __launch_bounds__(256, 6) k_redistribute_m(Geom g, int64_t norig
                                                           double* __restrict__ parcels, int64_t cap,
                                                           const int32_t* __restrict__ cell,
                                                           const uint8_t* __restrict__ near, RedistGrids RD) {
+  PDL_WAIT();
   const int64_t m = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
   if (m >= norig) return;
   auto F = [&](int pid) { return (float*)(parcels + (size_t)pid * cap); };
@@ -1505,6 +1532,7 @@ __global__ void __launch_bounds__(256, 6) k_redistribute_m(Geom g, int64_t norig
 __global__ void k_mix_uncount(Geom g, const int32_t* __restrict__ zlist, const int32_t* __restrict__ nz,
                               const int32_t* __restrict__ cell, int32_t* __restrict__ count,
                               uint8_t* __restrict__ near) {
+  PDL_WAIT();
   const int n = *nz;
   for (int t = blockIdx.x * blockDim.x + threadIdx.x; t < n; t += gridDim.x * blockDim.x) {
     const int32_t c = cell[zlist[t]];
@@ -1518,6 +1546,7 @@ __global__ void k_mix_uncount(Geom g, const int32_t* __restrict__ zlist, const i
 // then only the appended slots did)
 __global__ void k_mix_recount(Geom g, int64_t s0, int64_t norig, int64_t nfinal, const int32_t* __restrict__ keep,
                               const int32_t* __restrict__ cell, int32_t* __restrict__ count, DevInfo* info) {
+  PDL_WAIT();
   const int64_t hi = norig > nfinal ? norig : nfinal;
   for (int64_t s = s0 + (int64_t)blockIdx.x * blockDim.x + threadIdx.x; s < hi; s += (int64_t)gridDim.x * blockDim.x) {
     if (s < nfinal) {
@@ -1536,6 +1565,7 @@ __global__ void k_mix_recount(Geom g, int64_t s0, int64_t norig, int64_t nfinal,
 __global__ void k_backfill_m(const int32_t* __restrict__ zlist, const int32_t* __restrict__ nz,
                              const int32_t* __restrict__ olist, const int32_t* __restrict__ no,
                              double* __restrict__ parcels, int64_t cap, int32_t* __restrict__ cell, DevInfo* info) {
+  PDL_WAIT();
   const int nzero = *nz, nones = *no;
   if (blockIdx.x == 0 && threadIdx.x == 0 && nzero > nones) atomicCAS(&info->error, 0, PMPIC_ERR_BACKFILL);
   const int pids[11] = {PMPIC_PROP_X, PMPIC_PROP_Y, PMPIC_PROP_Z, PMPIC_PROP_P,   PMPIC_PROP_Q,      PMPIC_PROP_R,
@@ -1559,6 +1589,7 @@ __global__ void k_grid2par_m(Geom g, int64_t n, const int32_t* __restrict__ cell
                              const float* __restrict__ FY, const float* __restrict__ FZ, const float* __restrict__ G0,
                              const float* __restrict__ G1, const float* __restrict__ G2, float* __restrict__ O0,
                              float* __restrict__ O1, float* __restrict__ O2) {
+  PDL_WAIT();
   const int64_t t = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
   if (t >= n) return;
   const int32_t id = cell[t];
@@ -1574,6 +1605,7 @@ __global__ void k_grid2par_m(Geom g, int64_t n, const int32_t* __restrict__ cell
 // ---- test components (FP64 path) ---------------------------------------------------
 // euler_integrator.F90:68-76: one explicit step of x, y, z, p, q, r
 __global__ void k_euler(int64_t n, double* __restrict__ parcels, int64_t cap, const double* __restrict__ dtp) {
+  PDL_WAIT();
   const int64_t t = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
   if (t >= n) return;
   const double dt = *dtp;
@@ -1591,7 +1623,8 @@ __global__ void k_euler(int64_t n, double* __restrict__ parcels, int64_t cap, co
 struct VelGeom {
   double x0, y0, r0, xc1, yc1, xc2, yc2;
 };
-__global__ void k_prescribed_tag(int64_t n, double* __restrict__ parcels, int64_t cap, VelGeom vg) {  // :72-84
+__global__ void k_prescribed_tag(int64_t n, double* __restrict__ parcels, int64_t cap, VelGeom vg) {
+  PDL_WAIT();  // :72-84
   const int64_t t = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
   if (t >= n) return;
   double tag = 0;
@@ -1601,6 +1634,7 @@ __global__ void k_prescribed_tag(int64_t n, double* __restrict__ parcels, int64_
 }
 __global__ void k_prescribed_velocity(int64_t n, double* __restrict__ parcels, int64_t cap, int profile,
                                       VelGeom vg) {
+  PDL_WAIT();
   const int64_t t = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
   if (t >= n) return;
   const double x = parcels[(size_t)PMPIC_PROP_X * cap + t], y = parcels[(size_t)PMPIC_PROP_Y * cap + t];
@@ -1644,9 +1678,9 @@ static int compact(pmpic_ctx* ctx, Pred pr, int64_t n, int32_t* list, int32_t* d
   }
   int32_t* cnt = ctx->aux2;  // nb <= nbmax
   if (!counted) {
-    k_count<<<(unsigned)nb, 256, 0, ctx->stream>>>(pr, n, cnt); ++ctx->nlaunch;
+    launch(ctx->stream, (unsigned)nb, 256, 0, k_count<Pred>, pr, n, cnt); ++ctx->nlaunch;
   }
-  k_write<<<(unsigned)nb, 256, 0, ctx->stream>>>(pr, n, cnt, list, dcount, sc); ++ctx->nlaunch;
+  launch(ctx->stream, (unsigned)nb, 256, 0, k_write<Pred>, pr, n, cnt, list, dcount, sc); ++ctx->nlaunch;
   PMPIC_CUDA(cudaGetLastError());
   return 0;
 }
@@ -1663,15 +1697,15 @@ int flush_gathers(pmpic_ctx* ctx) {
     float* const* G = (float* const*)ctx->grid;
     const int64_t n = ctx->n;
     if (ctx->pending_uvw && n > 0) {
-      k_grid2par_m<<<nblk(n, 256), 256, 0, ctx->stream>>>(
-          ctx->g, n, ctx->cell, curoff(ctx, 0), curoff(ctx, 1), curoff(ctx, 2), G[PMPIC_GRID_U], G[PMPIC_GRID_V],
-          G[PMPIC_GRID_W], propf(ctx, PMPIC_PROP_DXDT), propf(ctx, PMPIC_PROP_DYDT), propf(ctx, PMPIC_PROP_DZDT));
+      launch(ctx->stream, nblk(n, 256), 256, 0, k_grid2par_m,  ctx->g, n, ctx->cell, curoff(ctx, 0), curoff(ctx, 1),
+             curoff(ctx, 2), G[PMPIC_GRID_U], G[PMPIC_GRID_V], G[PMPIC_GRID_W], propf(ctx, PMPIC_PROP_DXDT),
+             propf(ctx, PMPIC_PROP_DYDT), propf(ctx, PMPIC_PROP_DZDT));
       ++ctx->nlaunch;
     }
     if (ctx->pending_pqr && n > 0) {
-      k_grid2par_m<<<nblk(n, 256), 256, 0, ctx->stream>>>(
-          ctx->g, n, ctx->cell, curoff(ctx, 0), curoff(ctx, 1), curoff(ctx, 2), G[PMPIC_GRID_DP], G[PMPIC_GRID_DQ],
-          G[PMPIC_GRID_DR], propf(ctx, PMPIC_PROP_DPDT), propf(ctx, PMPIC_PROP_DQDT), propf(ctx, PMPIC_PROP_DRDT));
+      launch(ctx->stream, nblk(n, 256), 256, 0, k_grid2par_m,  ctx->g, n, ctx->cell, curoff(ctx, 0), curoff(ctx, 1),
+             curoff(ctx, 2), G[PMPIC_GRID_DP], G[PMPIC_GRID_DQ], G[PMPIC_GRID_DR], propf(ctx, PMPIC_PROP_DPDT),
+             propf(ctx, PMPIC_PROP_DQDT), propf(ctx, PMPIC_PROP_DRDT));
       ++ctx->nlaunch;
     }
     ctx->pending_uvw = ctx->pending_pqr = false;
@@ -1696,14 +1730,13 @@ int flush_gathers(pmpic_ctx* ctx) {
 int compute_btot(pmpic_ctx* ctx) {
   if (ctx->n == 0) return 0;
   if (ctx->mixed) {
-    k_btot_m<<<nblk(ctx->n, 256), 256, 0, ctx->stream>>>(ctx->g, ctx->n, propf(ctx, PMPIC_PROP_B),
-                                                         propf(ctx, PMPIC_PROP_H), ctx->cell, curoff(ctx, 2),
-                                                         propf(ctx, PMPIC_PROP_BTOT)); ++ctx->nlaunch;
+    launch(ctx->stream, nblk(ctx->n, 256), 256, 0, k_btot_m, ctx->g, ctx->n, propf(ctx, PMPIC_PROP_B), propf(ctx,
+           PMPIC_PROP_H), ctx->cell, curoff(ctx, 2), propf(ctx, PMPIC_PROP_BTOT)); ++ctx->nlaunch;
     PMPIC_CUDA(cudaGetLastError());
     return 0;
   }
-  k_btot<<<nblk(ctx->n, 256), 256, 0, ctx->stream>>>(ctx->n, prop(ctx, PMPIC_PROP_B), prop(ctx, PMPIC_PROP_H),
-                                                     prop(ctx, PMPIC_PROP_Z), prop(ctx, PMPIC_PROP_BTOT)); ++ctx->nlaunch;
+  launch(ctx->stream, nblk(ctx->n, 256), 256, 0, k_btot, ctx->n, prop(ctx, PMPIC_PROP_B), prop(ctx, PMPIC_PROP_H),
+         prop(ctx, PMPIC_PROP_Z), prop(ctx, PMPIC_PROP_BTOT)); ++ctx->nlaunch;
   PMPIC_CUDA(cudaGetLastError());
   return 0;
 }
@@ -1759,10 +1792,9 @@ int rk4_stage(pmpic_ctx* ctx, int stage) {
     // within pmpic_step the last stage also advances the stretch of the split
     // that follows (the haloswap in between moves it with its parcel)
     const bool adv = ctx->split_follows && stage == 4;
-    kern<<<nblk(ctx->n, 256), 256, 0, ctx->stream>>>(ctx->g, ctx->n, P, stage, &ctx->dinfo->dtm, ctx->dir,
-                                                     ctx->cell_count, ctx->dinfo,
-                                                     adv ? propf(ctx, PMPIC_PROP_STRETCH) : nullptr,
-                                                     store_tendencies(ctx, stage), ctx->aux2); ++ctx->nlaunch;
+    launch(ctx->stream, nblk(ctx->n, 256), 256, 0, kern, ctx->g, ctx->n, P, stage, &ctx->dinfo->dtm, ctx->dir,
+           ctx->cell_count, ctx->dinfo, adv ? propf(ctx, PMPIC_PROP_STRETCH) : nullptr, store_tendencies(ctx, stage),
+           ctx->aux2); ++ctx->nlaunch;
     ctx->stretch_advanced = adv;
     ctx->pending_uvw = ctx->pending_pqr = false;
     ctx->dir_ready = true;
@@ -1790,15 +1822,18 @@ int rk4_stage(pmpic_ctx* ctx, int stage) {
   if ((gu || gp) && !ctx->sorted_valid) return set_error(ctx, PMPIC_ERR_STATE, "deferred gather without binning");
   P.g6 = ctx->gpack;
   P.whint = ctx->whint;
-  const Zero2 z{{ctx->aux2, nullptr}, {ctx->nbmax, 0}};  // the mover counts
-  if (gu && gp) pack6<double>(ctx, P.grid, ctx->gpack, z);
-  else PMPIC_CUDA(cudaMemsetAsync(z.p[0], 0, sizeof(int32_t) * z.n[0], ctx->stream));
+  // the mover counts and the next binning's cell counts start at zero
+  const Zero2 z{{ctx->aux2, ctx->cell_count}, {ctx->nbmax, ctx->g.ncell + 1}};
+  if (gu && gp) {
+    pack6<double>(ctx, P.grid, ctx->gpack, z);
+    ctx->count_zero = true;
+  } else PMPIC_CUDA(cudaMemsetAsync(z.p[0], 0, sizeof(int32_t) * z.n[0], ctx->stream));
   auto kern = gu ? (gp ? k_rk4<true, true> : k_rk4<true, false>) : (gp ? k_rk4<false, true> : k_rk4<false, false>);
   // the next binning stays a separate pass on this path: its six IEEE
   // divisions per parcel cost the HBM-bound stage kernel more than the
   // position reads they would save
-  kern<<<nblk(ctx->n, 256), 256, 0, ctx->stream>>>(ctx->g, ctx->n, P, stage, &ctx->dinfo->dtm, ctx->cell, ctx->del,
-                                                   ctx->cap, ctx->dir, store_tendencies(ctx, stage), ctx->aux2); ++ctx->nlaunch;
+  launch(ctx->stream, nblk(ctx->n, 256), 256, 0, kern, ctx->g, ctx->n, P, stage, &ctx->dinfo->dtm, ctx->cell,
+         ctx->del, ctx->cap, ctx->dir, store_tendencies(ctx, stage), ctx->aux2); ++ctx->nlaunch;
   ctx->pending_uvw = ctx->pending_pqr = false;
   ctx->dir_ready = true;  // z reflected and directions classified
   ctx->sorted_valid = false;
@@ -1829,9 +1864,8 @@ int parcel_haloswap(pmpic_ctx* ctx) {
     // kernel that moves them: none is outside the domain
     PMPIC_CUDA(cudaMemsetAsync(ctx->dir, 0, (size_t)n, ctx->stream));
   } else if (!ready) {
-    k_reflect_classify<<<nblk(n, 256), 256, 0, ctx->stream>>>(ctx->g, n, prop(ctx, PMPIC_PROP_X),
-                                                              prop(ctx, PMPIC_PROP_Y), prop(ctx, PMPIC_PROP_Z),
-                                                              ctx->dir); ++ctx->nlaunch;
+    launch(ctx->stream, nblk(n, 256), 256, 0, k_reflect_classify, ctx->g, n, prop(ctx, PMPIC_PROP_X), prop(ctx,
+           PMPIC_PROP_Y), prop(ctx, PMPIC_PROP_Z), ctx->dir); ++ctx->nlaunch;
   }
   int32_t* V = ctx->aux;                 // vacated slots, ascending
   int32_t* M = ctx->keep;                // moved parcels in send order (keep is free outside mixing)
@@ -1842,15 +1876,16 @@ int parcel_haloswap(pmpic_ctx* ctx) {
   int32_t* nmc = dcounter(ctx, 1);
   int rc = compact(ctx, PredDirNZ{ctx->dir}, n, V, nm, ready, SwapCheck{nmc, ctx->swapcap, ctx->dinfo});
   if (rc) return rc;
-  k_partition_dirs<<<1, 1024, 0, ctx->stream>>>(V, nm, ctx->dir, M); ++ctx->nlaunch;
+  launch(ctx->stream, 1, 1024, 0, k_partition_dirs, V, nm, ctx->dir, M); ++ctx->nlaunch;
   if (ctx->mixed) {
-    k_swap_gather_m<<<592, 256, 0, ctx->stream>>>(ctx->g, nmc, M, ctx->dir, ctx->parcels, ctx->cap, ctx->cell,
-                                                   ctx->swapbuf); ++ctx->nlaunch;
-    k_swap_scatter_m<<<592, 256, 0, ctx->stream>>>(nmc, V, ctx->swapbuf, ctx->parcels, ctx->cap, ctx->cell);
+    launch(ctx->stream, 592, 256, 0, k_swap_gather_m, ctx->g, nmc, M, ctx->dir, ctx->parcels, ctx->cap, ctx->cell,
+           ctx->swapbuf); ++ctx->nlaunch;
+    launch(ctx->stream, 592, 256, 0, k_swap_scatter_m, nmc, V, ctx->swapbuf, ctx->parcels, ctx->cap, ctx->cell);
     ++ctx->nlaunch;
   } else {
-    k_swap_gather<<<592, 256, 0, ctx->stream>>>(ctx->g, nmc, M, ctx->dir, ctx->parcels, ctx->cap, ctx->swapbuf); ++ctx->nlaunch;
-    k_swap_scatter<<<592, 256, 0, ctx->stream>>>(nmc, V, ctx->swapbuf, ctx->parcels, ctx->cap); ++ctx->nlaunch;
+    launch(ctx->stream, 592, 256, 0, k_swap_gather, ctx->g, nmc, M, ctx->dir, ctx->parcels, ctx->cap,
+           ctx->swapbuf); ++ctx->nlaunch;
+    launch(ctx->stream, 592, 256, 0, k_swap_scatter, nmc, V, ctx->swapbuf, ctx->parcels, ctx->cap); ++ctx->nlaunch;
   }
   PMPIC_CUDA(cudaGetLastError());
   ctx->in_domain = true;  // (a staging overflow is reported as an error and ends the run)
@@ -1872,9 +1907,9 @@ int splitting(pmpic_ctx* ctx) {
       rc = compact(ctx, PredStretchM{propf(ctx, PMPIC_PROP_STRETCH)}, n, list, ns);
     } else {
       if (ctx->mixed)
-        k_split_flag_m<<<nblk(n, 256), 256, 0, ctx->stream>>>(n, ctx->parcels, ctx->cap, &ctx->dinfo->dtm, flag);
+        launch(ctx->stream, nblk(n, 256), 256, 0, k_split_flag_m, n, ctx->parcels, ctx->cap, &ctx->dinfo->dtm, flag);
       else
-        k_split_flag<<<nblk(n, 256), 256, 0, ctx->stream>>>(n, ctx->parcels, ctx->cap, &ctx->dinfo->dtm, flag);
+        launch(ctx->stream, nblk(n, 256), 256, 0, k_split_flag, n, ctx->parcels, ctx->cap, &ctx->dinfo->dtm, flag);
       ++ctx->nlaunch;
       rc = compact(ctx, PredFlag{flag}, n, list, ns);
     }
@@ -1911,11 +1946,11 @@ int splitting(pmpic_ctx* ctx) {
       dsplit = ctx->dir;
     }
     if (ctx->mixed)
-      k_split_apply_m<<<592, 256, 0, ctx->stream>>>(ctx->g, n, list, ns, ctx->parcels, ctx->cap, ctx->dinfo, dsplit,
-                                                    ctx->aux2, ctx->cell, keep_counts ? ctx->cell_count : nullptr);
+      launch(ctx->stream, 592, 256, 0, k_split_apply_m, ctx->g, n, list, ns, ctx->parcels, ctx->cap, ctx->dinfo,
+             dsplit, ctx->aux2, ctx->cell, keep_counts ? ctx->cell_count : nullptr);
     else
-      k_split_apply<<<592, 256, 0, ctx->stream>>>(ctx->g, n, list, ns, ctx->parcels, ctx->cap, ctx->dinfo, dsplit,
-                                                  ctx->aux2);
+      launch(ctx->stream, 592, 256, 0, k_split_apply, ctx->g, n, list, ns, ctx->parcels, ctx->cap, ctx->dinfo, dsplit,
+             ctx->aux2);
     ++ctx->nlaunch;
     ctx->dir_ready = dsplit != nullptr;
   }
@@ -1946,7 +1981,8 @@ int euler_step(pmpic_ctx* ctx) {
   int rc = flush_gathers(ctx);
   if (rc) return rc;
   if (ctx->n > 0) {
-    k_euler<<<nblk(ctx->n, 256), 256, 0, ctx->stream>>>(ctx->n, ctx->parcels, ctx->cap, &ctx->dinfo->dtm); ++ctx->nlaunch;
+    launch(ctx->stream, nblk(ctx->n, 256), 256, 0, k_euler, ctx->n, ctx->parcels, ctx->cap,
+           &ctx->dinfo->dtm); ++ctx->nlaunch;
   }
   ctx->sorted_valid = false;
   ctx->count_ready = false;
@@ -1967,10 +2003,10 @@ int prescribed_velocity(pmpic_ctx* ctx, int profile, bool tags) {
   if (rc) return rc;
   if (ctx->n > 0) {
     if (tags)
-      k_prescribed_tag<<<nblk(ctx->n, 256), 256, 0, ctx->stream>>>(ctx->n, ctx->parcels, ctx->cap, vel_geom(ctx));
+      launch(ctx->stream, nblk(ctx->n, 256), 256, 0, k_prescribed_tag, ctx->n, ctx->parcels, ctx->cap, vel_geom(ctx));
     else
-      k_prescribed_velocity<<<nblk(ctx->n, 256), 256, 0, ctx->stream>>>(ctx->n, ctx->parcels, ctx->cap, profile,
-                                                                        vel_geom(ctx));
+      launch(ctx->stream, nblk(ctx->n, 256), 256, 0, k_prescribed_velocity, ctx->n, ctx->parcels, ctx->cap, profile,
+             vel_geom(ctx));
     ++ctx->nlaunch;
   }
   PMPIC_CUDA(cudaGetLastError());
@@ -1996,16 +2032,18 @@ int mixing(pmpic_ctx* ctx) {
   if (rc) return rc;
   if (ctx->mixed) {  // the binning counts stay current through mixing
     PMPIC_CUDA(cudaMemsetAsync(ctx->near, 0, (size_t)g.ncell, ctx->stream));
-    k_mix_uncount<<<148, 256, 0, ctx->stream>>>(g, zlist, nz0, ctx->cell, ctx->cell_count, ctx->near); ++ctx->nlaunch;
+    launch(ctx->stream, 148, 256, 0, k_mix_uncount, g, zlist, nz0, ctx->cell, ctx->cell_count,
+           ctx->near); ++ctx->nlaunch;
   }
   int32_t hz0 = 0;
   PMPIC_CUDA(cudaMemcpyAsync(&hz0, nz0, sizeof(int32_t), cudaMemcpyDeviceToHost, ctx->stream));
   PMPIC_CUDA(cudaStreamSynchronize(ctx->stream));
   if (hz0 > 0 && norig > 0) {
     if (ctx->mixed)
-      k_keep_m<<<nblk(norig, 256), 256, 0, ctx->stream>>>(norig, propf(ctx, PMPIC_PROP_VOL), (float)g.vmin, ctx->keep);
+      launch(ctx->stream, nblk(norig, 256), 256, 0, k_keep_m, norig, propf(ctx, PMPIC_PROP_VOL), (float)g.vmin,
+             ctx->keep);
     else
-      k_keep<<<nblk(norig, 256), 256, 0, ctx->stream>>>(norig, prop(ctx, PMPIC_PROP_VOL), g.vmin, ctx->keep);
+      launch(ctx->stream, nblk(norig, 256), 256, 0, k_keep, norig, prop(ctx, PMPIC_PROP_VOL), g.vmin, ctx->keep);
     ++ctx->nlaunch;
   }
   if ((rc = launch_mix_grids(ctx, hz0 > 0))) return rc;
@@ -2049,18 +2087,17 @@ int mixing(pmpic_ctx* ctx) {
     float* por = (float*)ctx->newportion;
     // without removed parcels only the kept volume grid was made in full
     if (hz0 == 0 && (rc = launch_kept_corners(ctx, olist, nnew, hnew))) return rc;
-    k_new_parcels_m<<<592, 256, 0, ctx->stream>>>(g, olist, nnew, zlist, nz0, norig, ctx->cap, ctx->keep, ctx->parcels,
-                                                  KF[0], KF[1], KF[2], KF[3], KF[4], KF[5], ctx->newslot, por,
-                                                  (float)g.vmin, ctx->cell, ctx->near, ctx->dinfo); ++ctx->nlaunch;
-    k_residual_update_m<<<nblk(g.nphys, 256), 256, 0, ctx->stream>>>(g, RF, ctx->newslot, por, ctx->near);
+    launch(ctx->stream, 592, 256, 0, k_new_parcels_m, g, olist, nnew, zlist, nz0, norig, ctx->cap, ctx->keep,
+           ctx->parcels, KF[0], KF[1], KF[2], KF[3], KF[4], KF[5], ctx->newslot, por, (float)g.vmin, ctx->cell,
+           ctx->near, ctx->dinfo); ++ctx->nlaunch;
+    launch(ctx->stream, nblk(g.nphys, 256), 256, 0, k_residual_update_m, g, RF, ctx->newslot, por, ctx->near);
     ++ctx->nlaunch;
     if (norig > 0) {
       RedistGrids RD;
       RD.kv = KF[0];
       for (int q = 0; q < 6; ++q) RD.r[q] = RF.r[q];
-      k_redistribute_m<<<nblk(norig, 256), 256, 0, ctx->stream>>>(g, norig, hz0 > 0 ? ctx->keep : nullptr,
-                                                                  ctx->parcels, ctx->cap,
-                                                                  ctx->cell, ctx->near, RD);
+      launch(ctx->stream, nblk(norig, 256), 256, 0, k_redistribute_m, g, norig, hz0 > 0 ? ctx->keep : nullptr,
+             ctx->parcels, ctx->cap, ctx->cell, ctx->near, RD);
       ++ctx->nlaunch;
     }
   } else {
@@ -2068,26 +2105,25 @@ int mixing(pmpic_ctx* ctx) {
     if (hz0 == 0 && (rc = launch_kept_corners(ctx, olist, nnew, hnew))) return rc;
     PMPIC_CUDA(cudaMemsetAsync(ctx->near, 0, (size_t)g.ncell, ctx->stream));
     if (hz0 > 0) {
-      k_mark_removed<<<148, 256, 0, ctx->stream>>>(g, zlist, nz0, ctx->cell, ctx->near);
+      launch(ctx->stream, 148, 256, 0, k_mark_removed, g, zlist, nz0, ctx->cell, ctx->near);
       ++ctx->nlaunch;
     }
-    k_new_parcels<<<592, 256, 0, ctx->stream>>>(g, olist, nnew, zlist, nz0, norig, ctx->cap, ctx->keep, ctx->parcels,
-                                                K[0], K[1], K[2], K[3], K[4], K[5], ctx->newslot, ctx->newportion,
-                                                ctx->near, ctx->dinfo); ++ctx->nlaunch;
+    launch(ctx->stream, 592, 256, 0, k_new_parcels, g, olist, nnew, zlist, nz0, norig, ctx->cap, ctx->keep,
+           ctx->parcels, K[0], K[1], K[2], K[3], K[4], K[5], ctx->newslot, ctx->newportion, ctx->near,
+           ctx->dinfo); ++ctx->nlaunch;
     ResPtrs RP;
     for (int q = 0; q < 6; ++q) {
       RP.r[q] = ctx->mixres[q];
       RP.k[q] = K[q];
     }
-    k_residual_update<<<nblk(g.nphys, 256), 256, 0, ctx->stream>>>(g, RP, ctx->newslot, ctx->newportion, ctx->near);
+    launch(ctx->stream, nblk(g.nphys, 256), 256, 0, k_residual_update, g, RP, ctx->newslot, ctx->newportion, ctx->near);
     ++ctx->nlaunch;
     if (norig > 0) {
       RedistGridsD RD;
       RD.kv = K[0];
       for (int q = 0; q < 6; ++q) RD.r[q] = RP.r[q];
-      k_redistribute<<<nblk(norig, 256), 256, 0, ctx->stream>>>(g, norig, hz0 > 0 ? ctx->keep : nullptr,
-                                                                ctx->parcels, ctx->cap,
-                                                                ctx->cell, ctx->del, ctx->near, RD); ++ctx->nlaunch;
+      launch(ctx->stream, nblk(norig, 256), 256, 0, k_redistribute, g, norig, hz0 > 0 ? ctx->keep : nullptr,
+             ctx->parcels, ctx->cap, ctx->cell, ctx->del, ctx->near, RD); ++ctx->nlaunch;
     }
   }
   const int64_t nremove = hz0, nadd = hnew;
@@ -2109,9 +2145,9 @@ int mixing(pmpic_ctx* ctx) {
     if ((rc = compact(ctx, PredKeepEq{ctx->keep, 0}, norig, z2, nz2))) return rc;
     if ((rc = compact(ctx, PredKeepEq{ctx->keep, 1}, norig, ones, no))) return rc;
     if (ctx->mixed)
-      k_backfill_m<<<592, 256, 0, ctx->stream>>>(z2, nz2, ones, no, ctx->parcels, ctx->cap, ctx->cell, ctx->dinfo);
+      launch(ctx->stream, 592, 256, 0, k_backfill_m, z2, nz2, ones, no, ctx->parcels, ctx->cap, ctx->cell, ctx->dinfo);
     else
-      k_backfill<<<592, 256, 0, ctx->stream>>>(z2, nz2, ones, no, ctx->parcels, ctx->cap, ctx->dinfo);
+      launch(ctx->stream, 592, 256, 0, k_backfill, z2, nz2, ones, no, ctx->parcels, ctx->cap, ctx->dinfo);
     ++ctx->nlaunch;
     int32_t hz = 0;
     PMPIC_CUDA(cudaMemcpyAsync(&hz, nz2, sizeof(int32_t), cudaMemcpyDeviceToHost, ctx->stream));
@@ -2123,8 +2159,8 @@ int mixing(pmpic_ctx* ctx) {
     const int64_t s0 = nremove > 0 ? 0 : norig;
     const int64_t hi = std::max<int64_t>(norig, count);
     if (hi > s0) {
-      k_mix_recount<<<nblk(hi - s0, 256), 256, 0, ctx->stream>>>(g, s0, norig, count, ctx->keep, ctx->cell,
-                                                                 ctx->cell_count, ctx->dinfo);
+      launch(ctx->stream, nblk(hi - s0, 256), 256, 0, k_mix_recount, g, s0, norig, count, ctx->keep, ctx->cell,
+             ctx->cell_count, ctx->dinfo);
       ++ctx->nlaunch;
     }
   }

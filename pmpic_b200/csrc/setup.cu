@@ -106,6 +106,7 @@ __device__ __forceinline__ bool plume_accept(const PlumeLattice& L, int64_t col,
 
 // one warp per column: the number of accepted points
 __global__ void k_plume_count(PlumeLattice L, int32_t* __restrict__ count) {
+  PDL_WAIT();
   const int64_t col = ((int64_t)blockIdx.x * blockDim.x + threadIdx.x) >> 5;
   const int lane = threadIdx.x & 31;
   if (col >= L.npl + L.nbg) return;
@@ -123,6 +124,7 @@ __global__ void k_plume_count(PlumeLattice L, int32_t* __restrict__ count) {
 // one warp per column: the accepted points into slots off[col] + rank, in k
 // order, with the properties of :220-226 and :270-286
 __global__ void k_plume_write(PlumeLattice L, const int64_t* __restrict__ off, ParcelSink out) {
+  PDL_WAIT();
   const int64_t col = ((int64_t)blockIdx.x * blockDim.x + threadIdx.x) >> 5;
   const int lane = threadIdx.x & 31;
   if (col >= L.npl + L.nbg) return;
@@ -155,6 +157,7 @@ __global__ void k_plume_write(PlumeLattice L, const int64_t* __restrict__ off, P
 
 // the jittered thermal, one thread per parcel (the host generator's formula)
 __global__ void k_thermal(pmpic_thermal_params prm, ThermalGeom tg, int64_t n, ParcelSink out) {
+  PDL_WAIT();
   const int64_t t = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
   if (t >= n) return;
   const ThermalParcel p = thermal_parcel(prm, tg, t);
@@ -178,6 +181,7 @@ __device__ __forceinline__ double lattice_coord(double pmin, int n, double d, do
   return pmin + (double)(n - 1) * d + b;
 }
 __global__ void k_basic(BasicLattice L, int64_t n, ParcelSink out) {
+  PDL_WAIT();
   const int64_t t = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
   if (t >= n) return;
   const int64_t per_cell = (int64_t)L.s * L.s * L.s;
@@ -329,7 +333,7 @@ int setup_plume(pmpic_ctx* ctx, const pmpic_plume_params* prm, int64_t* n_plume_
     L.bbg = dtab + o_bbg; L.hbg = dtab + o_hbg;
     err = cudaMemcpyAsync(dtab, tab.data(), sizeof(double) * tab.size(), cudaMemcpyHostToDevice, ctx->stream);
     if (err == cudaSuccess) {
-      k_plume_count<<<nblk(ncol * 32, 256), 256, 0, ctx->stream>>>(L, dcount); ++ctx->nlaunch;
+      launch(ctx->stream, nblk(ncol * 32, 256), 256, 0, k_plume_count, L, dcount); ++ctx->nlaunch;
       err = cudaGetLastError();
     }
     // slots in the reference's loop order: an exclusive scan of the columns
@@ -350,7 +354,7 @@ int setup_plume(pmpic_ctx* ctx, const pmpic_plume_params* prm, int64_t* n_plume_
     if (!rc) {
       err = cudaMemcpyAsync(doff, off.data(), sizeof(int64_t) * ncol, cudaMemcpyHostToDevice, ctx->stream);
       if (err == cudaSuccess) {
-        k_plume_write<<<nblk(ncol * 32, 256), 256, 0, ctx->stream>>>(L, doff, sink_of(ctx)); ++ctx->nlaunch;
+        launch(ctx->stream, nblk(ncol * 32, 256), 256, 0, k_plume_write, L, doff, sink_of(ctx)); ++ctx->nlaunch;
         err = cudaGetLastError();
       }
       if (err == cudaSuccess) err = cudaStreamSynchronize(ctx->stream);
@@ -379,7 +383,7 @@ int setup_basic(pmpic_ctx* ctx, int n_per_dir) {
   L.dx = g.dx; L.dy = g.dy; L.dz = g.dz;
   L.bx = ctx->cfg.xmin; L.by = ctx->cfg.ymin; L.bz = ctx->cfg.zmin;
   if (n > 0) {
-    k_basic<<<nblk(n, 256), 256, 0, ctx->stream>>>(L, n, sink_of(ctx)); ++ctx->nlaunch;
+    launch(ctx->stream, nblk(n, 256), 256, 0, k_basic, L, n, sink_of(ctx)); ++ctx->nlaunch;
     PMPIC_CUDA(cudaGetLastError());
   }
   return finish_state(ctx, n, {PMPIC_PROP_X, PMPIC_PROP_Y, PMPIC_PROP_Z, PMPIC_PROP_VOL});
@@ -391,7 +395,7 @@ int setup_thermal_device(pmpic_ctx* ctx, const pmpic_thermal_params* prm) {
   if (n < 0) return set_error(ctx, PMPIC_ERR_ARG, "thermal set-up: bad parameters");
   if (n > ctx->cap) return set_error(ctx, PMPIC_ERR_CAPACITY, "thermal set-up: parcel count exceeds max_parcels");
   if (n > 0) {
-    k_thermal<<<nblk(n, 256), 256, 0, ctx->stream>>>(*prm, thermal_geom(prm), n, sink_of(ctx)); ++ctx->nlaunch;
+    launch(ctx->stream, nblk(n, 256), 256, 0, k_thermal, *prm, thermal_geom(prm), n, sink_of(ctx)); ++ctx->nlaunch;
     PMPIC_CUDA(cudaGetLastError());
   }
   return finish_state(ctx, n, {PMPIC_PROP_X, PMPIC_PROP_Y, PMPIC_PROP_Z, PMPIC_PROP_B, PMPIC_PROP_H, PMPIC_PROP_VOL,

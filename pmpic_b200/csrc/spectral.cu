@@ -31,6 +31,7 @@ inline unsigned nblk(int64_t n, int b) { return (unsigned)((n + b - 1) / b); }
 // to every element before the sum).
 // d, e: the zero-mode values of each level
 __global__ void k_zmode(Geom g, const double* __restrict__ d, const double* __restrict__ e, double* __restrict__ zb) {
+  PDL_WAIT();
   extern __shared__ double zs[];  // e(:,1,1), d(:,1,1), then ubar, vbar
   const int nz = g.nzp;
   double* es = zs;
@@ -73,6 +74,7 @@ __global__ void k_zmode(Geom g, const double* __restrict__ d, const double* __re
 // by the mixed-precision form
 __global__ void __launch_bounds__(256) k_hsum2(Geom g, const float* __restrict__ p, const float* __restrict__ q,
                                                double* __restrict__ hs) {
+  PDL_WAIT();
   __shared__ double sp[256], sq[256];
   const int k = blockIdx.x;
   const int64_t m = (int64_t)g.Ny * g.Nx;
@@ -142,17 +144,20 @@ __device__ __forceinline__ bool ew_index(const Geom& g, EwIdx& x) {
 }
 
 __global__ void k_diffx(Geom g, const double* __restrict__ in, double* __restrict__ out, const double* __restrict__ kx) {
+  PDL_WAIT();
   EwIdx x;
   if (!ew_index(g, x)) return;
   out[x.e] = dx_of(in, x.e, x.ip, kx);
 }
 __global__ void k_diffy(Geom g, const double* __restrict__ in, double* __restrict__ out, const double* __restrict__ ky) {
+  PDL_WAIT();
   EwIdx x;
   if (!ew_index(g, x)) return;
   out[x.e] = dy_of(in, x.e, x.jp, g.sx, ky);
 }
 __global__ void k_filter(Geom g, const double* __restrict__ in, double* __restrict__ out,
                          const double* __restrict__ filt) {
+  PDL_WAIT();
   EwIdx x;
   if (!ew_index(g, x)) return;
   out[x.e] = in[x.e] * filt[x.col];
@@ -172,6 +177,7 @@ __global__ void k_filter(Geom g, const double* __restrict__ in, double* __restri
 __global__ void k_diffz(Geom g, const double* __restrict__ f, double* __restrict__ out,
                         const double* __restrict__ bot, const double* __restrict__ top,
                         const double* __restrict__ coef /* a[nz], den[nz], cp[nz] */, double a1) {
+  PDL_WAIT();
   const int col = blockIdx.x * blockDim.x + threadIdx.x;
   const int cols = g.sx * g.sy;
   if (col >= cols) return;
@@ -238,6 +244,7 @@ __global__ void k_diffz(Geom g, const double* __restrict__ f, double* __restrict
 // blockIdx.y selects one of up to three arrays solved in the same launch
 __global__ void k_laplinv(Geom g, double* __restrict__ f, int df0, const double* __restrict__ tab,
                           const double* __restrict__ k2) {
+  PDL_WAIT();
   const int col = blockIdx.x * blockDim.x + threadIdx.x;
   const int cols = g.sx * g.sy;
   if (col >= cols) return;
@@ -318,6 +325,7 @@ __global__ void k_laplinv(Geom g, double* __restrict__ f, int df0, const double*
 
 // dt rule (vort2vel.F90:329-372, vorticity_tendency.F90:277-313), one thread
 __global__ void k_dt_velocity(Geom g, DevInfo* info, double dtmax) {
+  PDL_WAIT();
   double umax = sqrt(info->umax2), vmax = sqrt(info->vmax2), wmax = sqrt(info->wmax2);
   if (umax == 0) umax = f4(1.E-15f);
   if (vmax == 0) vmax = f4(1.E-15f);
@@ -333,6 +341,7 @@ __global__ void k_dt_velocity(Geom g, DevInfo* info, double dtmax) {
   }
 }
 __global__ void k_dt_vorticity(DevInfo* info, double prefactor, double dtmax) {
+  PDL_WAIT();
   double omax = sqrt(info->omax2);
   double dtw = (omax > 0.) ? prefactor / omax : dtmax;
   if (info->dtm > dtw) {
@@ -442,6 +451,7 @@ struct ZTab {
 };
 // rh = 1 / den rounded, rl = its residual: n rh + n rl is n / den before rounding
 __global__ void k_recip(int64_t n, const double* __restrict__ den, double* __restrict__ rh, double* __restrict__ rl) {
+  PDL_WAIT();
   const int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
   if (i >= n) return;
   const double d = den[i], h = 1.0 / d;
@@ -493,9 +503,10 @@ inline ZTab<float> lap_tab(pmpic_ctx* c, int form) {
 // FP64 before the FP32 transforms, then the FP64 mean-flow integral
 inline int zero_mode(pmpic_ctx* ctx) {
   const Geom& g = ctx->g;
-  k_hsum2<<<g.nzp, 256, 0, ctx->stream>>>(g, (const float*)ctx->grid[PMPIC_GRID_P], (const float*)ctx->grid[PMPIC_GRID_Q],
-                                          ctx->hsum); ++ctx->nlaunch;
-  k_zmode<<<1, 256, sizeof(double) * 4 * g.nzp, ctx->stream>>>(g, ctx->hsum, ctx->hsum + g.nzp, ctx->zmode); ++ctx->nlaunch;
+  launch(ctx->stream, g.nzp, 256, 0, k_hsum2, g, (const float*)ctx->grid[PMPIC_GRID_P],
+         (const float*)ctx->grid[PMPIC_GRID_Q], ctx->hsum); ++ctx->nlaunch;
+  launch(ctx->stream, 1, 256, sizeof(double) * 4 * g.nzp, k_zmode, g, ctx->hsum, ctx->hsum + g.nzp,
+         ctx->zmode); ++ctx->nlaunch;
   PMPIC_CUDA(cudaGetLastError());
   return 0;
 }
@@ -543,9 +554,9 @@ int spectral_init(pmpic_ctx* ctx) {
   PMPIC_CUDA(cudaMalloc(&ctx->zrec, sizeof(double) * (4 * nz + 4 * n)));
   for (int v = 0; v < 2; ++v) {
     double* r = ctx->zrec + v * 2 * nz;
-    k_recip<<<nblk(nz, 256), 256, 0, ctx->stream>>>(nz, f64::diffz_tab(ctx, v) + nz, r, r + nz);
+    launch(ctx->stream, nblk(nz, 256), 256, 0, k_recip, nz, f64::diffz_tab(ctx, v) + nz, r, r + nz);
     r = ctx->zrec + 4 * nz + v * 2 * n;
-    k_recip<<<nblk(n, 256), 256, 0, ctx->stream>>>(n, ctx->lapcp + 2 * v * n, r, r + n);
+    launch(ctx->stream, nblk(n, 256), 256, 0, k_recip, n, ctx->lapcp + 2 * v * n, r, r + n);
     ctx->nlaunch += 2;
   }
   PMPIC_CUDA(cudaStreamSynchronize(ctx->stream));
@@ -553,32 +564,33 @@ int spectral_init(pmpic_ctx* ctx) {
 }
 
 int spec_diffx(pmpic_ctx* ctx, const double* in, double* out) {
-  k_diffx<<<nblk(ctx->g.nspec, 256), 256, 0, ctx->stream>>>(ctx->g, in, out, ctx->kx); ++ctx->nlaunch;
+  launch(ctx->stream, nblk(ctx->g.nspec, 256), 256, 0, k_diffx, ctx->g, in, out, ctx->kx); ++ctx->nlaunch;
   PMPIC_CUDA(cudaGetLastError());
   return 0;
 }
 int spec_diffy(pmpic_ctx* ctx, const double* in, double* out) {
-  k_diffy<<<nblk(ctx->g.nspec, 256), 256, 0, ctx->stream>>>(ctx->g, in, out, ctx->ky); ++ctx->nlaunch;
+  launch(ctx->stream, nblk(ctx->g.nspec, 256), 256, 0, k_diffy, ctx->g, in, out, ctx->ky); ++ctx->nlaunch;
   PMPIC_CUDA(cudaGetLastError());
   return 0;
 }
 int spec_filter(pmpic_ctx* ctx, const double* in, double* out) {
-  k_filter<<<nblk(ctx->g.nspec, 256), 256, 0, ctx->stream>>>(ctx->g, in, out, ctx->filt); ++ctx->nlaunch;
+  launch(ctx->stream, nblk(ctx->g.nspec, 256), 256, 0, k_filter, ctx->g, in, out, ctx->filt); ++ctx->nlaunch;
   PMPIC_CUDA(cudaGetLastError());
   return 0;
 }
 int spec_diffz(pmpic_ctx* ctx, const double* in, double* out, const double* bot, const double* top) {
   TimerScope ts(ctx, T_DIFFZ);
   const Geom& g = ctx->g;
-  k_diffz<<<nblk((int64_t)g.sx * g.sy, 128), 128, 0, ctx->stream>>>(g, in, out, bot, top, f64::diffz_tab(ctx, bot ? 1 : 0),
-                                                                    f4div(1.f, 6.f)); ++ctx->nlaunch;
+  launch(ctx->stream, nblk((int64_t)g.sx * g.sy, 128), 128, 0, k_diffz, g, in, out, bot, top, f64::diffz_tab(ctx,
+         bot ? 1 : 0), f4div(1.f, 6.f)); ++ctx->nlaunch;
   PMPIC_CUDA(cudaGetLastError());
   return 0;
 }
 int spec_laplinv(pmpic_ctx* ctx, double* inout, bool df0) {
   TimerScope ts(ctx, T_LAPLINV);
   const Geom& g = ctx->g;
-  k_laplinv<<<nblk((int64_t)g.sx * g.sy, 128), 128, 0, ctx->stream>>>(g, inout, df0 ? 1 : 0, ctx->lapcp, ctx->k2); ++ctx->nlaunch;
+  launch(ctx->stream, nblk((int64_t)g.sx * g.sy, 128), 128, 0, k_laplinv, g, inout, df0 ? 1 : 0, ctx->lapcp,
+         ctx->k2); ++ctx->nlaunch;
   PMPIC_CUDA(cudaGetLastError());
   return 0;
 }
@@ -595,10 +607,11 @@ int field_max(pmpic_ctx* ctx, bool v2v, bool vt) {
   int rc = ctx->mixed ? f32::field_max_impl(ctx, v2v, vt) : f64::field_max_impl(ctx, v2v, vt);
   if (rc) return rc;
   if (v2v) {
-    k_dt_velocity<<<1, 1, 0, ctx->stream>>>(ctx->g, ctx->dinfo, ctx->cfg.dtmax); ++ctx->nlaunch;
+    launch(ctx->stream, 1, 1, 0, k_dt_velocity, ctx->g, ctx->dinfo, ctx->cfg.dtmax); ++ctx->nlaunch;
   }
   if (vt) {
-    k_dt_vorticity<<<1, 1, 0, ctx->stream>>>(ctx->dinfo, ctx->cfg.timestep_prefactor, ctx->cfg.dtmax); ++ctx->nlaunch;
+    launch(ctx->stream, 1, 1, 0, k_dt_vorticity, ctx->dinfo, ctx->cfg.timestep_prefactor,
+           ctx->cfg.dtmax); ++ctx->nlaunch;
   }
   PMPIC_CUDA(cudaGetLastError());
   return 0;

@@ -190,6 +190,7 @@ __host__ __device__ constexpr int inv_ring() {
 }
 template <int NC, bool GM>
 __global__ void __launch_bounds__(INV_T, 2) k_invert(Geom g, const __grid_constant__ InvArgs S) {
+  PDL_WAIT();
   constexpr int W = NC / 2, NG = INV_T / NC;
   extern __shared__ __align__(16) unsigned char zsm[];
   const int nz = g.nzp, sx = g.sx;
@@ -461,7 +462,7 @@ int invert_launch(pmpic_ctx* ctx, real* a, real* b, real* c, real* u, real* v, r
   S.rdzl = (real)(std::fma(-g.dz, r, 1.0) * r);
   S.rdz64 = 1.0 / (double)(real)g.dz;
   S.nxt = (g.sx + p.nc / 2 - 1) / (p.nc / 2);
-  invert_kernel(p, [&](auto k) { k<<<(unsigned)(S.nxt * (g.sy / 2)), INV_T, p.bytes, ctx->stream>>>(g, S); });
+  invert_kernel(p, [&](auto k) { launch(ctx->stream, (unsigned)(S.nxt * (g.sy / 2)), INV_T, p.bytes, k, g, S); });
   ++ctx->nlaunch;
   PMPIC_CUDA(cudaGetLastError());
   return 0;
@@ -483,6 +484,7 @@ __device__ __forceinline__ void cta_max(real m, double* __restrict__ out) {
 // vorticity_tendency.F90:279-282); non-negative doubles order like their bits
 __global__ void k_max_sq3(int64_t n, const real* __restrict__ u, const real* __restrict__ v,
                           const real* __restrict__ w, double* __restrict__ out3) {
+  PDL_WAIT();
   real mu = 0, mv = 0, mw = 0;
   for (int64_t e = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; e < n; e += (int64_t)gridDim.x * blockDim.x) {
     real a = u[e], b = v[e], c = w[e];
@@ -496,6 +498,7 @@ __global__ void k_max_sq3(int64_t n, const real* __restrict__ u, const real* __r
 }
 __global__ void k_max_vort(int64_t n, const real* __restrict__ p, const real* __restrict__ q,
                            const real* __restrict__ r, double* __restrict__ out) {
+  PDL_WAIT();
   real m = 0;
   for (int64_t e = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; e < n; e += (int64_t)gridDim.x * blockDim.x) {
     real a = p[e], b = q[e], c = r[e];
@@ -563,13 +566,13 @@ int field_max_impl(pmpic_ctx* ctx, bool v2v, bool vt) {
   const Geom& g = ctx->g;
   if (v2v) {
     PMPIC_CUDA(cudaMemsetAsync(&ctx->dinfo->umax2, 0, 3 * sizeof(double), ctx->stream));
-    k_max_sq3<<<592, 256, 0, ctx->stream>>>(g.nphys, G[PMPIC_GRID_U], G[PMPIC_GRID_V],
-                                            G[PMPIC_GRID_W], &ctx->dinfo->umax2); ++ctx->nlaunch;
+    launch(ctx->stream, 592, 256, 0, k_max_sq3, g.nphys, G[PMPIC_GRID_U], G[PMPIC_GRID_V], G[PMPIC_GRID_W],
+           &ctx->dinfo->umax2); ++ctx->nlaunch;
   }
   if (vt) {
     PMPIC_CUDA(cudaMemsetAsync(&ctx->dinfo->omax2, 0, sizeof(double), ctx->stream));
-    k_max_vort<<<592, 256, 0, ctx->stream>>>(g.nphys, G[PMPIC_GRID_P], G[PMPIC_GRID_Q],
-                                             G[PMPIC_GRID_R], &ctx->dinfo->omax2); ++ctx->nlaunch;
+    launch(ctx->stream, 592, 256, 0, k_max_vort, g.nphys, G[PMPIC_GRID_P], G[PMPIC_GRID_Q], G[PMPIC_GRID_R],
+           &ctx->dinfo->omax2); ++ctx->nlaunch;
   }
   PMPIC_CUDA(cudaGetLastError());
   return 0;
