@@ -182,16 +182,15 @@ __device__ __forceinline__ void zwalk(real* X, int k0, int k1, real below, real 
   }
 }
 
-constexpr int INV_T = 256;
 // values of the rings of the three chain warps
 template <int NC>
 __host__ __device__ constexpr int inv_ring() {
   return 3 * ZRING * ZCH * (NC / 4) * (sizeof(real) == 8 ? 2 : 1);
 }
-template <int NC, bool GM>
-__global__ void __launch_bounds__(INV_T, 2) k_invert(Geom g, const __grid_constant__ InvArgs S) {
+template <int NC, int NT, bool GM>
+__global__ void __launch_bounds__(NT, 512 / NT) k_invert(Geom g, const __grid_constant__ InvArgs S) {
   PDL_WAIT();
-  constexpr int W = NC / 2, NG = INV_T / NC;
+  constexpr int W = NC / 2, NG = NT / NC;
   extern __shared__ __align__(16) unsigned char zsm[];
   const int nz = g.nzp, sx = g.sx;
   const int64_t cs = (int64_t)sx * g.sy;
@@ -308,7 +307,7 @@ __global__ void __launch_bounds__(INV_T, 2) k_invert(Geom g, const __grid_consta
   if (threadIdx.x < 32) {
     thomas<NC, 1>(F + col, lanecol && in, 0, nz, f16, real(0), S.dz[0], 0, 1, ring);
   } else if (in) {
-    for (int k = (threadIdx.x - 32) / NC; k < nz; k += (INV_T - 32) / NC) {
+    for (int k = (threadIdx.x - 32) / NC; k < nz; k += (NT - 32) / NC) {
       S.a[at(k)] = A[k * NC + col] * fl;
       S.b[at(k)] = B[k * NC + col] * fl;
     }
@@ -413,29 +412,44 @@ __global__ void __launch_bounds__(INV_T, 2) k_invert(Geom g, const __grid_consta
   }
 }
 
-// Columns per tile: as many as let two CTAs share an SM's 227 KB, fewer while
-// the grid has not a tile per SM; one CTA per SM, and then global memory in
-// place of shared memory, only for more levels than 8 columns can hold.
+// Columns per tile and threads per CTA.  A tile costs five recurrences over
+// the levels one after the other, whatever its width, so:
+// - The narrowest tiles that are on the device all at once, four CTAs of 128
+//   threads to an SM at most (96^3 FP32, 32 columns: 0.224 ms a step, 0.332
+//   with two CTAs of 256 threads to an SM, and 0.321 for 16 columns, whose 576
+//   CTAs nearly fill the 592 places: hence nine tenths of them; 64^3, 8
+//   columns: 0.124, 0.197 for 16 and 256 threads).  With a CTA or less per SM,
+//   256 threads (32^3 FP64: 0.109 against 0.115).
+// - Else the widest tiles of which two share an SM, with 128 threads where
+//   three do (128^3 FP64, 16 columns: 0.787 against 0.850) and otherwise 256
+//   (256^3 FP32, 32 columns: 3.26 against 3.91, and 3.43 for 16 columns).
+// - One CTA per SM, and then global memory in place of shared memory, only for
+//   more levels than 8 columns can hold.
 struct InvPlan {
-  int nc;
+  int nc, nt;
   bool gm;
   size_t bytes;  // of shared memory
 };
 InvPlan invert_plan(const Geom& g) {
+  constexpr int64_t SMS = 148, KB = 1024;
   auto ring = [&](int nc) { return (size_t)3 * ZRING * ZCH * (nc / 4) * (sizeof(real) == 8 ? 2 : 1); };
   auto bytes = [&](int nc) { return ((size_t)3 * g.nzp * nc + ring(nc)) * sizeof(real); };
   auto tiles = [&](int nc) { return (int64_t)(g.sy / 2) * ((g.sx + nc / 2 - 1) / (nc / 2)); };
+  for (int nc = 8; nc <= 32; nc *= 2) {
+    const int64_t places = SMS * min((int64_t)4, 225 * KB / ((int64_t)bytes(nc) + KB));
+    if (tiles(nc) * 10 <= places * 9) return InvPlan{nc, tiles(nc) <= SMS ? 256 : 128, false, bytes(nc)};
+  }
   int nc = 32;
-  while (nc > 8 && (bytes(nc) > 112 * 1024 || tiles(nc) < 148)) nc /= 2;
-  const bool gm = bytes(nc) > 224 * 1024;
-  return InvPlan{nc, gm, gm ? ring(nc) * sizeof(real) : bytes(nc)};
+  while (nc > 8 && (int64_t)bytes(nc) > 112 * KB) nc /= 2;
+  if ((int64_t)bytes(nc) > 224 * KB) return InvPlan{nc, 256, true, ring(nc) * sizeof(real)};
+  return InvPlan{nc, (int64_t)bytes(nc) <= 74 * KB ? 128 : 256, false, bytes(nc)};
 }
 template <class F>
 void invert_kernel(const InvPlan& p, F&& f) {
-  if (p.gm) f(k_invert<8, true>);
-  else if (p.nc == 32) f(k_invert<32, false>);
-  else if (p.nc == 16) f(k_invert<16, false>);
-  else f(k_invert<8, false>);
+  if (p.gm) f(k_invert<8, 256, true>);
+  else if (p.nc == 32) f(p.nt == 128 ? k_invert<32, 128, false> : k_invert<32, 256, false>);
+  else if (p.nc == 16) f(p.nt == 128 ? k_invert<16, 128, false> : k_invert<16, 256, false>);
+  else f(p.nt == 128 ? k_invert<8, 128, false> : k_invert<8, 256, false>);
 }
 int invert_init(pmpic_ctx* ctx) {
   const Geom& g = ctx->g;
@@ -462,7 +476,7 @@ int invert_launch(pmpic_ctx* ctx, real* a, real* b, real* c, real* u, real* v, r
   S.rdzl = (real)(std::fma(-g.dz, r, 1.0) * r);
   S.rdz64 = 1.0 / (double)(real)g.dz;
   S.nxt = (g.sx + p.nc / 2 - 1) / (p.nc / 2);
-  invert_kernel(p, [&](auto k) { launch(ctx->stream, (unsigned)(S.nxt * (g.sy / 2)), INV_T, p.bytes, k, g, S); });
+  invert_kernel(p, [&](auto k) { launch(ctx->stream, (unsigned)(S.nxt * (g.sy / 2)), p.nt, p.bytes, k, g, S); });
   ++ctx->nlaunch;
   PMPIC_CUDA(cudaGetLastError());
   return 0;
