@@ -1147,6 +1147,16 @@ int par2grid_multi(pmpic_ctx* ctx, const double* const* fields, int nf, double* 
   }
 }
 
+// Six grids go through their packed copy (k_grid2par6: a corner's two levels
+// of all six in 12 consecutive values, where the grids themselves take 12
+// accesses of one value) when there are enough parcels to pay for the copy.
+// Measured, direct -> packed, in us: 128^3 with 8 parcels per cell at random
+// slots FP64 3097 -> 1485, FP32 2409 -> 963, in cell order 603 -> 480 and
+// 478 -> 237; one parcel to two cells, FP64, 198 -> 148 and 158 -> 97; to four
+// 104 -> 103, to eight 65 -> 80.  32^3 with 65,536 parcels 16.5 -> 16.7, with
+// 32,768 12.7 -> 14.9 (the copy's launch).  The same operations either way.
+static bool g2p_packs(const pmpic_ctx* ctx) { return 2 * ctx->n >= ctx->g.nphys && ctx->n >= 65536; }
+
 template <int NG>
 static int launch_g2p(pmpic_ctx* ctx, const double* const* grids, double* const* out) {
   TimerScope ts(ctx, T_G2P);
@@ -1213,7 +1223,10 @@ int grid2par_multi_m(pmpic_ctx* ctx, const float* const* grids, int ng, float* c
   switch (ng) {
     case 1: run(std::integral_constant<int, 1>{}); break;
     case 3: run(std::integral_constant<int, 3>{}); break;
-    case 6: run(std::integral_constant<int, 6>{}); break;
+    case 6:
+      if (g2p_packs(ctx)) return grid2par_six_m(ctx, grids, out);
+      run(std::integral_constant<int, 6>{});
+      break;
     default: return set_error(ctx, PMPIC_ERR_ARG, "grid2par_multi_m: 1, 3 or 6 grids");
   }
   PMPIC_CUDA(cudaGetLastError());
@@ -1229,7 +1242,11 @@ int grid2par_multi(pmpic_ctx* ctx, const double* const* grids, int ng, double* c
   switch (ng) {
     case 1: return launch_g2p<1>(ctx, grids, out);
     case 3: return launch_g2p<3>(ctx, grids, out);
-    case 6: return launch_g2p<6>(ctx, grids, out);
+    case 6: {
+      if (!g2p_packs(ctx)) return launch_g2p<6>(ctx, grids, out);
+      TimerScope ts(ctx, T_G2P);
+      return grid2par_six(ctx, grids, out);
+    }
     default: return set_error(ctx, PMPIC_ERR_ARG, "grid2par_multi: 1, 3 or 6 grids");
   }
 }
