@@ -27,7 +27,7 @@ inline real* RP(P* p) { return reinterpret_cast<real*>(p); }
 // Arithmetic and its order are the separate operators'.
 // Measured, ms per step for all that lies between the transforms (ten kernels
 // before, and the velocity spectra formed by the inverse x pass): 32^3 FP64
-// 0.60 -> 0.11, 96^3 FP32 0.85 -> 0.33, 128^3 FP64 2.0 -> 0.85; 256^3 FP32
+// 0.60 -> 0.11, 96^3 FP32 0.85 -> 0.22, 128^3 FP64 2.0 -> 0.79; 256^3 FP32
 // 3.25 -> 3.26, but its inverse transforms 5.0 instead of 6.5.
 struct InvArgs {
   real *a, *b, *c;           // in: the spectra; out: corrected and filtered
@@ -412,7 +412,7 @@ __global__ void __launch_bounds__(NT, 512 / NT) k_invert(Geom g, const __grid_co
   }
 }
 
-// Columns per tile and threads per CTA.  A tile costs five recurrences over
+// Columns per tile and threads per CTA.  A tile costs four recurrences over
 // the levels one after the other, whatever its width, so:
 // - The narrowest tiles that are on the device all at once, four CTAs of 128
 //   threads to an SM at most (96^3 FP32, 32 columns: 0.224 ms a step, 0.332
