@@ -323,6 +323,9 @@ int pmpic_create(const pmpic_config* cfg, pmpic_ctx** out) {
     DevInfo h{};
     h.dtm = cfg->dtm;  // rk4_integrator.F90:38-41
     e = cudaMemcpy(ctx->dinfo, &h, sizeof(DevInfo), cudaMemcpyHostToDevice);
+    // the tables' and counters' copies have arrived before the context's own
+    // stream, which does not wait for the default stream, reads any of them
+    if (e == cudaSuccess) e = cudaStreamSynchronize(nullptr);
     if (e != cudaSuccess) rc = cuda_fail(ctx, e, "dinfo", __LINE__);
   }
   for (int i = 0; i < 8 && !rc; ++i) {

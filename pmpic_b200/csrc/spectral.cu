@@ -552,6 +552,9 @@ int spectral_init(pmpic_ctx* ctx) {
   // the FP64 inversion's reciprocal pivots, from the pivots of both solvers
   const int64_t n = (int64_t)(g.sx >> 1) * (g.sy >> 1) * nz;
   PMPIC_CUDA(cudaMalloc(&ctx->zrec, sizeof(double) * (4 * nz + 4 * n)));
+  // A copy from pageable memory may return before it has arrived, and the
+  // context's stream does not wait for the default stream that makes it.
+  PMPIC_CUDA(cudaStreamSynchronize(nullptr));
   for (int v = 0; v < 2; ++v) {
     double* r = ctx->zrec + v * 2 * nz;
     launch(ctx->stream, nblk(nz, 256), 256, 0, k_recip, nz, f64::diffz_tab(ctx, v) + nz, r, r + nz);
