@@ -168,10 +168,19 @@ __global__ void __launch_bounds__(256) k_bin_scatter(int64_t n, const int32_t* _
 // lattices, or of splits) is no work for one thread: its warp ranks the slots
 // against each other, a lane an entry, and writes them to their places
 // (the plume set-up, whose plume has 64 parcels a cell: binning of 10 steps at
-// 64^3 FP32 7.3 -> 3.3 ms, 32^3 FP64 6.1 -> 2.0).
+// 64^3 FP32 7.0 -> 3.0 ms, 32^3 FP64 5.7 -> 1.6).
+// Which of the two: a warp's insertion sorts last as long as its fullest
+// cell's, up to the square of that cell's entries, while ranking takes the sum
+// over its cells, a step an entry and 32 of them.  So cells of more than
+// SORT_RANK entries are ranked where three times that sum is at most the
+// square, or where a cell has more than SORT_CROWD.  Evenly full cells stay
+// with the threads: binning at 48^3, 27 parcels a cell at random slots, 170 us
+// when all were ranked, 136 (FP32 156 and 124); 64^3 with 20, 254 and 220; the
+// plume's figures above are the same with either.
 constexpr int SORT_CELLS = 256;
 constexpr int SORT_CAP = 8192;  // index entries a CTA stages (32 KB)
 constexpr int SORT_RANK = 16, SORT_RANK_MAX = 512;  // entries of a cell that is ranked: above, at most
+constexpr int SORT_CROWD = 56;
 __global__ void __launch_bounds__(SORT_CELLS) k_sort_segments(int64_t ncell, const int32_t* __restrict__ start,
                                                               const int32_t* __restrict__ fill,
                                                               int32_t* __restrict__ sorted) {
@@ -204,7 +213,10 @@ __global__ void __launch_bounds__(SORT_CELLS) k_sort_segments(int64_t ncell, con
   if (m <= SORT_CAP) {  // uniform over the CTA
     for (int e = threadIdx.x; e < m; e += SORT_CELLS) buf[skew(e)] = sorted[base + e];
     __syncthreads();
-    const bool ranked = len > SORT_RANK && len <= SORT_RANK_MAX;
+    bool ranked = len > SORT_RANK && len <= SORT_RANK_MAX;
+    const int fullest = __reduce_max_sync(0xffffffffu, len);
+    const int steps = __reduce_add_sync(0xffffffffu, ranked ? len * ((len + 31) / 32) : 0);
+    ranked = ranked && (fullest > SORT_CROWD || 3 * steps <= fullest * fullest);
     if (!ranked) isort(buf, s0, len, skew);
     __syncthreads();
     for (int e = threadIdx.x; e < m; e += SORT_CELLS) sorted[base + e] = buf[skew(e)];
