@@ -177,9 +177,18 @@ __global__ void __launch_bounds__(256) k_bin_scatter(int64_t n, const int32_t* _
 // with the threads: binning at 48^3, 27 parcels a cell at random slots, 170 us
 // when all were ranked, 136 (FP32 156 and 124); 64^3 with 20, 254 and 220; the
 // plume's figures above are the same with either.
+// A range of more than SORT_CAP entries (more than 32 a cell on average) is
+// staged in several passes, as many whole cells in each as fit; only a cell
+// that is longer by itself is sorted in place, by one thread.  Of ranked cells
+// a warp takes its own where one pass does, and every eighth where a pass holds
+// the cells of a few warps; a cell of more than SORT_WIDE entries all threads
+// take together.  Against sorting such ranges in place and such cells by one
+// thread: 64^3 with 64 parcels a cell jittered across cells 4.2 -> 0.75 ms
+// (before the ranking 4.05), 32^3 with 700 in every eighth cell 1.8 to 22 ms,
+// by their order, -> 1.0 to 1.9.
 constexpr int SORT_CELLS = 256;
-constexpr int SORT_CAP = 8192;  // index entries a CTA stages (32 KB)
-constexpr int SORT_RANK = 16, SORT_RANK_MAX = 512;  // entries of a cell that is ranked: above, at most
+constexpr int SORT_CAP = 8192;                  // index entries a CTA stages (32 KB)
+constexpr int SORT_RANK = 16, SORT_WIDE = 256;  // entries above which a cell is ranked, and by the whole CTA
 constexpr int SORT_CROWD = 56;
 __global__ void __launch_bounds__(SORT_CELLS) k_sort_segments(int64_t ncell, const int32_t* __restrict__ start,
                                                               const int32_t* __restrict__ fill,
@@ -188,16 +197,18 @@ __global__ void __launch_bounds__(SORT_CELLS) k_sort_segments(int64_t ncell, con
   // staged position e sits at e + e/8: segments (~8 parcels each) start in
   // different banks for neighbouring threads
   __shared__ int32_t buf[SORT_CAP + SORT_CAP / 8];
+  // a cell's first entry, from the CTA's first; the top bit marks cells that are not
+  // their own warp's to rank.  (With one word more, an SM would hold five CTAs, not six.)
+  __shared__ unsigned first[SORT_CELLS];
+  const int t = threadIdx.x;
   const int64_t c0 = (int64_t)blockIdx.x * SORT_CELLS;
-  const int64_t c = c0 + threadIdx.x;
-  if (!__syncthreads_or(c < ncell && fill[c] != 0)) return;  // every segment here is one run: in order
+  const int64_t c = c0 + t;
+  const bool unordered = c < ncell && fill[c] != 0;
+  if (!__syncthreads_or(unordered)) return;  // every segment here is one run: in order
   const int64_t c1 = min(c0 + SORT_CELLS, ncell);
   const int base = start[c0], m = start[c1] - base;
-  int s0 = 0, len = 0;
-  if (c < ncell) {
-    s0 = start[c] - base;
-    len = start[c + 1] - base - s0;
-  }
+  const int s0 = c < ncell ? start[c] - base : m, s1 = c < ncell ? start[c + 1] - base : m;
+  const int len = unordered ? s1 - s0 : 0;
   auto isort = [](int32_t* s, int s0, int len, auto at) {
     for (int u = 1; u < len; ++u) {
       const int32_t v = s[at(s0 + u)];
@@ -210,30 +221,59 @@ __global__ void __launch_bounds__(SORT_CELLS) k_sort_segments(int64_t ncell, con
     }
   };
   auto skew = [](int e) { return e + (e >> 3); };
-  if (m <= SORT_CAP) {  // uniform over the CTA
-    for (int e = threadIdx.x; e < m; e += SORT_CELLS) buf[skew(e)] = sorted[base + e];
+  // a cell of cl entries from cs on in the buffer, by the threads i, i + step, ...
+  auto rank = [&](int cs, int cl, int b, int i, int step) {
+    for (int e = i; e < cl; e += step) {
+      const int32_t v = buf[skew(cs + e)];
+      int r = 0;  // (the slots of a cell are distinct)
+      for (int q = 0; q < cl; ++q) r += buf[skew(cs + q)] < v;
+      sorted[base + b + cs + r] = v;
+    }
+  };
+  const bool one = m <= SORT_CAP;  // (uniform over the CTA)
+  const bool wide = len > SORT_WIDE && len <= SORT_CAP;
+  bool ranked = len > SORT_RANK && len <= SORT_WIDE;
+  const int fullest = __reduce_max_sync(0xffffffffu, len);
+  const int steps = __reduce_add_sync(0xffffffffu, ranked ? len * ((len + 31) / 32) : 0);
+  ranked = ranked && (fullest > SORT_CROWD || 3 * steps <= fullest * fullest);
+  const bool shared = wide || (ranked && !one);
+  first[t] = (unsigned)s0 | (shared ? 1u << 31 : 0u);
+  auto begin = [&](int u) { return u < SORT_CELLS ? (int)(first[u] & 0x7fffffffu) : m; };
+  if (!one) __syncthreads();
+  for (int u0 = 0; u0 < SORT_CELLS;) {  // (uniform over the CTA)
+    const int b = one ? 0 : begin(u0);
+    // s1 rises with t: cells u0 .. u0 + fit - 1
+    const int fit = one ? SORT_CELLS : __syncthreads_count(t >= u0 && s1 - b <= SORT_CAP);
+    if (fit == 0) {
+      if (t == u0) isort(sorted + base, s0, len, [](int e) { return e; });
+      ++u0;
+      continue;
+    }
+    const int u1 = u0 + fit, k = one ? m : begin(u1) - b;
+    for (int e = t; e < k; e += SORT_CELLS) buf[skew(e)] = sorted[base + b + e];
     __syncthreads();
-    bool ranked = len > SORT_RANK && len <= SORT_RANK_MAX;
-    const int fullest = __reduce_max_sync(0xffffffffu, len);
-    const int steps = __reduce_add_sync(0xffffffffu, ranked ? len * ((len + 31) / 32) : 0);
-    ranked = ranked && (fullest > SORT_CROWD || 3 * steps <= fullest * fullest);
-    if (!ranked) isort(buf, s0, len, skew);
-    __syncthreads();
-    for (int e = threadIdx.x; e < m; e += SORT_CELLS) sorted[base + e] = buf[skew(e)];
-    unsigned big = __ballot_sync(0xffffffffu, ranked);
+    if (!ranked && !wide && t >= u0 && t < u1) isort(buf, s0 - b, len, skew);
+    const bool any = __syncthreads_or(shared);
+    for (int e = t; e < k; e += SORT_CELLS) sorted[base + b + e] = buf[skew(e)];
+    unsigned own = __ballot_sync(0xffffffffu, ranked && one);
     __syncthreads();  // the ranked cells' entries are written again, after that copy
-    while (big) {
-      const int src = __ffs(big) - 1, cs = __shfl_sync(0xffffffffu, s0, src), cl = __shfl_sync(0xffffffffu, len, src);
-      big &= big - 1;
-      for (int e = threadIdx.x & 31; e < cl; e += 32) {
-        const int32_t v = buf[skew(cs + e)];
-        int r = 0;  // (the slots of a cell are distinct)
-        for (int u = 0; u < cl; ++u) r += buf[skew(cs + u)] < v;
-        sorted[base + cs + r] = v;
+    for (; own; own &= own - 1) {
+      const int src = __ffs(own) - 1;
+      rank(__shfl_sync(0xffffffffu, s0, src), __shfl_sync(0xffffffffu, len, src), 0, t & 31, 32);
+    }
+    int turn = 0;
+    for (int w = u0 >> 5; any && 32 * w < u1; ++w) {
+      unsigned left = __ballot_sync(0xffffffffu, first[32 * w + (t & 31)] >> 31);
+      for (; left; left &= left - 1) {
+        const int u = 32 * w + __ffs(left) - 1;
+        if (u < u0 || u >= u1) continue;
+        const int cs = begin(u) - b, cl = begin(u + 1) - b - cs;
+        if (cl > SORT_WIDE) rank(cs, cl, b, t, SORT_CELLS);
+        else if ((turn++ & (SORT_CELLS / 32 - 1)) == t >> 5) rank(cs, cl, b, t & 31, 32);
       }
     }
-  } else {  // cells holding more than SORT_CAP parcels together: in place in global memory
-    isort(sorted + base, s0, len, [](int e) { return e; });
+    u0 = u1;
+    if (u0 < SORT_CELLS) __syncthreads();  // the buffer is filled again
   }
 }
 

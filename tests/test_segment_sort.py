@@ -39,3 +39,15 @@ def index_order(shape, counts, precision, seed):
 def test_which_cells_are_ranked(counts, precision):
     got, want = index_order((8, 6, 16), counts, precision, 7)
     np.testing.assert_array_equal(got, want)
+
+
+# cells that a warp and that the whole CTA ranks, CTAs whose 256 cells hold more than the 8192 entries that
+# are staged at a time, cells of just 8192 and more, and all of these beside ordinary and empty ones
+@pytest.mark.parametrize("counts", [[33], [64], [256, 257], [513, 0, 8], [700, 3], [8191, 1, 8], [8192, 8], [8193, 17, 64],
+                                    [9000, 0, 0, 40, 40], [30] * 31 + [8192], [2000, 6000, 192, 1]])
+@pytest.mark.parametrize("shape", [(4, 4, 3), (8, 6, 11)])
+def test_staged_in_passes(counts, shape):
+    if sum(counts) / len(counts) * np.prod(shape) > 2e6:
+        counts = counts + [8] * 30
+    got, want = index_order(shape, counts, "fp64", 9)
+    np.testing.assert_array_equal(got, want)
