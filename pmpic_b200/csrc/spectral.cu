@@ -26,46 +26,73 @@ namespace {
 
 inline unsigned nblk(int64_t n, int b) { return (unsigned)((n + b - 1) / b); }
 
-// mean flow of the zero mode (vort2vel.F90:230-241), one thread: the trapezoid
-// integral and the reference's average (`1./nz` in REAL(4), 0.5*ubar(nz) added
-// to every element before the sum).
-// d, e: the zero-mode values of each level
-__global__ void k_zmode(Geom g, const double* __restrict__ d, const double* __restrict__ e, double* __restrict__ zb) {
+// mean flow of the zero mode (vort2vel.F90:230-241): the trapezoid integral
+// and the reference's average (`1./nz` in REAL(4), 0.5*ubar(nz) added to every
+// element before the sum), both by one thread in order.
+// d, e: the zero-mode values of each level.  The columns pass through shared
+// memory ZM_L levels at a time, so that a box of any depth runs; one of more
+// levels keeps the integrals in zb in between.
+constexpr int ZM_L = 1024;
+__global__ void __launch_bounds__(256) k_zmode(Geom g, const double* __restrict__ d, const double* __restrict__ e,
+                                               double* zb) {
   PDL_WAIT();
-  extern __shared__ double zs[];  // e(:,1,1), d(:,1,1), then ubar, vbar
-  const int nz = g.nzp;
-  double* es = zs;
-  double* ds = zs + nz;
-  for (int k = threadIdx.x; k < nz; k += blockDim.x) {  // stage the zero-mode columns
-    es[k] = e[k];
-    ds[k] = d[k];
-  }
-  __syncthreads();
-  if (threadIdx.x != 0) return;
+  __shared__ double es[ZM_L + 1], ds[ZM_L + 1], us[ZM_L], vs[ZM_L], avg[2];
+  const int nz = g.nzp, t = threadIdx.x;
+  const bool deep = nz > ZM_L;
   double* ubar = zb;
   double* vbar = zb + nz;
   const double dz = g.dz;
   double u = 0, v = 0;
-  double* us = zs + 2 * nz;
-  double* vs = zs + 3 * nz;
-  us[0] = 0;
-  vs[0] = 0;
-  for (int k = 0; k < nz - 1; ++k) {
-    u = u + dz / 2. * (es[k] + es[k + 1]);
-    v = v - dz / 2. * (ds[k] + ds[k + 1]);
-    us[k + 1] = u;
-    vs[k + 1] = v;
+  for (int k0 = 0; k0 < nz; k0 += ZM_L) {
+    const int n = min(ZM_L, nz - k0);
+    for (int i = t; i < min(n + 1, nz - k0); i += 256) {
+      es[i] = e[k0 + i];
+      ds[i] = d[k0 + i];
+    }
+    __syncthreads();
+    if (t == 0) {
+      for (int i = 0; i < n; ++i) {
+        us[i] = u;
+        vs[i] = v;
+        if (k0 + i < nz - 1) {
+          u = u + dz / 2. * (es[i] + es[i + 1]);
+          v = v - dz / 2. * (ds[i] + ds[i + 1]);
+        }
+      }
+    }
+    __syncthreads();
+    for (int i = t; deep && i < n; i += 256) {
+      ubar[k0 + i] = us[i];
+      vbar[k0 + i] = vs[i];
+    }
   }
   const double inz = (double)(1.0f / (float)nz);
   double su = 0.0, sv = 0.0;
-  for (int k = 0; k < nz - 1; ++k) {
-    su = su + (us[k] + f4(0.5f) * us[nz - 1]);
-    sv = sv + (vs[k] + f4(0.5f) * vs[nz - 1]);
+  for (int k0 = 0; k0 < nz - 1; k0 += ZM_L) {
+    const int n = min(ZM_L, nz - 1 - k0);
+    if (deep) {
+      __syncthreads();
+      for (int i = t; i < n; i += 256) {
+        us[i] = ubar[k0 + i];
+        vs[i] = vbar[k0 + i];
+      }
+      __syncthreads();
+    }
+    if (t == 0) {
+      for (int i = 0; i < n; ++i) {
+        su = su + (us[i] + f4(0.5f) * u);
+        sv = sv + (vs[i] + f4(0.5f) * v);
+      }
+    }
   }
-  double uavg = inz * su, vavg = inz * sv;
-  for (int k = 0; k < nz; ++k) {
-    ubar[k] = us[k] - uavg;
-    vbar[k] = vs[k] - vavg;
+  if (t == 0) {
+    avg[0] = inz * su;
+    avg[1] = inz * sv;
+  }
+  __syncthreads();
+  for (int k = t; k < nz; k += 256) {
+    ubar[k] = (deep ? ubar[k] : us[k]) - avg[0];
+    vbar[k] = (deep ? vbar[k] : vs[k]) - avg[1];
   }
 }
 
@@ -505,7 +532,7 @@ inline int zero_mode(pmpic_ctx* ctx) {
   const Geom& g = ctx->g;
   launch(ctx->stream, g.nzp, 256, 0, k_hsum2, g, (const float*)ctx->grid[PMPIC_GRID_P],
          (const float*)ctx->grid[PMPIC_GRID_Q], ctx->hsum); ++ctx->nlaunch;
-  launch(ctx->stream, 1, 256, sizeof(double) * 4 * g.nzp, k_zmode, g, ctx->hsum, ctx->hsum + g.nzp,
+  launch(ctx->stream, 1, 256, 0, k_zmode, g, ctx->hsum, ctx->hsum + g.nzp,
          ctx->zmode); ++ctx->nlaunch;
   PMPIC_CUDA(cudaGetLastError());
   return 0;
@@ -543,12 +570,7 @@ int spectral_init(pmpic_ctx* ctx) {
   PMPIC_CUDA(cudaMemcpy(ctx->wn32, t32.data(), sizeof(float) * t32.size(), cudaMemcpyHostToDevice));
   PMPIC_CUDA(cudaMalloc(&ctx->hsum, sizeof(double) * 2 * g.nzp));
   if ((rc = laplinv_tables(ctx, tabs.data() + 2 * cols))) return rc;
-  if (ctx->mixed) {
-    const size_t zs = sizeof(double) * 4 * (size_t)nz;  // k_zmode's columns
-    if (zs > 48 * 1024)
-      PMPIC_CUDA(cudaFuncSetAttribute(k_zmode, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)zs));
-    return f32::invert_init(ctx);
-  }
+  if (ctx->mixed) return f32::invert_init(ctx);
   // the FP64 inversion's reciprocal pivots, from the pivots of both solvers
   const int64_t n = (int64_t)(g.sx >> 1) * (g.sy >> 1) * nz;
   PMPIC_CUDA(cudaMalloc(&ctx->zrec, sizeof(double) * (4 * nz + 4 * n)));
