@@ -344,7 +344,7 @@ struct pmpic_ctx {
   int32_t* cell_fill;        // ncell
   int32_t* keep;             // cap (mixing)
   int32_t* aux;              // cap (scans / migration lists)
-  int32_t* aux2;             // 2*nbmax + cap (compaction block counts, offsets, lists)
+  int32_t* aux2;             // nbmax + cap (compaction block counts, a list)
   int64_t nbmax;             // max compaction blocks: ceil(max(cap, ncell)/1024) + 8
   int8_t* dir;               // cap (haloswap direction)
   double* swapbuf;           // staging for migrating parcels (29 doubles each)
@@ -370,7 +370,6 @@ struct pmpic_ctx {
   float* ftw32;              // the same twiddles as float2 (mixed-precision form)
   double* zrec;              // reciprocal pivots of the FP64 inversion's z solves (spectral.cu)
   void* zwork;               // the inversion's columns when they exceed shared memory (else null)
-  int64_t zwork_bytes;
   float* wn32;               // FP32 kx, ky, k2, filter tables and diffz factors
   double* hsum;              // FP64 horizontal sums of p and q per level (mixed form's zero mode)
   double* stage64;           // mixed form: FP64 staging of host transfers (stage_n values, two halves)

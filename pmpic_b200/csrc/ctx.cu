@@ -264,13 +264,13 @@ int pmpic_create(const pmpic_config* cfg, pmpic_ctx** out) {
   }
   if (!rc) rc = dalloc(ctx, &ctx->keep, cap);
   if (!rc) rc = dalloc(ctx, &ctx->aux, cap);
-  if (!rc) rc = dalloc(ctx, &ctx->aux2, 2 * (size_t)ctx->nbmax + cap);
+  if (!rc) rc = dalloc(ctx, &ctx->aux2, (size_t)ctx->nbmax + cap);
   if (!rc) rc = dalloc(ctx, &ctx->dir, cap);
   if (!rc) rc = dalloc(ctx, &ctx->cell_count, (size_t)g.ncell + 1);
   if (!rc) rc = dalloc(ctx, &ctx->cell_start, (size_t)g.ncell + 1);
   if (!rc) rc = dalloc(ctx, &ctx->cell_fill, (size_t)g.ncell);
   if (!rc) rc = dalloc(ctx, &ctx->swapbuf, (size_t)ctx->swapcap * 30);  // 29 properties (+ the mixed form's cell id)
-  if (!rc) rc = dalloc(ctx, (int32_t**)&ctx->scan_tmp, (size_t)(std::max<int64_t>(std::max<int64_t>(g.ncell, ctx->cap), ctx->nbmax) / 4096 + 64));
+  if (!rc) rc = dalloc(ctx, (int32_t**)&ctx->scan_tmp, (size_t)(g.ncell / 4096 + 64));
   for (int i = 0; i < PMPIC_NGRID && !rc; ++i) rc = dalloc(ctx, &ctx->grid[i], (size_t)g.nphys);
   for (int i = 0; i < 5 && !rc; ++i) rc = dalloc(ctx, &ctx->gwork[i], (size_t)g.nphys);
   if (!rc) rc = dalloc(ctx, &ctx->mixres[0], 6 * (size_t)g.nphys);

@@ -98,7 +98,6 @@ FftPlan make_plan(int n, std::vector<double2>& tw) {
   FftPlan p{};
   std::vector<int> rad;
   if (!factor(n, rad) || (int)rad.size() > FFT_MAX_STAGES) return p;
-  factor(n, rad);
   p.n = n;
   p.nst = (int)rad.size();
   int len = n;

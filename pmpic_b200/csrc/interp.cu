@@ -1332,7 +1332,7 @@ namespace {
 constexpr int64_t SP_MAX_PARCELS = 131072;  // parcels per call
 constexpr int64_t SP_MAX_CELLS = 32768;     // nx*ny*nz per call
 constexpr int64_t SP_MAX_COLCHUNKS = 4096;  // ceil(nz/16)*nx*ny per call (row partials of par2grid)
-constexpr int64_t SP_MAX_TILES = (SP_MAX_CELLS + SCAN_TILE - 1) / SCAN_TILE + 1;
+static_assert(SP_MAX_CELLS <= (int64_t)SCAN_DIRECT * SCAN_TILE, "the static call's scan is one launch, without tile sums");
 constexpr size_t sp_round(size_t b) { return (b + 255) / 256 * 256; }
 // scratch layout (byte offsets)
 constexpr size_t SP_DEL = 0;                                                         // double[3][MAX_PARCELS]
@@ -1341,8 +1341,7 @@ constexpr size_t SP_CELL = SP_SORTED + sp_round(sizeof(int32_t) * SP_MAX_PARCELS
 constexpr size_t SP_COUNT = SP_CELL + sp_round(sizeof(int32_t) * SP_MAX_PARCELS);     // int32[MAX_CELLS+1]
 constexpr size_t SP_START = SP_COUNT + sp_round(sizeof(int32_t) * (SP_MAX_CELLS + 1));  // int32[MAX_CELLS+1]
 constexpr size_t SP_FILL = SP_START + sp_round(sizeof(int32_t) * (SP_MAX_CELLS + 1));   // int32[MAX_CELLS]
-constexpr size_t SP_TILES = SP_FILL + sp_round(sizeof(int32_t) * SP_MAX_CELLS);         // int32[MAX_TILES]
-constexpr size_t SP_INFO = SP_TILES + sp_round(sizeof(int32_t) * SP_MAX_TILES);         // DevInfo
+constexpr size_t SP_INFO = SP_FILL + sp_round(sizeof(int32_t) * SP_MAX_CELLS);          // DevInfo
 constexpr size_t SP_ROWS = SP_INFO + sp_round(sizeof(DevInfo));                         // double[MAX_COLCHUNKS][RPS]
 constexpr size_t SP_BYTES = SP_ROWS + sp_round(sizeof(double) * SP_MAX_COLCHUNKS * P2GLayout<1, 0, false>::RPS);
 static_assert(SP_BYTES < 8u << 20, "static par2grid scratch stays below 8 MB");
@@ -1384,7 +1383,6 @@ extern "C" int pmpic_par2grid_static(int32_t nx, int32_t ny, int32_t nz, double 
   int32_t* count = (int32_t*)(base + SP_COUNT);
   int32_t* cstart = (int32_t*)(base + SP_START);
   int32_t* fill = (int32_t*)(base + SP_FILL);
-  int32_t* tiles = (int32_t*)(base + SP_TILES);
   DevInfo* info = (DevInfo*)(base + SP_INFO);
   double* rows = (double*)(base + SP_ROWS);
   cudaStream_t st = (cudaStream_t)stream;
@@ -1411,7 +1409,7 @@ extern "C" int pmpic_par2grid_static(int32_t nx, int32_t ny, int32_t nz, double 
     launch(st, nblk(n, 256), 256, 0, k_bin_count, g, n, x, y, z, cell, del, SP_MAX_PARCELS, count, info,
            (int32_t*)nullptr);
   int64_t nl = 0;
-  scan_launch(count, ncell, cstart, fill, -1, info, tiles, st, nl);
+  scan_launch(count, ncell, cstart, fill, -1, info, nullptr, st, nl);
   if (n > 0) {
     launch(st, nblk(n, 256 * SC_ITEMS), 256, 0, k_bin_scatter, n, cell, count, cstart, fill, sorted, SP_MAX_PARCELS);
     launch(st, nblk(ncell, SORT_CELLS), SORT_CELLS, 0, k_sort_segments, ncell, cstart, fill, sorted);

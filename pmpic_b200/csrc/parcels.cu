@@ -2193,7 +2193,7 @@ int mixing(pmpic_ctx* ctx) {
     // is no keep==0 slot and the reference's loop (:350-389) does nothing.
     int32_t* z2 = ctx->aux;
     int32_t* nz2 = dcounter(ctx, 5);
-    int32_t* ones = ctx->aux2 + 2 * ctx->nbmax;
+    int32_t* ones = ctx->aux2 + ctx->nbmax;
     int32_t* no = dcounter(ctx, 6);
     if ((rc = compact(ctx, PredKeepEq{ctx->keep, 0}, norig, z2, nz2))) return rc;
     if ((rc = compact(ctx, PredKeepEq{ctx->keep, 1}, norig, ones, no))) return rc;
