@@ -462,7 +462,8 @@ struct PhysOut {
 };
 int fft_init(pmpic_ctx* ctx);
 // Forward and inverse transforms of nb arrays (1..6) at once.  mids: nb
-// scratch arrays of nspec values that are no input or output of the call.
+// scratch arrays of (Nz+1) (Ny+2) Nx values, an x-transformed field each, that
+// are no input or output of the call.
 int fft_forward(pmpic_ctx* ctx, int nb, const double* const* phys, double* const* spec, double* const* mids);
 int fft_forward(pmpic_ctx* ctx, int nb, const float* const* phys, float* const* spec, float* const* mids);
 int fft_inverse(pmpic_ctx* ctx, int nb, const SpecIn<double>& S, double* const* phys, double* const* mids);

@@ -44,7 +44,8 @@ bool factor(int n, std::vector<int>& out) {
 // Powers of two from 16 to 256 take the four-step split (st false: any
 // factorisation, one twiddle table).  The other lengths take a prefix of the
 // Stockham path's stages as n1 and the rest as n2 (st true), so that their
-// rows keep that path's arithmetic.  Of several the most even one.
+// rows keep that path's order of radices (fft_impl.cuh: fs_step1).  Of several
+// the most even one.
 void fs_split(FftPlan& p, bool st) {
   p.n1 = p.n2 = 0;
   p.st = st;

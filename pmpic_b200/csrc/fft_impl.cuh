@@ -354,8 +354,11 @@ __global__ void __launch_bounds__(FFT_THREADS) k_inv_y(Geom g, int TXF, FftPlan 
 // The kernels are instantiated for the splits (N1c, N2c) of FS_SPLITS and once
 // for every other length with the split read at run time (N1c = N2c = 0): the
 // radix then selects among the register DFTs by a branch that is uniform over
-// the grid.  What bounds them is L1 / shared memory: the twiddles are laid out
-// [k1][n2], so that the lanes of a warp, which differ in n2, read one line.
+// the grid.  What bounds them, by counters at 128^3: the FP32 x passes L1
+// (62-74% of its throughput), the FP64 ones L1 (46-59%) and the latency of few
+// warps (17-29% active); the y passes the latency of a row's loads and
+// barriers (33-47% of L1, 17-36% of DRAM).  The twiddles are laid out [k1][n2],
+// so that the lanes of a warp, which differ in n2, read one line.
 
 // W_16^m = exp(-2 pi i m / 16), m known at compile time after unrolling
 __device__ __forceinline__ real2 w16(int m) {
@@ -492,8 +495,11 @@ __device__ __forceinline__ void with_radix(int r, F&& f) {
 }
 // step 1 of one row: a[n1] = x[n2 + N2 n1] on entry; Y row [k1][n2] (padded).
 // ST: the first one or two stages of the Stockham path themselves, with its
-// twiddles (the length's other stages are the step-3 DFTs): a row then has the
-// bits that the Stockham kernels give it, whichever of the two runs.
+// twiddles (the length's other stages are the step-3 DFTs): the radices and
+// the order of the Stockham kernels.  Rows of the two differ at most where a
+// composite DFT has a quarter turn exactly, (0, -1), and the table its rounding
+// in long double, (-2.5e-20, -1): bits change only where the components of a
+// value differ by a factor above 1000 (FP64).
 // Otherwise an R-point DFT and the twiddle W_n^(n2 k1).
 template <int R, bool ST>
 __device__ __forceinline__ void fs_step1(real2* a, int n2, int N2, real2* Yrow, const real2* __restrict__ tw4) {
@@ -680,7 +686,7 @@ __global__ void __launch_bounds__(FS_THREADS, sizeof(real) == 4 ? 5 : 3) k4_inv_
 // forward y pass (phys -> mid): one z level, FS_YV consecutive pairs of x
 // columns per CTA; thread order puts consecutive x on consecutive threads, so
 // a warp's access is whole 128-byte lines (FP32 with 8 pairs, half lines: 4
-// instead of 2 lines an access, and L1 is what bounds the y passes)
+// instead of 2 lines an access)
 template <int N1c, int N2c, bool ST>
 __global__ void __launch_bounds__(FS_YT) k4_fwd_y(Geom g, int n1, int n2_,
                                                        const real2* __restrict__ tw4, Arr6<const real> physs,

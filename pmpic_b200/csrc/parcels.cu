@@ -77,6 +77,9 @@ struct SwapCheck {
 };
 // The list from the per-CTA counts.  A CTA with a true item sums the counts
 // before its own itself (no scan between the two passes), CTA 0 the total.
+// Where every CTA has one (the kept parcels of a backfill), that is at most
+// 0.5 GB out of L2 at 134 M parcels: mixing with removals there takes 9.69 ms,
+// with a scan between the passes 9.68.
 template <class Pred>
 __global__ void __launch_bounds__(256) k_write(Pred pr, int64_t n, const int32_t* __restrict__ blockcnt,
                                                int32_t* __restrict__ list, int32_t* __restrict__ dcount, SwapCheck sc) {

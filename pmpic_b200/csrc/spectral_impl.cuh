@@ -531,7 +531,8 @@ int vort2vel_spectral_impl(pmpic_ctx* ctx) {
   real* const* G = (real* const*)ctx->grid;
   if ((rc = zero_mode(ctx))) return rc;
   // scratch of the transforms: these arrays hold nothing that the inversion
-  // reads (the packed gather grids are made afresh before they are used)
+  // reads (the packed gather grids are made afresh before they are used, and
+  // their six grids hold three of the arrays: Ny + 2 <= 2 Ny)
   const size_t nmid = (size_t)g.nzp * g.sy * g.Nx;
   real* pk = RP(ctx->gpack);
   real* mids[6] = {RP(ctx->fftmid), RP(ctx->sas), RP(ctx->sbs), pk, pk + nmid, pk + 2 * nmid};
