@@ -418,6 +418,8 @@ int grid2par_multi(pmpic_ctx* ctx, const double* const* grids, int ng, double* c
 int par2grid_multi_m(pmpic_ctx* ctx, const float* const* fields, int nf, float* const* out, bool btot_from_bhz = false);
 int grid2par_multi_m(pmpic_ctx* ctx, const float* const* grids, int ng, float* const* out);
 // the same of six grids through their packed copy (parcels.cu)
+// (packable: the packing's launch can hold the grid)
+bool packable(const Geom& g);
 int grid2par_six(pmpic_ctx* ctx, const double* const* grids, double* const* out);
 int grid2par_six_m(pmpic_ctx* ctx, const float* const* grids, float* const* out);
 int cell_ids(pmpic_ctx* ctx, int32_t* dcells);

@@ -1207,7 +1207,9 @@ int par2grid_multi(pmpic_ctx* ctx, const double* const* fields, int nf, double* 
 // 478 -> 237; one parcel to two cells, FP64, 198 -> 148 and 158 -> 97; to four
 // 104 -> 103, to eight 65 -> 80.  32^3 with 65,536 parcels 16.5 -> 16.7, with
 // 32,768 12.7 -> 14.9 (the copy's launch).  The same operations either way.
-static bool g2p_packs(const pmpic_ctx* ctx) { return 2 * ctx->n >= ctx->g.nphys && ctx->n >= 65536; }
+static bool g2p_packs(const pmpic_ctx* ctx) {
+  return 2 * ctx->n >= ctx->g.nphys && ctx->n >= 65536 && packable(ctx->g);
+}
 
 template <int NG>
 static int launch_g2p(pmpic_ctx* ctx, const double* const* grids, double* const* out) {

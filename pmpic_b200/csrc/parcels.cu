@@ -248,13 +248,16 @@ __global__ void __launch_bounds__(256) k_pack(Geom g, Six<R> S, R* __restrict__ 
     }
   }
 }
+// a row of y and PK_K levels to a block in the grid's y and z: 65535 of either at most
+static dim3 pack_grid(const Geom& g) {
+  return dim3((g.Nx + PK_T - 1) / PK_T, (g.nzp + PK_K - 1) / PK_K, g.Ny);
+}
 template <class R>
 static void pack6(pmpic_ctx* ctx, const R* const* grids, R* out, const Zero2& z) {
   const Geom& g = ctx->g;
-  dim3 gr((g.Nx + PK_T - 1) / PK_T, (g.nzp + PK_K - 1) / PK_K, g.Ny);
   Six<R> S;
   for (int f = 0; f < 6; ++f) S.g[f] = grids[f];
-  launch(ctx->stream, gr, 256, 0, k_pack<R>, g, S, out, z);
+  launch(ctx->stream, pack_grid(g), 256, 0, k_pack<R>, g, S, out, z);
   ++ctx->nlaunch;
 }
 // the six fields at the two levels of xy corner (ci, cj) of a cell of level ck:
@@ -1714,6 +1717,10 @@ __global__ void k_prescribed_velocity(int64_t n, double* __restrict__ parcels, i
 
 }  // namespace
 
+bool packable(const Geom& g) {
+  const dim3 gr = pack_grid(g);
+  return gr.y <= 65535 && gr.z <= 65535;
+}
 int grid2par_six(pmpic_ctx* ctx, const double* const* grids, double* const* out) {
   return g2p6<double>(ctx, grids, ctx->del, ctx->del + ctx->cap, ctx->del + 2 * ctx->cap, out);
 }
