@@ -179,7 +179,8 @@ __global__ void __launch_bounds__(256) k_bin_scatter(int64_t n, const int32_t* _
 // plume's figures above are the same with either.
 // A range of more than SORT_CAP entries (more than 32 a cell on average) is
 // staged in several passes, as many whole cells in each as fit; only a cell
-// that is longer by itself is sorted in place, by one thread.  Of ranked cells
+// that is longer by itself is sorted in place, by its thread, beside the
+// CTA's other such cells.  Of ranked cells
 // a warp takes its own where one pass does, and every eighth where a pass holds
 // the cells of a few warps; a cell of more than SORT_WIDE entries all threads
 // take together.  Against sorting such ranges in place and such cells by one
@@ -239,13 +240,15 @@ __global__ void __launch_bounds__(SORT_CELLS) k_sort_segments(int64_t ncell, con
   const bool shared = wide || (ranked && !one);
   first[t] = (unsigned)s0 | (shared ? 1u << 31 : 0u);
   auto begin = [&](int u) { return u < SORT_CELLS ? (int)(first[u] & 0x7fffffffu) : m; };
-  if (!one) __syncthreads();
+  if (!one) {
+    if (len > SORT_CAP) isort(sorted + base, s0, len, [](int e) { return e; });
+    __syncthreads();
+  }
   for (int u0 = 0; u0 < SORT_CELLS;) {  // (uniform over the CTA)
     const int b = one ? 0 : begin(u0);
     // s1 rises with t: cells u0 .. u0 + fit - 1
     const int fit = one ? SORT_CELLS : __syncthreads_count(t >= u0 && s1 - b <= SORT_CAP);
-    if (fit == 0) {
-      if (t == u0) isort(sorted + base, s0, len, [](int e) { return e; });
+    if (fit == 0) {  // sorted above
       ++u0;
       continue;
     }
